@@ -1,0 +1,65 @@
+// hm_ara.h -- what the stages of the batched ARA build share: the problems of
+// a batch, their state, and the launchers of the per-block stages.
+//
+// Workspace layout of a problem (working precision W): Q (m x k), Y (m x s)
+// and B (n x k), column-major with the row count rounded up to 4 (ara_ld), so
+// that every column starts on a 16-byte boundary; the padding rows are zero.
+#pragma once
+#include <vector>
+
+#include "hm_internal.h"
+
+namespace hm {
+
+constexpr int kMaxCols = 256;  // max basis columns of one block (rank cap)
+constexpr int kMaxBs = 32;     // max sample columns of a round
+
+__host__ __device__ __forceinline__ int ara_ld(int rows) { return (rows + 3) & ~3; }
+
+struct Prob {
+  int r0, m, c0, n;
+  int kmax;
+  int level;
+  int u, v;
+  long long qoff, yoff, boff;  // workspace offsets (elements)
+  double tscale2;              // (this block's tolerance / the build's)^2: 1, or the level schedule's
+};
+
+struct ProbState {
+  double normA2;
+  double est;
+  int k;
+  int active;
+  int converged;
+  int rounds;
+  int r;      // rank after truncation (<= k)
+  int rhi;    // mixed precision: columns [0, rhi) keep a BF16 low part
+};
+
+// ---- orthogonalisation of one round's samples (hm_orth.cu) -------------------
+// The problems of a batch by the kernel shape that handles them: the height m
+// decides (one CTA with the sample resident in shared memory, or a cluster of
+// CTAs that split the rows).
+struct OrthPlan {
+  struct Class {
+    int rows = 0;     // rows of a CTA's slice that stay in shared memory
+    int cluster = 1;  // CTAs per problem
+    int first = 0, count = 0;  // problems: ids[first .. first + count)
+    int kcap = 0;     // widest basis of the class
+  };
+  std::vector<Class> classes;
+  DevBuf<int> ids;
+};
+
+// W: float or double.  Fills the plan (ids copied on `s`).
+template <typename W>
+hm_status orth_plan(const std::vector<Prob>& probs, OrthPlan* plan, cudaStream_t s);
+
+// One ARA round of every active problem: Y's bs sample columns are projected
+// against Q, tested (est = ||Y'||^2 / bs <= thresh2 tscale2 ||A||^2), and
+// otherwise orthonormalised and appended to Q.
+template <typename W>
+hm_status orth_round(const OrthPlan& plan, const Prob* probs, ProbState* st, W* ws, int bs, double thresh2,
+                     cudaStream_t s);
+
+}  // namespace hm

@@ -30,6 +30,7 @@
 #include <numeric>
 #include <type_traits>
 
+#include "hm_ara.h"
 #include "hm_hmatrix.h"
 #include "hm_mma.cuh"
 #include "hm_structure.h"
@@ -43,39 +44,8 @@ namespace {
 constexpr int kTR = 64;        // rows of a KMM tile
 constexpr int kTC = 64;        // columns per KMM chunk
 constexpr int kKmmThreads = 256;
-constexpr int kOrthThreads = 256;
-constexpr int kMaxCols = 256;  // max basis columns of one block (rank cap)
 constexpr int kTruncMax = 128; // widest basis the SVD truncation handles (wider: kept as sampled)
 constexpr int kColGroup = 128; // projection columns per sketch launch
-constexpr int kMaxBs = 32;     // max sample block (the option)
-// widest sample (basis + test columns) one orthogonalisation handles; the
-// shared memory and per-thread arrays of k_orth scale with it (64 halves the
-// CTAs per SM, measured slower while the sample stays at 32 columns)
-template <typename W>
-constexpr int max_bs() {
-  return 32;
-}
-
-struct Prob {
-  int r0, m, c0, n;
-  int kmax;
-  int level;
-  int u, v;
-  long long qoff, yoff, boff;  // workspace offsets (floats)
-  double tscale2;              // (this block's tolerance / the build's)^2: 1, or the level schedule's
-};
-
-struct ProbState {
-  double normA2;
-  double est;
-  int k;
-  int active;
-  int converged;
-  int rounds;
-  int r;      // rank after truncation (<= k)
-  int rhi;    // mixed precision: columns [0, rhi) keep a BF16 low part
-};
-
 template <typename W>
 struct KmmArgs {
   const Prob* probs;
@@ -118,8 +88,9 @@ __global__ void __launch_bounds__(kKmmThreads) k_kmm(KmmArgs<W> a) {
   const int nc = a.mode ? P.m : P.n;        // columns of the operator
   const int rbase = a.mode ? P.c0 : P.r0;
   const int cbase = a.mode ? P.r0 : P.c0;
-  W* out = a.ws + (a.mode ? P.boff : P.yoff) + (size_t)col0 * mr;
-  const W* Q = a.ws + P.qoff + (size_t)col0 * P.m;  // mode 1: W = Q (m x k, ld m)
+  const int ldo = ara_ld(mr), ldq = ara_ld(P.m);
+  W* out = a.ws + (a.mode ? P.boff : P.yoff) + (size_t)col0 * ldo;
+  const W* Q = a.ws + P.qoff + (size_t)col0 * ldq;  // mode 1: W = Q (m x k)
   const int nslab = s <= 32 ? 1 : (s <= 64 ? 2 : 4);
   const int ncg = 4 / nslab;
   const int t = threadIdx.x, r = t & 63, q = t >> 6;
@@ -151,7 +122,7 @@ __global__ void __launch_bounds__(kKmmThreads) k_kmm(KmmArgs<W> a) {
         if (a.mode == 0)
           w = (W)gauss_at(a.seed, (uint32_t)it.x, (uint32_t)j, (uint32_t)(a.round * kMaxBs + cc));
         else
-          w = Q[(size_t)cc * P.m + j];
+          w = Q[(size_t)cc * ldq + j];
       }
       Wsm[jj * kColGroup + cc] = w;
     }
@@ -191,11 +162,10 @@ __global__ void __launch_bounds__(kKmmThreads) k_kmm(KmmArgs<W> a) {
       }
     }
   }
-  if (cg == 0 && row_ok) {
-    const int ld = mr;
+  if (cg == 0 && row < ldo) {  // the padding rows get their zeros
     for (int c = 0; c < 32; ++c) {
       int col = slab * 32 + c;
-      if (col < s) out[(size_t)col * ld + row] = acc[c];
+      if (col < s) out[(size_t)col * ldo + row] = acc[c];
     }
   }
   if (want_norm) {
@@ -299,8 +269,8 @@ __global__ void __launch_bounds__(128) k_kmm_fast(KmmFastArgs a) {
   const int nc = MODE ? P.m : P.n;
   const int rbase = MODE ? P.c0 : P.r0;
   const int cbase = MODE ? P.r0 : P.c0;
-  const int mr_ld = mr;
-  float* out = a.ws + (MODE ? P.boff : P.yoff) + (size_t)col0 * mr_ld;
+  const int ld = ara_ld(mr);
+  float* out = a.ws + (MODE ? P.boff : P.yoff) + (size_t)col0 * ld;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
   const int ra = it.y * kTR + warp * 16 + g, rb = ra + 8;
   const bool ra_ok = ra < mr, rb_ok = rb < mr;
@@ -403,16 +373,16 @@ __global__ void __launch_bounds__(128) k_kmm_fast(KmmFastArgs a) {
       }
     }
   }
-  const int ld = mr;
+  // rows mr .. ld - 1 (padding) get their zeros
 #pragma unroll
   for (int nt = 0; nt < NT; ++nt) {
     if (nt < ntiles) {
       const int c = nt * 8 + 2 * t;
-      if (ra_ok) {
+      if (ra < ld) {
         if (c < s) out[(size_t)c * ld + ra] = acc[nt][0];
         if (c + 1 < s) out[(size_t)(c + 1) * ld + ra] = acc[nt][1];
       }
-      if (rb_ok) {
+      if (rb < ld) {
         if (c < s) out[(size_t)c * ld + rb] = acc[nt][2];
         if (c + 1 < s) out[(size_t)(c + 1) * ld + rb] = acc[nt][3];
       }
@@ -469,7 +439,7 @@ __global__ void k_pack_q(const Prob* probs, const ProbState* st, const float* ws
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
       const int row = i + (r & 1) + 8 * (r >> 1);
-      x[r] = (c < k && row < P.m) ? Q[(size_t)c * P.m + row] : 0.f;
+      x[r] = (c < k && row < P.m) ? Q[(size_t)c * ara_ld(P.m) + row] : 0.f;
     }
     uint4 o;
     split_bf16x2(x[0], x[1], o.x, o.z);
@@ -517,340 +487,6 @@ void launch_kmm_fast(int d, int kind, int mode, int nt, unsigned grid, cudaStrea
 }
 
 // ---------------------------------------------------------------------------
-// per-block orthogonalisation of the new sample
-// ---------------------------------------------------------------------------
-template <typename W>
-struct OrthArgs {
-  const Prob* probs;
-  ProbState* st;
-  W* ws;
-  int bs;          // sample columns of this round
-  int bst;         // of which the last bst are test columns (0: none)
-  double thresh2;  // stop when est <= thresh2 * normA2
-  int round;
-};
-
-// C[j][c] = sum_i Q[i, j] Y[i, c]  (k x bs), result in shared Csm.  Each
-// thread owns a TA x 4 tile of C (rows j = 8 * TA-blocks, columns c in fours),
-// so that a staged value serves TA or 4 FMAs instead of one; TA grows with k
-// so that the 256 threads stay busy.  Every output sums its products in the
-// same order (rows of a 32-row chunk in turn, chunks in turn) for any TA.
-template <typename W, int TA>
-__device__ void block_qty_t(const W* Q, const W* Y, int m, int k, int bs, W* Csm, W* stage) {
-  const int t = threadIdx.x;
-  const int jg = t >> 3, cg = t & 7;  // 32 row groups of TA x 8 column groups of 4
-  W acc[TA][4];
-#pragma unroll
-  for (int a = 0; a < TA; ++a) acc[a][0] = acc[a][1] = acc[a][2] = acc[a][3] = W(0);
-  W* Qs = stage;                  // [kMaxCols][33]
-  W* Ys = stage + kMaxCols * 33;  // [max_bs][33]
-  const bool act = jg * TA < k && cg * 4 < bs;
-  for (int i0 = 0; i0 < m; i0 += 32) {
-    for (int e = t; e < 32 * k; e += kOrthThreads) {
-      int ii = e & 31, j = e >> 5;
-      Qs[j * 33 + ii] = (i0 + ii < m) ? Q[(size_t)j * m + i0 + ii] : W(0);
-    }
-    for (int e = t; e < 32 * bs; e += kOrthThreads) {
-      int ii = e & 31, c = e >> 5;
-      Ys[c * 33 + ii] = (i0 + ii < m) ? Y[(size_t)c * m + i0 + ii] : W(0);
-    }
-    __syncthreads();
-    if (act) {
-      for (int ii = 0; ii < 32; ++ii) {
-        W q[TA], y[4];
-#pragma unroll
-        for (int a = 0; a < TA; ++a) q[a] = Qs[(jg * TA + a) * 33 + ii];  // rows j >= k: never stored
-#pragma unroll
-        for (int b = 0; b < 4; ++b) y[b] = Ys[(cg * 4 + b) * 33 + ii];
-#pragma unroll
-        for (int a = 0; a < TA; ++a)
-#pragma unroll
-          for (int b = 0; b < 4; ++b) acc[a][b] = fma(q[a], y[b], acc[a][b]);
-      }
-    }
-    __syncthreads();
-  }
-  if (act) {
-#pragma unroll
-    for (int a = 0; a < TA; ++a)
-#pragma unroll
-      for (int b = 0; b < 4; ++b) {
-        const int j = jg * TA + a, c = cg * 4 + b;
-        if (j < k && c < bs) Csm[j * bs + c] = acc[a][b];
-      }
-  }
-  __syncthreads();
-}
-
-template <typename W>
-__device__ void block_qty(const W* Q, const W* Y, int m, int k, int bs, W* Csm, W* stage) {
-  if (k <= 32)
-    block_qty_t<W, 1>(Q, Y, m, k, bs, Csm, stage);
-  else if (k <= 64)
-    block_qty_t<W, 2>(Q, Y, m, k, bs, Csm, stage);
-  else if (k <= 128)
-    block_qty_t<W, 4>(Q, Y, m, k, bs, Csm, stage);
-  else
-    block_qty_t<W, 8>(Q, Y, m, k, bs, Csm, stage);
-}
-
-// Y -= Q C
-template <typename W>
-__device__ void block_update(const W* Q, W* Y, int m, int k, int bs, const W* Csm) {
-  for (int i = threadIdx.x; i < m; i += kOrthThreads) {
-    W y[max_bs<W>()];
-    for (int c = 0; c < bs; ++c) y[c] = Y[(size_t)c * m + i];
-    for (int j = 0; j < k; ++j) {
-      W qv = Q[(size_t)j * m + i];
-      for (int c = 0; c < bs; ++c) y[c] = fma(-qv, Csm[j * bs + c], y[c]);
-    }
-    for (int c = 0; c < bs; ++c) Y[(size_t)c * m + i] = y[c];
-  }
-  __syncthreads();
-}
-
-// G = Y^T Y in FP64 (cols x cols), into shared Gs.  Each thread owns a 2 x 2
-// tile of the upper triangle (the lower one is its mirror: a product of two
-// values is the same in either order), so a staged value serves two
-// products; every entry sums its products in row order.
-template <typename W>
-__device__ void gram64(const W* Y, int m, int cols, double* Gs, W* stage) {
-  static_assert(max_bs<W>() <= 32, "2 x 2 tiles of 16 x 16 threads cover 32 columns");
-  const int t = threadIdx.x;
-  const int ta = t >> 4, tb = t & 15;  // rows 2 ta, 2 ta + 1; columns 2 tb, 2 tb + 1
-  const bool act = ta <= tb && 2 * tb < cols;
-  double acc[2][2] = {{0.0, 0.0}, {0.0, 0.0}};
-  W* Ys = stage;  // [max_bs][33]
-  for (int i0 = 0; i0 < m; i0 += 32) {
-    for (int e = t; e < 32 * cols; e += kOrthThreads) {
-      int ii = e & 31, c = e >> 5;
-      Ys[c * 33 + ii] = (i0 + ii < m) ? Y[(size_t)c * m + i0 + ii] : W(0);
-    }
-    __syncthreads();
-    if (act) {
-      for (int ii = 0; ii < 32; ++ii) {
-        const double y0 = (double)Ys[(2 * ta) * 33 + ii], y1 = (double)Ys[(2 * ta + 1) * 33 + ii];
-        const double z0 = (double)Ys[(2 * tb) * 33 + ii], z1 = (double)Ys[(2 * tb + 1) * 33 + ii];
-        acc[0][0] += y0 * z0;
-        acc[0][1] += y0 * z1;
-        acc[1][0] += y1 * z0;
-        acc[1][1] += y1 * z1;
-      }
-    }
-    __syncthreads();
-  }
-  if (act) {
-#pragma unroll
-    for (int u = 0; u < 2; ++u)
-#pragma unroll
-      for (int v = 0; v < 2; ++v) {
-        const int a = 2 * ta + u, b = 2 * tb + v;
-        if (a < cols && b < cols) {
-          Gs[a * cols + b] = acc[u][v];
-          Gs[b * cols + a] = acc[u][v];
-        }
-      }
-  }
-  __syncthreads();
-}
-
-// Cholesky of the leading principal part of G (cols x cols, row-major), in
-// place into its lower triangle, with symmetric pivoting when `pivot`; stops at
-// the first pivot <= tau.  perm receives the column order.  Returns the rank.
-// Runs on thread 0 (cols <= 32).
-__device__ int chol_pivoted(double* G, int cols, int* perm, bool pivot, double tau) {
-  for (int i = 0; i < cols; ++i) perm[i] = i;
-  int rank = 0;
-  for (int j = 0; j < cols; ++j) {
-    int p = j;
-    if (pivot) {
-      for (int i = j + 1; i < cols; ++i)
-        if (G[i * cols + i] > G[p * cols + p]) p = i;
-    }
-    if (!(G[p * cols + p] > tau)) break;
-    if (p != j) {
-      // symmetric swap of rows/cols j and p
-      for (int c = 0; c < cols; ++c) {
-        double x = G[j * cols + c];
-        G[j * cols + c] = G[p * cols + c];
-        G[p * cols + c] = x;
-      }
-      for (int r = 0; r < cols; ++r) {
-        double x = G[r * cols + j];
-        G[r * cols + j] = G[r * cols + p];
-        G[r * cols + p] = x;
-      }
-      int x = perm[j];
-      perm[j] = perm[p];
-      perm[p] = x;
-    }
-    double d = sqrt(G[j * cols + j]);
-    G[j * cols + j] = d;
-    for (int i = j + 1; i < cols; ++i) G[i * cols + j] /= d;
-    for (int i = j + 1; i < cols; ++i)
-      for (int c = j + 1; c <= i; ++c) {
-        G[i * cols + c] -= G[i * cols + j] * G[c * cols + j];
-        G[c * cols + i] = G[i * cols + c];
-      }
-    rank = j + 1;
-  }
-  return rank;
-}
-
-// Y[:, 0:r] <- Y[:, perm[0:r]] L^{-T}  (row by row, in place)
-template <typename W>
-__device__ void apply_linv(W* Y, int m, int cols, const double* L, const int* perm, int r) {
-  for (int i = threadIdx.x; i < m; i += kOrthThreads) {
-    W y[max_bs<W>()];
-    for (int c = 0; c < cols; ++c) y[c] = Y[(size_t)c * m + i];
-    double x[max_bs<W>()];
-    for (int a = 0; a < r; ++a) {
-      double v = y[perm[a]];
-      for (int b = 0; b < a; ++b) v -= L[a * cols + b] * x[b];
-      x[a] = v / L[a * cols + a];
-    }
-    for (int a = 0; a < r; ++a) Y[(size_t)a * m + i] = (W)x[a];
-  }
-  __syncthreads();
-}
-
-// Orthonormalises the `cols` columns of Y (already projected against Q[0..k))
-// in place: pivoted Cholesky-QR, then two Cholesky-QR refinements; R^{-1} of
-// an ill-conditioned sample magnifies whatever the Gram-Schmidt left along
-// the old basis, so after the first refinement the block is projected against
-// Q once more.  Returns the rank r; Y[0..r) is the new orthonormal block.
-template <typename W>
-__device__ int cholqr_block(const W* Q, int k, W* Y, int m, int cols, double* Gs, int* perm, int* rank_sh,
-                            W* Csm, W* stage) {
-  gram64(Y, m, cols, Gs, stage);
-  if (threadIdx.x == 0) {
-    double tr = 0;
-    for (int c = 0; c < cols; ++c) tr += Gs[c * cols + c];
-    // columns whose norm is below FP32 resolution of the sample are noise
-    *rank_sh = chol_pivoted(Gs, cols, perm, true, 1e-10 * tr);
-  }
-  __syncthreads();
-  int r = *rank_sh;
-  if (r == 0) return 0;
-  apply_linv(Y, m, cols, Gs, perm, r);
-  for (int pass = 0; pass < 2 && r > 0; ++pass) {
-    if (pass == 1 && k > 0) {
-      block_qty(Q, Y, m, k, r, Csm, stage);
-      block_update(Q, Y, m, k, r, Csm);
-    }
-    const int rg = r;  // dimension (and row stride) of this Gram matrix
-    gram64(Y, m, rg, Gs, stage);
-    if (threadIdx.x == 0) *rank_sh = chol_pivoted(Gs, rg, perm, pass == 1, pass == 1 ? 1e-12 * rg : 0.0);
-    __syncthreads();
-    r = *rank_sh;  // a refinement that loses rank keeps the leading columns
-    if (r > 0) apply_linv(Y, m, rg, Gs, perm, r);
-  }
-  return r;
-}
-
-template <typename W>
-__device__ double trace_gram(const W* Y, int m, int cols, double* Gs, W* stage) {
-  gram64(Y, m, cols, Gs, stage);
-  double tr = 0;
-  for (int c = 0; c < cols; ++c) tr += Gs[c * cols + c];
-  return tr;
-}
-
-// One ARA round of one block.  The sample Y (m x bs) holds bs - bst basis
-// columns and bst test columns (bst = 0: every column is a basis column and
-// the estimate comes from the whole sample, as in the reference's ARA).
-//  1. the whole sample is projected against Q (classical Gram-Schmidt, twice);
-//  2. the test columns' projected norm estimates the residual
-//     ||(I - QQ^T) A||_F^2 ~ ||Y_t'||^2 / bst: below the threshold, done;
-//  3. the basis columns are orthonormalised and appended to Q;
-//  4. the test columns, projected against the new columns as well, estimate
-//     the residual left by the grown basis: below the threshold, done in this
-//     round (no extra pass); otherwise they are a sample of that residual and
-//     are orthonormalised and appended too.
-template <typename W>
-__global__ void __launch_bounds__(kOrthThreads) k_orth(OrthArgs<W> a) {
-  constexpr int MB = max_bs<W>();
-  extern __shared__ __align__(16) unsigned char osm[];
-  double* Gs = reinterpret_cast<double*>(osm);         // [MB*MB]
-  W* Csm = reinterpret_cast<W*>(Gs + MB * MB);         // [kMaxCols*MB]
-  W* stage = Csm + kMaxCols * MB;                      // (kMaxCols+MB)*33
-  __shared__ int perm[MB];
-  __shared__ int rank_sh;
-  __shared__ int decision;  // 0 continue, 1 converged, 2 cap reached
-
-  const int p = blockIdx.x;
-  ProbState S = a.st[p];
-  if (!S.active) return;
-  const Prob P = a.probs[p];
-  const int m = P.m, bs = a.bs, bst = a.bst, bsb = bs - bst;
-  W* Q = a.ws + P.qoff;
-  W* Y = a.ws + P.yoff;
-  W* Yt = Y + (size_t)bsb * m;
-  int k = S.k;
-  for (int pass = 0; pass < 2 && k > 0; ++pass) {
-    block_qty(Q, Y, m, k, bs, Csm, stage);
-    block_update(Q, Y, m, k, bs, Csm);
-  }
-  {
-    const int ne = bst > 0 ? bst : bs;
-    const double tr = trace_gram(bst > 0 ? Yt : Y, m, ne, Gs, stage);
-    if (threadIdx.x == 0) {
-      const double est = tr / ne;
-      S.est = est;
-      S.rounds += 1;
-      if (est <= a.thresh2 * P.tscale2 * S.normA2 || S.normA2 == 0.0) decision = 1;
-      else if (k + bsb > P.kmax) decision = 2;
-      else decision = 0;
-    }
-    __syncthreads();
-  }
-  if (decision != 0) {
-    if (threadIdx.x == 0) {
-      S.active = 0;
-      S.converged = decision == 1;
-      a.st[p] = S;
-    }
-    return;
-  }
-  int r = cholqr_block(Q, k, Y, m, bsb, Gs, perm, &rank_sh, Csm, stage);
-  for (int c = 0; c < r; ++c)
-    for (int i = threadIdx.x; i < m; i += kOrthThreads) Q[(size_t)(k + c) * m + i] = Y[(size_t)c * m + i];
-  __syncthreads();
-  k += r;
-  bool conv = false;
-  if (bst > 0) {
-    if (r > 0) {
-      const W* Qn = Q + (size_t)(k - r) * m;
-      for (int pass = 0; pass < 2; ++pass) {
-        block_qty(Qn, Yt, m, r, bst, Csm, stage);
-        block_update(Qn, Yt, m, r, bst, Csm);
-      }
-    }
-    const double tr = trace_gram(Yt, m, bst, Gs, stage);
-    if (threadIdx.x == 0) S.est = tr / bst;
-    conv = tr / bst <= a.thresh2 * P.tscale2 * S.normA2;
-    if (!conv && k < P.kmax) {
-      int rt = cholqr_block(Q, k, Yt, m, bst, Gs, perm, &rank_sh, Csm, stage);
-      rt = min(rt, P.kmax - k);
-      for (int c = 0; c < rt; ++c)
-        for (int i = threadIdx.x; i < m; i += kOrthThreads) Q[(size_t)(k + c) * m + i] = Yt[(size_t)c * m + i];
-      __syncthreads();
-      k += rt;
-    }
-  } else {
-    conv = r == 0;
-  }
-  if (threadIdx.x == 0) {
-    S.k = k;
-    if (conv) {
-      S.active = 0;
-      S.converged = 1;
-    }
-    a.st[p] = S;
-  }
-}
-
-// ---------------------------------------------------------------------------
 // truncation: A ~ Q B^T with B = A^T Q; eig(B^T B) = W diag(lambda) W^T gives
 // the singular values of A's approximation, sqrt(lambda), and
 // A ~ (Q W_r)(B W_r)^T with the smallest r whose discarded sum of lambda fits
@@ -881,7 +517,7 @@ __global__ void __launch_bounds__(kGramThreads) k_gram_big(const Prob* probs, co
   for (int i0 = 0; i0 < P.n; i0 += 16) {
     for (int e = t; e < 16 * k; e += kGramThreads) {
       int ii = e % 16, j = e / 16;
-      Bs[ii][j] = (i0 + ii < P.n) ? (double)B[(size_t)j * P.n + i0 + ii] : 0.0;
+      Bs[ii][j] = (i0 + ii < P.n) ? (double)B[(size_t)j * ara_ld(P.n) + i0 + ii] : 0.0;
     }
     __syncthreads();
     if (active) {
@@ -1075,10 +711,11 @@ __global__ void k_pack_trunc(const Prob* probs, const ProbState* st, const W* ws
   const Prob P = probs[p];
   if (k > kTruncMax) {  // kept as sampled (W = I): U = Q, V = B, a copy
     for (int side = 0; side < 2; ++side) {
-      const size_t cnt = (size_t)(side ? P.n : P.m) * r;
+      const int rows = side ? P.n : P.m, ld = ara_ld(rows);
       const W* src = ws + (side ? P.boff : P.qoff);
       float* out = dst + (side ? dst_v[p] : dst_u[p]);
-      for (size_t e = threadIdx.x; e < cnt; e += blockDim.x) out[e] = (float)src[e];
+      for (size_t e = threadIdx.x; e < (size_t)rows * r; e += blockDim.x)
+        out[e] = (float)src[e / rows * ld + e % rows];
     }
     return;
   }
@@ -1091,14 +728,14 @@ __global__ void k_pack_trunc(const Prob* probs, const ProbState* st, const W* ws
     for (int e = threadIdx.x; e < k * nc; e += blockDim.x) ws_sh[e] = w[(size_t)(c0 + e / k) * k + e % k];
     __syncthreads();
     for (int side = 0; side < 2; ++side) {
-      const int rows = side ? P.n : P.m;
+      const int rows = side ? P.n : P.m, ld = ara_ld(rows);
       const W* src = ws + (side ? P.boff : P.qoff);
       float* out = dst + (side ? dst_v[p] : dst_u[p]);
       for (int i = threadIdx.x; i < rows; i += blockDim.x) {
         float acc[32];
         for (int c = 0; c < nc; ++c) acc[c] = 0.f;
         for (int a = 0; a < k; ++a) {
-          float x = (float)src[(size_t)a * rows + i];
+          float x = (float)src[(size_t)a * ld + i];
           for (int c = 0; c < nc; ++c) acc[c] = fmaf(x, ws_sh[c * k + a], acc[c]);
         }
         for (int c = 0; c < nc; ++c) out[(size_t)(c0 + c) * rows + i] = acc[c];
@@ -1158,12 +795,6 @@ template <typename W>
 size_t kmm_smem() {
   return sizeof(W) * (kTC * kColGroup) + sizeof(float) * (kTC * kTR + kMaxDim * kTC) +
          sizeof(double) * (kKmmThreads / 32);
-}
-
-template <typename W>
-size_t orth_smem() {
-  constexpr int MB = max_bs<W>();
-  return sizeof(double) * MB * MB + sizeof(W) * kMaxCols * MB + sizeof(W) * (kMaxCols + MB) * 33;
 }
 
 }  // namespace
@@ -1313,18 +944,16 @@ hm_status hmatrix_build(hm_kdtree t, hm_structure s, const double* d_points, con
     using W = decltype(tag);
     const size_t budget_elems = budget_bytes / sizeof(W);
     HM_CUDA(cudaFuncSetAttribute(k_kmm<W>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kmm_smem<W>()));
-    HM_CUDA(cudaFuncSetAttribute(k_orth<W>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)orth_smem<W>()));
     // The specialised sketch kernels draw a double-width first sample (the
     // generation of the kernel block, not its product with the sample, is
     // the cost of a pass, so blocks of rank bs..2 bs finish a pass earlier).
-    // Separate test columns (k_orth's bst) are supported but measured slower
-    // on the 2^20-point Matern build (wider first passes, wider bases), so
-    // rounds use bst = 0, the reference ARA's estimate from the sample itself.
+    // The residual is estimated from the sample itself, as in the reference's
+    // ARA (separate test columns measured slower on the 2^20-point Matern
+    // build: wider first passes, wider bases).
     constexpr bool kTensorW = std::is_same<W, float>::value;
     const bool fastW = kTensorW && t->d <= 3;
-    const int bst = 0;
-    const int bs_first = fastW ? std::min(2 * bs, kMaxBs) : bs;  // round 0 basis columns
-    const int wmax = std::max(bs_first, bs) + bst;                // widest sample
+    const int bs_first = fastW ? std::min(2 * bs, kMaxBs) : bs;  // round 0 columns
+    const int wmax = std::max(bs_first, bs);                      // widest sample
     // greedy batches under the workspace budget; one workspace for all of
     // them (child blocks of split problems come in later batches, whose
     // workspace is no larger unless a batch of them packs tighter)
@@ -1333,7 +962,8 @@ hm_status hmatrix_build(hm_kdtree t, hm_structure s, const double* d_points, con
       size_t wsz = 0;
       while (pe < (long long)probs.size()) {
         const Prob& P = probs[pe];
-        size_t need = (size_t)P.m * (P.kmax + wmax) + (size_t)P.m * wmax + (size_t)P.n * (P.kmax + wmax);
+        const size_t lm = ara_ld(P.m), ln = ara_ld(P.n);
+        size_t need = lm * (P.kmax + wmax) + lm * wmax + ln * (P.kmax + wmax);
         if (pe > ps && wsz + need > budget_elems) break;
         wsz += need;
         ++pe;
@@ -1367,11 +997,11 @@ hm_status hmatrix_build(hm_kdtree t, hm_structure s, const double* d_points, con
       for (int i = 0; i < nb; ++i) {
         Prob& P = bp[i];
         P.qoff = (long long)off;
-        off += (size_t)P.m * (P.kmax + wmax);
+        off += (size_t)ara_ld(P.m) * (P.kmax + wmax);
         P.yoff = (long long)off;
-        off += (size_t)P.m * wmax;
+        off += (size_t)ara_ld(P.m) * wmax;
         P.boff = (long long)off;
-        off += (size_t)P.n * (P.kmax + wmax);
+        off += (size_t)ara_ld(P.n) * (P.kmax + wmax);
         for (int tt = 0; tt * kTR < P.m; ++tt) items_rows.push_back(make_int2(i, tt));
         for (int tt = 0; tt * kTR < P.n; ++tt) items_cols.push_back(make_int2(i, tt));
       }
@@ -1404,24 +1034,19 @@ hm_status hmatrix_build(hm_kdtree t, hm_structure s, const double* d_points, con
       ka.bs = bs;
       ka.seed = (uint32_t)(opt.seed ^ (opt.seed >> 32)) ^ 0x5bd1e995u;
       ka.ws = ws.p;
-      OrthArgs<W> oa;
-      oa.probs = dprobs.p;
-      oa.st = dst.p;
-      oa.ws = ws.p;
-      oa.bs = bs;
-      oa.bst = 0;
-      oa.thresh2 = thresh2;
+      OrthPlan orth;
+      if ((st = orth_plan<W>(bp, &orth, stream))) return st;
       // FP32 working precision and d <= 3: specialised tensor-core sketch
       // kernels; otherwise the SIMT kernel in the working precision
       constexpr bool kTensor = std::is_same<W, float>::value;
       const bool fast = kTensor && t->d <= 3;
       KmmFastArgs kf{};
       DevBuf<uint2> om2;
-      // round 0 basis columns: as wide as every block's rank cap allows
+      // round 0 columns: as wide as every block's rank cap allows
       int bs0 = bs_first;
       for (const Prob& P : bp)
         if (P.kmax < bs0) bs0 = std::max(bs, P.kmax / 8 * 8);
-      const int bs8 = (bs0 + bst + 7) & ~7;
+      const int bs8 = (bs0 + 7) & ~7;
       int om_rows2 = 0;
       if (fast) {
         int max_n = 1;
@@ -1452,20 +1077,18 @@ hm_status hmatrix_build(hm_kdtree t, hm_structure s, const double* d_points, con
       tr.mark("batch setup", stream, nb, 0);
       const int max_rounds = kMaxCols / bs + 2;
       for (int round = 0; round < max_rounds; ++round) {
+        // sample columns: double width in the first round and again from the
+        // fourth on (the blocks still active by then are the high-rank ones;
+        // entry generation, not the sample width, is the cost of a round, so
+        // wider rounds mean fewer of them; earlier, a wider basis would cost
+        // more in the projection than it saves)
+        const int rbs = fast && round != 1 && round != 2 ? bs0 : bs;
         if (fast) {
-          // basis + test columns: double width in the first round and again
-          // from the fourth on (the blocks still active by then are the
-          // high-rank ones; entry generation, not the sample width, is the
-          // cost of a round, so wider rounds mean fewer of them; earlier, a
-          // wider basis would cost more in the projection than it saves)
-          const int rbs = (round == 1 || round == 2 ? bs : bs0) + bst;
           k_omega_pack<<<592, 256, 0, stream>>>(om2.p, om_rows2 / 8, rbs, bs8 / 8, ka.seed, round);
           HM_LAUNCH_CHECK();
           kf.round = round;
           kf.bs = rbs;
           kf.items = drows.p;
-          oa.bs = rbs;
-          oa.bst = bst;
           launch_kmm_fast(t->d, opt.kernel, 0, (rbs + 7) / 8, (unsigned)items_rows.size(), stream, kf);
         } else {
           ka.mode = 0;
@@ -1476,9 +1099,7 @@ hm_status hmatrix_build(hm_kdtree t, hm_structure s, const double* d_points, con
         }
         HM_LAUNCH_CHECK();
         tr.mark("  round sketch", stream, round, 1);
-        oa.round = round;
-        k_orth<W><<<nb, kOrthThreads, orth_smem<W>(), stream>>>(oa);
-        HM_LAUNCH_CHECK();
+        if ((st = orth_round<W>(orth, dprobs.p, dst.p, ws.p, rbs, thresh2, stream))) return st;
         tr.mark("  round orth", stream, round, 2);
         HM_CUDA(cudaMemcpyAsync(hst.data(), dst.p, sizeof(ProbState) * nb, cudaMemcpyDeviceToHost, stream));
         HM_CUDA(cudaStreamSynchronize(stream));
