@@ -62,4 +62,29 @@ template <typename W>
 hm_status orth_round(const OrthPlan& plan, const Prob* probs, ProbState* st, W* ws, int bs, double thresh2,
                      cudaStream_t s);
 
+// ---- truncation (hm_trunc.cu) --------------------------------------------------
+constexpr int kTruncMax = 128;  // widest basis the SVD truncation handles (wider: kept as sampled)
+
+// Eigenvectors of the truncated blocks of a batch: problem p's W_r (k x r,
+// FP32, column-major) starts at w + woff[p].
+struct TruncWork {
+  DevBuf<long long> woff;
+  DevBuf<float> w;
+};
+
+// From B = A^T Q and the states (k set; hst: their host copies): the rank r
+// and low-part columns rhi of every problem, and W_r.  tol2, rbudget: the
+// truncation and BF16 rounding budgets relative to ||A||_F^2.
+template <typename W>
+hm_status trunc_rank(const std::vector<Prob>& bp, const std::vector<ProbState>& hst, const Prob* probs, ProbState* st,
+                     const W* ws, double tol2, double rbudget, TruncWork* tw, cudaStream_t s);
+
+// U = Q W_r and V = B W_r of the problems with dst_u >= 0, FP32, column-major
+// without padding.  rows, cols: the batch's 64-row tiles (problem, tile) over
+// the blocks' rows and columns.
+template <typename W>
+hm_status trunc_pack(const Prob* probs, const ProbState* st, const W* ws, const TruncWork& tw, const int2* rows,
+                     size_t nrows, const int2* cols, size_t ncols, const long long* dst_u, const long long* dst_v,
+                     float* dst, cudaStream_t s);
+
 }  // namespace hm

@@ -44,7 +44,6 @@ namespace {
 constexpr int kTR = 64;        // rows of a KMM tile
 constexpr int kTC = 64;        // columns per KMM chunk
 constexpr int kKmmThreads = 256;
-constexpr int kTruncMax = 128; // widest basis the SVD truncation handles (wider: kept as sampled)
 constexpr int kColGroup = 128; // projection columns per sketch launch
 template <typename W>
 struct KmmArgs {
@@ -487,287 +486,8 @@ void launch_kmm_fast(int d, int kind, int mode, int nt, unsigned grid, cudaStrea
 }
 
 // ---------------------------------------------------------------------------
-// truncation: A ~ Q B^T with B = A^T Q; eig(B^T B) = W diag(lambda) W^T gives
-// the singular values of A's approximation, sqrt(lambda), and
-// A ~ (Q W_r)(B W_r)^T with the smallest r whose discarded sum of lambda fits
-// the tolerance left after the sampling residual.  Columns come out in
-// decreasing singular value, U = Q W_r orthonormal, |V_j| = sigma_j.
+// dense blocks
 // ---------------------------------------------------------------------------
-constexpr int kGramThreads = 256;
-
-// G = B^T B (k x k, FP64) into global memory at goff, 8x8 register tiles
-template <typename W>
-__global__ void __launch_bounds__(kGramThreads) k_gram_big(const Prob* probs, const ProbState* st, const W* ws,
-                                                           const long long* goff, double* G) {
-  __shared__ double Bs[16][kMaxCols + 1];
-  const int p = blockIdx.x;
-  const int k = st[p].k;
-  if (k <= 1 || k > kTruncMax) return;  // wider bases are kept as sampled
-  const Prob P = probs[p];
-  const W* B = ws + P.boff;
-  const int nt = (k + 7) / 8;
-  const int t = threadIdx.x;
-  const int ti = t / 16, tj = t % 16;  // tile (ti, tj) of up to 16 x 16 tiles
-  const bool active = ti < nt && tj < nt && ti <= tj;
-  double acc[8][8];
-#pragma unroll
-  for (int a = 0; a < 8; ++a)
-#pragma unroll
-    for (int b = 0; b < 8; ++b) acc[a][b] = 0.0;
-  for (int i0 = 0; i0 < P.n; i0 += 16) {
-    for (int e = t; e < 16 * k; e += kGramThreads) {
-      int ii = e % 16, j = e / 16;
-      Bs[ii][j] = (i0 + ii < P.n) ? (double)B[(size_t)j * ara_ld(P.n) + i0 + ii] : 0.0;
-    }
-    __syncthreads();
-    if (active) {
-      for (int ii = 0; ii < 16; ++ii) {
-        double x[8], y[8];
-#pragma unroll
-        for (int a = 0; a < 8; ++a) {
-          int ja = ti * 8 + a, jb = tj * 8 + a;
-          x[a] = ja < k ? Bs[ii][ja] : 0.0;
-          y[a] = jb < k ? Bs[ii][jb] : 0.0;
-        }
-#pragma unroll
-        for (int a = 0; a < 8; ++a)
-#pragma unroll
-          for (int b = 0; b < 8; ++b) acc[a][b] = fma(x[a], y[b], acc[a][b]);
-      }
-    }
-    __syncthreads();
-  }
-  if (active) {
-    double* g = G + goff[p];
-#pragma unroll
-    for (int a = 0; a < 8; ++a)
-#pragma unroll
-      for (int b = 0; b < 8; ++b) {
-        int ja = ti * 8 + a, jb = tj * 8 + b;
-        if (ja < k && jb < k) {
-          g[ja * k + jb] = acc[a][b];
-          g[jb * k + ja] = acc[a][b];
-        }
-      }
-  }
-}
-
-// Parallel cyclic Jacobi on G (k x k) in shared memory; the rotations are
-// accumulated into Wm (FP32).  Writes the truncated rank to st[p].r and the
-// leading r eigenvectors (columns in decreasing eigenvalue) to Wr (k x r, at
-// the same offset as G).
-__global__ void __launch_bounds__(kGramThreads) k_jacobi(const Prob* probs, ProbState* st, const long long* goff,
-                                                         const double* Gin, float* Wr, double tol2,
-                                                         double rbudget) {
-  extern __shared__ __align__(16) unsigned char jsm[];
-  const int p = blockIdx.x;
-  ProbState S = st[p];
-  const int k = S.k;
-  const int t = threadIdx.x;
-  if (k <= 1 || k > kTruncMax) {
-    // no truncation: W = identity, every column keeps its low part
-    for (int e = t; e < k * k; e += kGramThreads) Wr[goff[p] + e] = (e / k == e % k) ? 1.f : 0.f;
-    if (t == 0) {
-      st[p].r = k;
-      st[p].rhi = k;
-    }
-    return;
-  }
-  const int kp = (k + 1) & ~1;  // even size: an odd k gets a zero row and column
-  double* G = reinterpret_cast<double*>(jsm);              // [kp][kp]
-  float* Wm = reinterpret_cast<float*>(G + kp * kp);        // [kp][kp]
-  double* cs = reinterpret_cast<double*>(Wm + kp * kp);     // [kp/2][2]
-  int* pr = reinterpret_cast<int*>(cs + kp);                // [kp] tournament positions
-  int* order = pr + kp;                                     // [kp]
-  __shared__ double off_sh;
-  const double* g = Gin + goff[p];
-  for (int e = t; e < kp * kp; e += kGramThreads) {
-    int a = e / kp, b = e % kp;
-    G[e] = (a < k && b < k) ? g[a * k + b] : 0.0;
-    Wm[e] = a == b ? 1.f : 0.f;
-  }
-  for (int i = t; i < kp; i += kGramThreads) pr[i] = i;
-  __syncthreads();
-  double scale = 0;
-  for (int i = 0; i < k; ++i) scale += G[i * kp + i];
-  const int npairs = kp / 2;
-  for (int sweep = 0; sweep < 12; ++sweep) {
-    if (t == 0) off_sh = 0;
-    __syncthreads();
-    for (int step = 0; step < kp - 1; ++step) {
-      // pair i: (pr[i], pr[kp-1-i]); angles
-      for (int i = t; i < npairs; i += kGramThreads) {
-        int a = pr[i], b = pr[kp - 1 - i];
-        int pp = min(a, b), qq = max(a, b);
-        double apq = G[pp * kp + qq];
-        double c = 1, s = 0;
-        if (fabs(apq) > 1e-300 && fabs(apq) > 1e-18 * scale) {
-          double th = (G[qq * kp + qq] - G[pp * kp + pp]) / (2 * apq);
-          double tt = (th >= 0 ? 1.0 : -1.0) / (fabs(th) + sqrt(th * th + 1.0));
-          c = 1.0 / sqrt(tt * tt + 1.0);
-          s = tt * c;
-          atomicAdd(&off_sh, apq * apq);
-        }
-        cs[2 * i] = c;
-        cs[2 * i + 1] = s;
-      }
-      __syncthreads();
-      // rows
-      for (int e = t; e < npairs * kp; e += kGramThreads) {
-        int i = e / kp, j = e % kp;
-        int a = pr[i], b = pr[kp - 1 - i];
-        int pp = min(a, b), qq = max(a, b);
-        double c = cs[2 * i], s = cs[2 * i + 1];
-        double gp = G[pp * kp + j], gq = G[qq * kp + j];
-        G[pp * kp + j] = c * gp - s * gq;
-        G[qq * kp + j] = s * gp + c * gq;
-      }
-      __syncthreads();
-      // columns, and the accumulated rotation
-      for (int e = t; e < npairs * kp; e += kGramThreads) {
-        int i = e / kp, j = e % kp;
-        int a = pr[i], b = pr[kp - 1 - i];
-        int pp = min(a, b), qq = max(a, b);
-        double c = cs[2 * i], s = cs[2 * i + 1];
-        double gp = G[j * kp + pp], gq = G[j * kp + qq];
-        G[j * kp + pp] = c * gp - s * gq;
-        G[j * kp + qq] = s * gp + c * gq;
-        float wp = Wm[j * kp + pp], wq = Wm[j * kp + qq];
-        Wm[j * kp + pp] = (float)(c * wp - s * wq);
-        Wm[j * kp + qq] = (float)(s * wp + c * wq);
-      }
-      __syncthreads();
-      // next tournament round: keep position 0, rotate the rest
-      if (t == 0) {
-        int last = pr[kp - 1];
-        for (int i = kp - 1; i > 1; --i) pr[i] = pr[i - 1];
-        pr[1] = last;
-      }
-      __syncthreads();
-    }
-    if (off_sh <= 1e-26 * scale * scale) break;
-    __syncthreads();
-  }
-  // order by decreasing eigenvalue (rank by counting), then the rank
-  for (int i = t; i < k; i += kGramThreads) {
-    double li = G[i * kp + i];
-    int rk = 0;
-    for (int j = 0; j < k; ++j) {
-      double lj = G[j * kp + j];
-      rk += (lj > li) || (lj == li && j < i);
-    }
-    order[rk] = i;
-  }
-  __syncthreads();
-  __shared__ int r_sh;
-  if (t == 0) {
-    // discard the smallest eigenvalues while their sum fits the budget
-    const double ts2 = probs[p].tscale2;
-    double budget = tol2 * ts2 * S.normA2 - S.est;
-    double tail = 0;
-    int r = k;
-    if (S.converged && budget > 0) {
-      while (r > 1) {
-        double l = fmax(G[order[r - 1] * kp + order[r - 1]], 0.0);
-        if (tail + l > budget) break;
-        tail += l;
-        --r;
-      }
-    }
-    r_sh = r;
-    st[p].r = r;
-    // Mixed precision: column j of U V^T carries |u_j||v_j| = sigma_j; rounding
-    // both to BF16 perturbs it by at most ~2 * 2^-9 sigma_j.  The trailing
-    // columns whose rounding error fits rbudget keep only their BF16 high part.
-    int rhi = r;
-    if (rbudget > 0) {
-      double rt = 0;
-      const double c = 2.0 * 0x1p-18;  // (2^-9)^2 for each of u_j and v_j
-      while (rhi > 0) {
-        double l = fmax(G[order[rhi - 1] * kp + order[rhi - 1]], 0.0);
-        if (rt + c * l > rbudget * ts2 * S.normA2) break;
-        rt += c * l;
-        --rhi;
-      }
-    }
-    st[p].rhi = rhi;
-  }
-  __syncthreads();
-  const int r = r_sh;
-  float* w = Wr + goff[p];
-  for (int e = t; e < k * r; e += kGramThreads) {
-    int a = e % k, c = e / k;
-    w[c * k + a] = Wm[a * kp + order[c]];  // column c: eigenvector order[c]
-  }
-}
-
-// U = Q W_r (m x r), V = B W_r (n x r), FP32
-template <typename W>
-__global__ void k_pack_trunc(const Prob* probs, const ProbState* st, const W* ws, const long long* goff,
-                             const float* Wr, const long long* dst_u, const long long* dst_v, float* dst) {
-  const int p = blockIdx.x;
-  const int k = st[p].k, r = st[p].r;
-  if (dst_u[p] < 0 || r <= 0) return;
-  const Prob P = probs[p];
-  if (k > kTruncMax) {  // kept as sampled (W = I): U = Q, V = B, a copy
-    for (int side = 0; side < 2; ++side) {
-      const int rows = side ? P.n : P.m, ld = ara_ld(rows);
-      const W* src = ws + (side ? P.boff : P.qoff);
-      float* out = dst + (side ? dst_v[p] : dst_u[p]);
-      for (size_t e = threadIdx.x; e < (size_t)rows * r; e += blockDim.x)
-        out[e] = (float)src[e / rows * ld + e % rows];
-    }
-    return;
-  }
-  const float* w = Wr + goff[p];
-  __shared__ float ws_sh[kMaxCols * 32];
-  const int rc = min(r, 32);
-  for (int c0 = 0; c0 < r; c0 += 32) {
-    const int nc = min(32, r - c0);
-    __syncthreads();
-    for (int e = threadIdx.x; e < k * nc; e += blockDim.x) ws_sh[e] = w[(size_t)(c0 + e / k) * k + e % k];
-    __syncthreads();
-    for (int side = 0; side < 2; ++side) {
-      const int rows = side ? P.n : P.m, ld = ara_ld(rows);
-      const W* src = ws + (side ? P.boff : P.qoff);
-      float* out = dst + (side ? dst_v[p] : dst_u[p]);
-      for (int i = threadIdx.x; i < rows; i += blockDim.x) {
-        float acc[32];
-        for (int c = 0; c < nc; ++c) acc[c] = 0.f;
-        for (int a = 0; a < k; ++a) {
-          float x = (float)src[(size_t)a * ld + i];
-          for (int c = 0; c < nc; ++c) acc[c] = fmaf(x, ws_sh[c * k + a], acc[c]);
-        }
-        for (int c = 0; c < nc; ++c) out[(size_t)(c0 + c) * rows + i] = acc[c];
-      }
-    }
-  }
-  (void)rc;
-}
-
-size_t jacobi_smem(int kmax) {
-  int kp = (kmax + 1) & ~1;
-  return sizeof(double) * kp * kp + sizeof(float) * kp * kp + sizeof(double) * kp + sizeof(int) * 2 * kp + 64;
-}
-
-
-// ---------------------------------------------------------------------------
-// packing and dense blocks
-// ---------------------------------------------------------------------------
-struct PackItem {
-  long long src_q, src_b;  // workspace offsets
-  long long dst_u, dst_v;  // offsets in the chunk
-  int m, n, k;
-};
-
-template <typename W>
-__global__ void k_pack(const PackItem* items, int nitems, const W* ws, float* dst) {
-  const PackItem it = items[blockIdx.x];
-  size_t nu = (size_t)it.m * it.k, nv = (size_t)it.n * it.k;
-  for (size_t e = threadIdx.x; e < nu; e += blockDim.x) dst[it.dst_u + e] = (float)ws[it.src_q + e];
-  for (size_t e = threadIdx.x; e < nv; e += blockDim.x) dst[it.dst_v + e] = (float)ws[it.src_b + e];
-}
-
 struct DenseItem {
   int r0, m, c0, n;
   long long off;
@@ -1172,36 +892,17 @@ hm_status hmatrix_build(hm_kdtree t, hm_structure s, const double* d_points, con
       HM_LAUNCH_CHECK();
 
       tr.mark("projection", stream, nb, 3);
-      // ---- truncation: Gram of B, Jacobi eigen, truncated rank -------------
+      // ---- truncation: Gram of B, its eigenpairs, truncated rank ------------
       HM_CUDA(cudaMemcpyAsync(hst.data(), dst.p, sizeof(ProbState) * nb, cudaMemcpyDeviceToHost, stream));
       HM_CUDA(cudaStreamSynchronize(stream));
-      std::vector<long long> goff(nb);
-      size_t gtot = 0;
-      int kbig = 2;
-      for (int i = 0; i < nb; ++i) {
-        goff[i] = (long long)gtot;
-        gtot += (size_t)hst[i].k * hst[i].k;
-        if (hst[i].k <= kTruncMax) kbig = std::max(kbig, hst[i].k);
-      }
-      DevBuf<long long> dgoff;
-      DevBuf<double> Gbuf;
-      DevBuf<float> Wr;
-      if ((st = dgoff.alloc_async(nb, stream)) || (st = Gbuf.alloc_async(std::max<size_t>(gtot, 1), stream)) ||
-          (st = Wr.alloc_async(std::max<size_t>(gtot, 1), stream)))
-        return st;
-      HM_CUDA(cudaMemcpyAsync(dgoff.p, goff.data(), sizeof(long long) * nb, cudaMemcpyHostToDevice, stream));
-      k_gram_big<W><<<nb, kGramThreads, 0, stream>>>(dprobs.p, dst.p, ws.p, dgoff.p, Gbuf.p);
-      HM_LAUNCH_CHECK();
-      HM_CUDA(cudaFuncSetAttribute(k_jacobi, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   (int)jacobi_smem(kTruncMax)));
       // error budget (relative, squared): sampling residual <= 0.09 tol^2 (the
       // stopping test), truncation 0.45 tol^2 (FP32 form) or 0.35 tol^2 plus
       // 0.15 tol^2 of BF16 rounding (mixed form)
       const bool mixed = opt.precision == HM_PREC_MIXED;
-      k_jacobi<<<nb, kGramThreads, jacobi_smem(kbig), stream>>>(
-          dprobs.p, dst.p, dgoff.p, Gbuf.p, Wr.p, (mixed ? 0.35 : 0.45) * opt.tol * opt.tol,
-          mixed ? 0.15 * opt.tol * opt.tol : 0.0);
-      HM_LAUNCH_CHECK();
+      TruncWork tw;
+      if ((st = trunc_rank<W>(bp, hst, dprobs.p, dst.p, ws.p, (mixed ? 0.35 : 0.45) * opt.tol * opt.tol,
+                              mixed ? 0.15 * opt.tol * opt.tol : 0.0, &tw, stream)))
+        return st;
       HM_CUDA(cudaMemcpyAsync(hst.data(), dst.p, sizeof(ProbState) * nb, cudaMemcpyDeviceToHost, stream));
       HM_CUDA(cudaStreamSynchronize(stream));
 
@@ -1280,8 +981,10 @@ hm_status hmatrix_build(hm_kdtree t, hm_structure s, const double* d_points, con
       if ((st = ddu.alloc_async(nb, stream)) || (st = ddv.alloc_async(nb, stream))) return st;
       HM_CUDA(cudaMemcpyAsync(ddu.p, du.data(), sizeof(long long) * nb, cudaMemcpyHostToDevice, stream));
       HM_CUDA(cudaMemcpyAsync(ddv.p, dv.data(), sizeof(long long) * nb, cudaMemcpyHostToDevice, stream));
-      k_pack_trunc<W><<<nb, 256, 0, stream>>>(dprobs.p, dst.p, ws.p, dgoff.p, Wr.p, ddu.p, ddv.p, chunk.p);
-      HM_LAUNCH_CHECK();
+      static_assert(kTR == 64, "trunc_pack's tiles are the sketch's row tiles");
+      if ((st = trunc_pack<W>(dprobs.p, dst.p, ws.p, tw, drows.p, items_rows.size(), dcols.p, items_cols.size(), ddu.p,
+                              ddv.p, chunk.p, stream)))
+        return st;
       if (!dens.empty()) {
         if ((st = ddi.alloc_async(dens.size(), stream))) return st;
         HM_CUDA(cudaMemcpyAsync(ddi.p, dens.data(), sizeof(DenseItem) * dens.size(), cudaMemcpyHostToDevice,

@@ -89,4 +89,13 @@ __device__ __forceinline__ void mma_bf16(float (&c)[4], uint32_t a0, uint32_t a1
       : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
+// ---- FP64 m8n8k4 (lane = 4*g + t) ------------------------------------------
+//   A (8x4): a = A[g][t];  B (4x8): b = B[t][g];  C (8x8): c0, c1 = C[g][2t], C[g][2t+1]
+__device__ __forceinline__ void mma_f64(double (&d)[2], double a, double b) {
+  asm volatile(
+      "mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
+      : "+d"(d[0]), "+d"(d[1])
+      : "d"(a), "d"(b));
+}
+
 }  // namespace hm

@@ -37,6 +37,7 @@
 #include <algorithm>
 
 #include "hm_ara.h"
+#include "hm_mma.cuh"
 
 namespace hm {
 namespace {
@@ -61,13 +62,6 @@ struct Vec<double> {
   static __device__ __forceinline__ void get(const T& v, double (&x)[2]) { x[0] = v.x, x[1] = v.y; }
   static __device__ __forceinline__ T put(const double (&x)[2]) { return make_double2(x[0], x[1]); }
 };
-
-__device__ __forceinline__ void mma_f64(double (&d)[2], double a, double b) {
-  asm volatile(
-      "mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
-      : "+d"(d[0]), "+d"(d[1])
-      : "d"(a), "d"(b));
-}
 
 // The ten 8 x 8 tiles of the upper triangle of a 32 x 32 Gram matrix, dealt to
 // four warps (three, three, two, two).
