@@ -106,10 +106,10 @@ extern "C" hm_status hm_autotune(hm_hmatrix h, int nrhs, const char* cache_path,
     std::vector<Choice> cand;
     if (is_mixed(h)) {
       for (int ring : {1, 0})
-        for (int ch : {16, 32, 64, 128})
+        for (int ch : {8, 16, 32, 64, 128})
           for (int g : {4, 8}) cand.push_back(Choice{ch, g, ring});
     } else {
-      for (int ch : {16, 32, 64, 128})
+      for (int ch : {8, 16, 32, 64, 128})
         for (int g : {2, 4}) cand.push_back(Choice{ch, g, 0});
       for (int r : {256, 1024}) cand.push_back(Choice{r, 0, 0});
     }

@@ -23,6 +23,7 @@
 //   {T[c=t][r=g], T[t+4][g], T[t][g+8], T[t+4][g+8]} (c column, r right-hand
 //   side): phase 2's two B fragments in one 16-byte load.
 #include <algorithm>
+#include <type_traits>
 #include <vector>
 
 #include "hm_hmatrix.h"
@@ -81,7 +82,8 @@ __device__ __forceinline__ int2 fp_tslot_pair(const int* __restrict__ tslot, lon
 __global__ void __launch_bounds__(128) k_fp_split_x(const float* __restrict__ X, int ldx, int nr, int num_tiles,
                                                     const int* __restrict__ tile_leaf,
                                                     const int* __restrict__ leaf_tile0,
-                                                    const int* __restrict__ leaf_off, uint4* __restrict__ Xf) {
+                                                    const int* __restrict__ leaf_off, const int* __restrict__ perm,
+                                                    uint4* __restrict__ Xf) {
   __shared__ float xs[4][16][33];
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int G = blockIdx.x * 4 + w;
@@ -89,8 +91,9 @@ __global__ void __launch_bounds__(128) k_fp_split_x(const float* __restrict__ X,
   const int x = tile_leaf[G];
   const int row = leaf_off[x] + 32 * (G - leaf_tile0[x]) + lane;
   const bool ok = row < leaf_off[x + 1];
+  const int src = ok && perm ? __ldg(perm + row) : row;  // X in the points' original order
 #pragma unroll
-  for (int r = 0; r < 16; ++r) xs[w][r][lane] = (ok && r < nr) ? __ldg(X + (size_t)r * ldx + row) : 0.f;
+  for (int r = 0; r < 16; ++r) xs[w][r][lane] = (ok && r < nr) ? __ldg(X + (size_t)r * ldx + src) : 0.f;
   __syncwarp();
   const int g = lane >> 2, t = lane & 3;
 #pragma unroll
@@ -223,13 +226,14 @@ __global__ void k_fp_reduce(const int2* __restrict__ mtiles, long long nmt, cons
 // ---- phase 2 ----------------------------------------------------------------
 // acc[mt][nb] += A (rows 16 mt.., 8 columns; hi / lo) B (8 columns x right-hand
 // sides 8 nb..; hi / lo)
-__device__ __forceinline__ void fp_p2_step(float (&acc)[2][2][4], const uint32_t (&ah)[2][4],
+template <int NB>
+__device__ __forceinline__ void fp_p2_step(float (&acc)[2][NB][4], const uint32_t (&ah)[2][4],
                                            const uint32_t (&al)[2][4], const uint32_t (&bh)[2][2],
                                            const uint32_t (&bl)[2][2]) {
 #pragma unroll
   for (int mt = 0; mt < 2; ++mt)
 #pragma unroll
-    for (int nb = 0; nb < 2; ++nb) {
+    for (int nb = 0; nb < NB; ++nb) {
       float d[4] = {0.f, 0.f, 0.f, 0.f};
       mma_tf32(d, al[mt][0], al[mt][1], al[mt][2], al[mt][3], bh[nb][0], bh[nb][1]);
       mma_tf32(d, ah[mt][0], ah[mt][1], ah[mt][2], ah[mt][3], bl[nb][0], bl[nb][1]);
@@ -238,51 +242,68 @@ __device__ __forceinline__ void fp_p2_step(float (&acc)[2][2][4], const uint32_t
     }
 }
 
-// One warp per global row tile (32 rows of one leaf), as the mixed form's
-// phase 2: every ancestor cluster's panel rows times its T, then the dense
-// blocks of the leaf row.
-__global__ void __launch_bounds__(32, 24) k_fp_p2(int tile0, int tile_end, int depth,
-                                                  const int* __restrict__ tile_leaf,
-                                                  const int* __restrict__ leaf_tile0,
-                                                  const int* __restrict__ leaf_off, const int* __restrict__ pan_of,
-                                                  const MxPanel* __restrict__ panels,
-                                                  const uint4* __restrict__ store, const float* __restrict__ T,
-                                                  const int* __restrict__ leaf_dptr,
-                                                  const int* __restrict__ leaf_dblk, const MxDense* __restrict__ dense,
-                                                  const uint4* __restrict__ Xf, float* __restrict__ Y, int ldy,
-                                                  int nr) {
+// One row tile (32 rows of one leaf) per CTA: every ancestor cluster's panel
+// rows times its T, then the dense blocks of the leaf row.  NB: halves of 8
+// right-hand sides (a pass of up to 8 multiplies one).  SP warps share the row
+// tile's column tiles (its sources laid end to end, cut into SP equal runs)
+// and their sums are added in warp order; SP = 1: one warp, 24 per SM.
+template <int NB, int SP>
+__global__ void __launch_bounds__(32 * SP, SP == 1 ? 24 : 16 / SP)
+    k_fp_p2(int tile0, int tile_end, int depth, const int* __restrict__ tile_leaf, const int* __restrict__ leaf_tile0,
+            const int* __restrict__ leaf_off, const int* __restrict__ pan_of, const MxPanel* __restrict__ panels,
+            const uint4* __restrict__ store, const float* __restrict__ T, const int* __restrict__ leaf_dptr,
+            const int* __restrict__ leaf_dblk, const MxDense* __restrict__ dense, const uint4* __restrict__ Xf,
+            const int* __restrict__ perm, float* __restrict__ Y, int ldy, int nr) {
+  constexpr int NA = 2 * NB * 4;  // sums per lane
+  __shared__ float red[SP > 1 ? SP * NA * 32 : 1];
   const int G = tile0 + blockIdx.x;
   if (G >= tile_end) return;
-  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int x = tile_leaf[G];
-  float acc[2][2][4];
+  float acc[2][NB][4];
 #pragma unroll
   for (int mt = 0; mt < 2; ++mt)
 #pragma unroll
-    for (int nb = 0; nb < 2; ++nb) acc[mt][nb][0] = acc[mt][nb][1] = acc[mt][nb][2] = acc[mt][nb][3] = 0.f;
+    for (int nb = 0; nb < NB; ++nb) acc[mt][nb][0] = acc[mt][nb][1] = acc[mt][nb][2] = acc[mt][nb][3] = 0.f;
   // every ancestor's panel descriptor at once (lane l - 1 holds level l's)
-  int my_p = -1, my_nct = 0;
+  int my_nct = 0;
   long long my_u = 0, my_t = 0;
   if (lane < depth) {
     const int l = lane + 1;
-    my_p = __ldg(pan_of + (1 << l) - 1 + (x >> (depth - l)));
-    if (my_p >= 0) {
-      const MxPanel P = panels[my_p];
+    const int p = __ldg(pan_of + (1 << l) - 1 + (x >> (depth - l)));
+    if (p >= 0) {
+      const MxPanel P = panels[p];
       my_u = P.hi2 + (long long)(G - P.tile0) * P.nct * 2;
       my_t = P.t0;
       my_nct = P.nct;
     }
   }
+  const int d0 = leaf_dptr[x], d1 = leaf_dptr[x + 1];
+  // this warp's run [lo, hi) of the row tile's column tiles
+  int lo = 0, hi = 0, my_end = 0;
+  if (SP > 1) {
+    my_end = warp_scan(my_nct, lane);
+    int total = __shfl_sync(0xffffffffu, my_end, 31);
+    for (int q = d0; q < d1; q += 32)
+      total += __reduce_add_sync(0xffffffffu, q + lane < d1 ? dense[leaf_dblk[q + lane]].nct : 0);
+    lo = (int)((long long)total * warp / SP);
+    hi = (int)((long long)total * (warp + 1) / SP);
+  }
   for (int l = 1; l <= depth; ++l) {
-    const int p = __shfl_sync(0xffffffffu, my_p, l - 1);
-    if (p < 0) continue;
+    int c1 = __shfl_sync(0xffffffffu, my_nct, l - 1), c0 = 0;
+    if (c1 == 0) continue;
+    if (SP > 1) {
+      const int at = __shfl_sync(0xffffffffu, my_end, l - 1) - c1;
+      c0 = max(0, lo - at);
+      c1 = min(c1, hi - at);
+      if (c0 >= c1) continue;
+    }
     const long long ou = __shfl_sync(0xffffffffu, my_u, l - 1);
     const long long ot = __shfl_sync(0xffffffffu, my_t, l - 1);
-    const int nct = __shfl_sync(0xffffffffu, my_nct, l - 1);
     const uint4* up = store + ou * 32 + lane;
     const uint4* tp = reinterpret_cast<const uint4*>(T + ot * 128) + lane;
-#pragma unroll 2
-    for (int ct = 0; ct < nct; ++ct) {
+#pragma unroll(SP == 1 ? 2 : 4)
+    for (int ct = c0; ct < c1; ++ct) {
       const uint4 a0 = __ldcs(up + (2 * ct) * 32), a1 = __ldcs(up + (2 * ct + 1) * 32);
       const uint4 tq = __ldg(tp + ct * 32);
       uint32_t ah[2][4], al[2][4], th[4], tl[4];
@@ -291,41 +312,68 @@ __global__ void __launch_bounds__(32, 24) k_fp_p2(int tile0, int tile_end, int d
       split4(tq, th, tl);
       const uint32_t bh[2][2] = {{th[0], th[1]}, {th[2], th[3]}};
       const uint32_t bl[2][2] = {{tl[0], tl[1]}, {tl[2], tl[3]}};
-      fp_p2_step(acc, ah, al, bh, bl);
+      fp_p2_step<NB>(acc, ah, al, bh, bl);
     }
   }
-  for (int q = leaf_dptr[x]; q < leaf_dptr[x + 1]; ++q) {
-    const MxDense D = dense[leaf_dblk[q]];
-    const long long rt = G - D.row_tile0;
-    const uint4* dp = store + (D.hi + rt * D.nct * 2) * 32 + lane;
-    for (int ct = 0; ct < D.nct; ++ct) {
-      const uint4 a0 = __ldcs(dp + (2 * ct) * 32), a1 = __ldcs(dp + (2 * ct + 1) * 32);
-      const size_t xt = ((size_t)(D.col_tile0 + (ct >> 2)) * 8 + (ct & 3)) * 32 + lane;
-      const uint4 xh = __ldg(Xf + xt), xl = __ldg(Xf + xt + 128);
-      uint32_t ah[2][4], al[2][4];
-      split4(a0, ah[0], al[0]);
-      split4(a1, ah[1], al[1]);
-      const uint32_t bh[2][2] = {{xh.x, xh.z}, {xh.y, xh.w}};
-      const uint32_t bl[2][2] = {{xl.x, xl.z}, {xl.y, xl.w}};
-      fp_p2_step(acc, ah, al, bh, bl);
+  int at = SP > 1 ? __shfl_sync(0xffffffffu, my_end, 31) : 0;
+  for (int q0 = d0; q0 < d1; q0 += 32) {
+    // up to 32 dense blocks' descriptors at once
+    long long my_d = 0;
+    int my_x = 0, my_c = 0, my_e = 0;
+    if (q0 + lane < d1) {
+      const MxDense D = dense[leaf_dblk[q0 + lane]];
+      my_d = D.hi + (long long)(G - D.row_tile0) * D.nct * 2;
+      my_x = D.col_tile0;
+      my_c = D.nct;
+    }
+    if (SP > 1) my_e = at + warp_scan(my_c, lane);
+    const int nq = min(32, d1 - q0);
+    for (int q = 0; q < nq; ++q) {
+      int c1 = __shfl_sync(0xffffffffu, my_c, q), c0 = 0;
+      if (SP > 1) {
+        const int a = __shfl_sync(0xffffffffu, my_e, q) - c1;
+        c0 = max(0, lo - a);
+        c1 = min(c1, hi - a);
+        if (c0 >= c1) continue;
+      }
+      const uint4* dp = store + __shfl_sync(0xffffffffu, my_d, q) * 32 + lane;
+      const int xt0 = __shfl_sync(0xffffffffu, my_x, q);
+#pragma unroll(SP == 1 ? 1 : 4)
+      for (int ct = c0; ct < c1; ++ct) {
+        const uint4 a0 = __ldcs(dp + (2 * ct) * 32), a1 = __ldcs(dp + (2 * ct + 1) * 32);
+        const size_t xt = ((size_t)(xt0 + (ct >> 2)) * 8 + (ct & 3)) * 32 + lane;
+        const uint4 xh = __ldg(Xf + xt), xl = __ldg(Xf + xt + 128);
+        uint32_t ah[2][4], al[2][4];
+        split4(a0, ah[0], al[0]);
+        split4(a1, ah[1], al[1]);
+        const uint32_t bh[2][2] = {{xh.x, xh.z}, {xh.y, xh.w}};
+        const uint32_t bl[2][2] = {{xl.x, xl.z}, {xl.y, xl.w}};
+        fp_p2_step<NB>(acc, ah, al, bh, bl);
+      }
+    }
+    if (SP > 1) at = __shfl_sync(0xffffffffu, my_e, 31);
+  }
+  const int base = leaf_off[x] + 32 * (G - leaf_tile0[x]), lim = leaf_off[x + 1];
+  // sum i of lane L: rows 16 mt + g (+ 8), column 8 nb + 2 t (+ 1) of C fragment (mt, nb)
+  auto store_y = [&](int i, int L, float v) {
+    const int row = base + 16 * (i / (4 * NB)) + (L >> 2) + 8 * ((i >> 1) & 1);
+    const int c = 8 * ((i >> 2) % NB) + 2 * (L & 3) + (i & 1);
+    if (row < lim && c < nr) Y[(size_t)c * ldy + (perm ? __ldg(perm + row) : row)] = v;
+  };
+  if (SP == 1) {
+#pragma unroll
+    for (int i = 0; i < NA; ++i) store_y(i, lane, acc[i / (4 * NB)][(i >> 2) % NB][i & 3]);
+  } else {
+#pragma unroll
+    for (int i = 0; i < NA; ++i) red[(warp * NA + i) * 32 + lane] = acc[i / (4 * NB)][(i >> 2) % NB][i & 3];
+    __syncthreads();
+    for (int e = threadIdx.x; e < NA * 32; e += 32 * SP) {
+      float v = red[e];
+#pragma unroll
+      for (int w = 1; w < SP; ++w) v += red[w * NA * 32 + e];
+      store_y(e >> 5, e & 31, v);
     }
   }
-  const int base = leaf_off[x] + 32 * (G - leaf_tile0[x]);
-  const int lim = leaf_off[x + 1];
-#pragma unroll
-  for (int mt = 0; mt < 2; ++mt)
-#pragma unroll
-    for (int nb = 0; nb < 2; ++nb) {
-      const int ra = base + 16 * mt + g, rb = ra + 8, c = 8 * nb + 2 * t;
-      if (c < nr) {
-        if (ra < lim) Y[(size_t)c * ldy + ra] = acc[mt][nb][0];
-        if (rb < lim) Y[(size_t)c * ldy + rb] = acc[mt][nb][2];
-      }
-      if (c + 1 < nr) {
-        if (ra < lim) Y[(size_t)(c + 1) * ldy + ra] = acc[mt][nb][1];
-        if (rb < lim) Y[(size_t)(c + 1) * ldy + rb] = acc[mt][nb][3];
-      }
-    }
 }
 
 // ---- conversion (build time) ------------------------------------------------
@@ -459,7 +507,7 @@ hm_status fp32_convert(hm_hmatrix_s* h, const std::vector<const float*>& colsrc,
 // One pass of nr <= 16 right-hand sides in tree order; scratch holds
 // scratch_floats(1) floats: X fragments, chunk partials, T.
 hm_status fp32_run_panel(hm_hmatrix_s* h, int nr, const float* X, int ldx, float* Y, int ldy, float* scratch,
-                         cudaStream_t s, KernelMarks* km) {
+                         const int* perm, cudaStream_t s, KernelMarks* km) {
   MxPlan& M = h->mx;
   if (nr < 1 || nr > 16) return fail(HM_ERR_INVALID, "FP32 panel product: a pass holds 1 to 16 right-hand sides");
   uint4* Xf = reinterpret_cast<uint4*>(scratch);
@@ -469,7 +517,7 @@ hm_status fp32_run_panel(hm_hmatrix_s* h, int nr, const float* X, int ldx, float
   const long long xbytes = 4ll * h->n * 16 * 2;  // the X fragments, hi + lo
   if (M.num_tiles > 0) {
     k_fp_split_x<<<(M.num_tiles + 3) / 4, 128, 0, s>>>(X, ldx, nr, M.num_tiles, M.tile_leaf.p, M.leaf_tile0.p,
-                                                       leaf_off, Xf);
+                                                       leaf_off, perm, Xf);
     HM_LAUNCH_CHECK();
     if (km) km->mark("k_fp_split_x", 4ll * h->n * nr + xbytes, s);
   }
@@ -485,13 +533,29 @@ hm_status fp32_run_panel(hm_hmatrix_s* h, int nr, const float* X, int ldx, float
     if (km) km->mark("k_fp_reduce", 512ll * M.s_tiles + 512ll * M.nmt, s);
   }
   if (M.p2_tiles > 0) {
-    k_fp_p2<<<(unsigned)M.p2_tiles, 32, 0, s>>>(M.p2_tile0, M.p2_tile0 + M.p2_tiles, h->depth, M.tile_leaf.p,
-                                                M.leaf_tile0.p, leaf_off, M.pan_of.p, M.panels.p, M.store.p, T,
-                                                M.leaf_dptr.p, M.leaf_dblk.p, M.dense.p, Xf, Y, ldy, nr);
+    auto p2 = [&](auto nb, auto sp) {
+      constexpr int NB = decltype(nb)::value, SP = decltype(sp)::value;
+      k_fp_p2<NB, SP><<<(unsigned)M.p2_tiles, 32 * SP, 0, s>>>(
+          M.p2_tile0, M.p2_tile0 + M.p2_tiles, h->depth, M.tile_leaf.p, M.leaf_tile0.p, leaf_off, M.pan_of.p,
+          M.panels.p, M.store.p, T, M.leaf_dptr.p, M.leaf_dblk.p, M.dense.p, Xf, perm, Y, ldy, nr);
+    };
+    auto p2_shared = [&](auto nb) {
+      const int sp = p2_share(M.p2_tiles, 6000);
+      if (sp == 8)
+        p2(nb, std::integral_constant<int, 8>{});
+      else if (sp == 4)
+        p2(nb, std::integral_constant<int, 4>{});
+      else
+        p2(nb, std::integral_constant<int, 1>{});
+    };
+    if (nr <= 8)
+      p2_shared(std::integral_constant<int, 1>{});
+    else
+      p2_shared(std::integral_constant<int, 2>{});
     HM_LAUNCH_CHECK();
     if (km) km->mark("k_fp_p2", M.bytes_p2 + xbytes + 4ll * h->n * nr, s);
   }
-  if (h->diag_fly) HM_TRY(diag_fly_panel(h, nr, X, ldx, Y, ldy, s, km));
+  if (h->diag_fly) HM_TRY(diag_fly_panel(h, nr, X, ldx, Y, ldy, s, km));  // (perm is null then)
   return HM_OK;
 }
 

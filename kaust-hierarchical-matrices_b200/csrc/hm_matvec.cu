@@ -31,7 +31,7 @@
 // holds this array until the process exits.  Host code must not take its
 // address directly (on the host the name is only a stand-in); the device
 // address comes from cudaGetSymbolAddress, once per device.
-static __device__ __align__(256) float hm_noalloc_scratch[size_t(4) << 20];
+static __device__ __align__(256) float hm_noalloc_scratch[hm::kNoallocFloats];
 
 namespace hm {
 
@@ -354,9 +354,9 @@ __global__ void __launch_bounds__(kFlyT) k_diag_fly(const int* __restrict__ leaf
 // One pass of nr <= pass_width(h) right-hand sides (X, Y in tree order); T:
 // projection scratch (FP32 form: 16 x kpad per block, then the chunk
 // partials; mixed form: see mixed_run_panel).
-hm_status run_panel(hm_hmatrix h, int nr, const float* X, int ldx, float* Y, int ldy, float* T, cudaStream_t s,
-                    KernelMarks* km) {
-  if (h->mx.enabled) return mixed_run_panel(h, nr, X, ldx, Y, ldy, T, s, km);
+hm_status run_panel(hm_hmatrix h, int nr, const float* X, int ldx, float* Y, int ldy, float* T, const int* perm,
+                    cudaStream_t s, KernelMarks* km) {
+  if (h->mx.enabled) return mixed_run_panel(h, nr, X, ldx, Y, ldy, T, perm, s, km);
   MatvecPlan& P = h->plan;
   float* Tpart = T + P.t_floats;
   if (P.num_p1 > 0) {
@@ -534,7 +534,12 @@ hm_status hmatvec(hm_hmatrix h, int trans, int nrhs, const float* X, int ldx, fl
     int ldxt = ldx;
     float* Yt = Yout;
     int ldyt = ldy;
-    if (original_order) {
+    // the panel products read X and write Y through the permutation; the
+    // others (and diagonal blocks from coordinates, which read X after Y is
+    // written) work on permuted copies
+    const bool fused = h->mx.enabled && !h->diag_fly;
+    const int* perm = original_order && fused ? h->tree->perm.p : nullptr;
+    if (original_order && !fused) {
       k_gather_rows<<<592, 256, 0, stream>>>(Xin, ldx, h->tree->perm.p, n, nr, P.Xp.p);
       HM_LAUNCH_CHECK();
       Xt = P.Xp.p;
@@ -542,8 +547,8 @@ hm_status hmatvec(hm_hmatrix h, int trans, int nrhs, const float* X, int ldx, fl
       Yt = P.Yp.p;
       ldyt = n;
     }
-    HM_TRY(run_panel(h, nr, Xt, ldxt, Yt, ldyt, P.T.p, stream, nullptr));
-    if (original_order) {
+    HM_TRY(run_panel(h, nr, Xt, ldxt, Yt, ldyt, P.T.p, perm, stream, nullptr));
+    if (original_order && !fused) {
       k_scatter_rows<<<592, 256, 0, stream>>>(P.Yp.p, h->tree->perm.p, n, nr, Yout, ldy);
       HM_LAUNCH_CHECK();
     }
@@ -569,7 +574,7 @@ hm_status hmatvec_f64(hm_hmatrix h, int trans, int nrhs, const double* X, int ld
     const int nr = std::min(pass_width(h), nrhs - c0);
     k_narrow_rows<<<592, 256, 0, stream>>>(X + (size_t)c0 * ldx, ldx, perm, n, nr, P.Xp.p);
     HM_LAUNCH_CHECK();
-    HM_TRY(run_panel(h, nr, P.Xp.p, n, P.Yp.p, n, P.T.p, stream, nullptr));
+    HM_TRY(run_panel(h, nr, P.Xp.p, n, P.Yp.p, n, P.T.p, nullptr, stream, nullptr));
     k_widen_rows<<<592, 256, 0, stream>>>(P.Yp.p, perm, n, nr, Y + (size_t)c0 * ldy, ldy);
     HM_LAUNCH_CHECK();
     c0 += nr;
@@ -601,7 +606,6 @@ void matvec_bytes(hm_hmatrix h, int nrhs, long long* b_project, long long* b_exp
 
 namespace {
 
-constexpr size_t kNoallocScratchFloats = size_t(4) << 20;
 constexpr int kMaxDevices = 64;
 std::mutex g_noalloc_mu;
 float* g_noalloc_ptr[kMaxDevices] = {};
@@ -645,7 +649,7 @@ hm_status timed_panel(hm_hmatrix h, int nr, const float* X, int ldx, float* Y, i
   for (auto& x : km->ev) HM_CUDA(cudaEventCreate(&x));
   km->n = 0;
   HM_CUDA(cudaEventRecord(km->ev[0], s));
-  HM_TRY(run_panel(h, nr, X, ldx, Y, ldy, h->plan.T.p, s, km));
+  HM_TRY(run_panel(h, nr, X, ldx, Y, ldy, h->plan.T.p, nullptr, s, km));
   HM_CUDA(cudaEventSynchronize(km->ev[km->n]));
   return HM_OK;
 }
@@ -661,7 +665,7 @@ extern "C" hm_status hm_hmatvec_noalloc(hm_hmatrix h, int nrhs, const float* X, 
     return hm::fail(HM_ERR_INVALID, "hm_hmatvec_noalloc: bad vector arguments");
   hm::MatvecPlan& P = h->plan;
   const size_t need = h->mx.enabled ? (size_t)h->mx.scratch_floats() : (size_t)P.t_floats + (size_t)P.part_floats;
-  if (need > hm::kNoallocScratchFloats) {
+  if (need > (size_t)hm::kNoallocFloats) {
     const std::string what =
         !h->mx.enabled ? " floats of projection scratch for a 16-column pass of the FP32 form's per-block product "
                          "(16 per factor column, plus chunk partials)"
@@ -671,7 +675,7 @@ extern "C" hm_status hm_hmatvec_noalloc(hm_hmatrix h, int nrhs, const float* X, 
                            "fragments, plus chunk partials and projections)";
     return hm::fail(HM_ERR_UNSUPPORTED, "hm_hmatvec_noalloc: this matrix needs " + std::to_string(need) + what +
                                             "; the static scratch holds " +
-                                            std::to_string(hm::kNoallocScratchFloats) + " (16 MiB)");
+                                            std::to_string(hm::kNoallocFloats) + " (16 MiB)");
   }
   float* T = nullptr;
   HM_TRY(hm::noalloc_scratch(&T));
@@ -681,7 +685,7 @@ extern "C" hm_status hm_hmatvec_noalloc(hm_hmatrix h, int nrhs, const float* X, 
     // the scratch keeps the previous call's contents, which need no clearing:
     // every scratch word the pass reads (X fragments, chunk partials,
     // projections, padding columns as zeros) is written earlier in the pass
-    HM_TRY(hm::run_panel(h, nr, X + (size_t)c0 * ldx, ldx, Y + (size_t)c0 * ldy, ldy, T, s, nullptr));
+    HM_TRY(hm::run_panel(h, nr, X + (size_t)c0 * ldx, ldx, Y + (size_t)c0 * ldy, ldy, T, nullptr, s, nullptr));
     c0 += nr;
   }
   return HM_OK;

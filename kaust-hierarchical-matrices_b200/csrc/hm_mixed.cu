@@ -30,6 +30,7 @@
 // each short chain of MMAs goes into a zeroed temporary that is added to the
 // running FP32 sum with an ordinary FADD.
 #include <algorithm>
+#include <type_traits>
 #include <vector>
 
 #include "hm_hmatrix.h"
@@ -39,6 +40,8 @@
 namespace hm {
 namespace {
 
+template <int N>
+using kInt = std::integral_constant<int, N>;
 
 // A P1 tile (32 rows x 8 columns of a factor) keeps lane (g,t)'s 16 bytes
 // -- column g at rows rho(t, 0..7) -- at word 4 g + (t ^ ((g >> 1) & 3)): the
@@ -144,8 +147,8 @@ __device__ __forceinline__ int2 tslot_pair(const int* __restrict__ tslot, long l
 __global__ void __launch_bounds__(128) k_mx_split_x(const float* __restrict__ X, int ldx, int nr, int num_tiles,
                                                     const int* __restrict__ tile_leaf,
                                                     const int* __restrict__ leaf_tile0,
-                                                    const int* __restrict__ leaf_off, uint4* __restrict__ Xf,
-                                                    uint4* __restrict__ Xtc) {
+                                                    const int* __restrict__ leaf_off, const int* __restrict__ perm,
+                                                    uint4* __restrict__ Xf, uint4* __restrict__ Xtc) {
   __shared__ float xs[4][16][33];
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int G = blockIdx.x * 4 + w;
@@ -157,8 +160,9 @@ __global__ void __launch_bounds__(128) k_mx_split_x(const float* __restrict__ X,
   const int x = tile_leaf[G];
   const int row = leaf_off[x] + 32 * (G - leaf_tile0[x]) + lane;
   const bool ok = row < leaf_off[x + 1];
+  const int src = ok && perm ? __ldg(perm + row) : row;  // X in the points' original order
 #pragma unroll
-  for (int r = 0; r < 16; ++r) xs[w][r][lane] = (ok && r < nr) ? __ldg(X + (size_t)r * ldx + row) : 0.f;
+  for (int r = 0; r < 16; ++r) xs[w][r][lane] = (ok && r < nr) ? __ldg(X + (size_t)r * ldx + src) : 0.f;
   __syncwarp();
   if (Xtc) {  // this part's 16 right-hand sides x 4 K blocks (no fragments)
 #pragma unroll
@@ -593,31 +597,37 @@ __device__ __forceinline__ void mx_p2_step_hi(float (&acc)[2][2][4], const uint4
   }
 }
 
-// One warp per global row tile (32 rows of one leaf): every ancestor cluster's
-// panel rows times its T, then the dense blocks of the leaf row.
+// One row tile (32 rows of one leaf): every ancestor cluster's panel rows
+// times its T, then the dense blocks of the leaf row.
 // (one warp per CTA, 28 per SM, measured: the kernel is bound by loads in
 // flight, and a warp that finishes its row tile frees its slot at once)
 // With two halves of 16 right-hand sides every U tile is loaded once for both,
 // and the warp holds twice the accumulators (16 warps per SM, 128 registers).
 // WPC > 1 (passes of more than 32 right-hand sides): the CTA's warps take the
-// same row tile, warp w parts w NH .., and share its factor tiles through L1.
+// same row tile, part group w % WPC parts w NH .., and share its factor tiles
+// through L1.
+// SP > 1 (few row tiles, passes of up to 32): SP warps share the row tile's
+// sources.  A source step is one pair of column tiles; steps with low parts
+// count twice; the steps are laid end to end and warp s takes the s-th
+// of SP equal runs.  The warps' sums are added in order.
 constexpr int kP2PerSm = 28, kP2PerSm2 = 16;
-template <int NH, int WPC>
-__global__ void __launch_bounds__(32 * WPC, (NH == 1 ? kP2PerSm : kP2PerSm2) / WPC)
-    k_mx_p2(int tile0, int tile_end, int depth, const int* __restrict__ tile_leaf,
-                                               const int* __restrict__ leaf_tile0, const int* __restrict__ leaf_off,
-                                               const int* __restrict__ pan_of, const MxPanel* __restrict__ panels,
-                                               const uint4* __restrict__ store, const uint32_t* __restrict__ T,
-                                               const int* __restrict__ leaf_dptr, const int* __restrict__ leaf_dblk,
-                                               const MxDense* __restrict__ dense, const uint4* __restrict__ Xf,
-                                               float* __restrict__ Y, int ldy, int nr, long long xh_, long long th) {
+template <int NH, int WPC, int SP>
+__global__ void __launch_bounds__(32 * WPC * SP, (NH == 1 && SP == 1 ? kP2PerSm : kP2PerSm2) / (WPC * SP))
+    k_mx_p2(int tile0, int tile_end, int depth, const int* __restrict__ tile_leaf, const int* __restrict__ leaf_tile0,
+            const int* __restrict__ leaf_off, const int* __restrict__ pan_of, const MxPanel* __restrict__ panels,
+            const uint4* __restrict__ store, const uint32_t* __restrict__ T, const int* __restrict__ leaf_dptr,
+            const int* __restrict__ leaf_dblk, const MxDense* __restrict__ dense, const uint4* __restrict__ Xf,
+            const int* __restrict__ perm, float* __restrict__ Y, int ldy, int nr, long long xh_, long long th) {
+  constexpr int NA = NH * 16;  // sums per lane
+  __shared__ float red[SP > 1 ? SP * WPC * NA * 32 : 1];
   // global row tiles [tile0, tile_end): every tile, or a block-row shard's
   const int G = tile0 + blockIdx.x;
   if (G >= tile_end) return;
-  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const int lane = threadIdx.x & 31;
+  const int pg = (threadIdx.x >> 5) % WPC, sp = (threadIdx.x >> 5) / WPC;  // part group, share
   constexpr bool SH = WPC > 1;
   if (SH) {  // this warp's parts
-    const int h0 = (threadIdx.x >> 5) * NH;
+    const int h0 = pg * NH;
     T += h0 * th;
     Xf += h0 * xh_;
     Y += (size_t)16 * h0 * ldy;
@@ -635,14 +645,13 @@ __global__ void __launch_bounds__(32 * WPC, (NH == 1 ? kP2PerSm : kP2PerSm2) / W
   const uint4 z = make_uint4(0u, 0u, 0u, 0u);
   // every ancestor's panel descriptor at once (lane l - 1 holds level l's),
   // instead of a chain of dependent loads per level
-  int my_p = -1;
   long long my_u = 0, my_l = 0, my_t = 0;
   int my_nct = 0, my_nctl = 0;
   if (lane < depth) {
     const int l = lane + 1;
-    my_p = __ldg(pan_of + (1 << l) - 1 + (x >> (depth - l)));
-    if (my_p >= 0) {
-      const MxPanel P = panels[my_p];
+    const int p = __ldg(pan_of + (1 << l) - 1 + (x >> (depth - l)));
+    if (p >= 0) {
+      const MxPanel P = panels[p];
       const long long rt = G - P.tile0;
       my_u = P.hi2 + rt * P.nct;
       my_l = P.lo2 + rt * P.nctl;
@@ -651,20 +660,47 @@ __global__ void __launch_bounds__(32 * WPC, (NH == 1 ? kP2PerSm : kP2PerSm2) / W
       my_nctl = P.nctl;
     }
   }
+  const int d0 = leaf_dptr[x], d1 = leaf_dptr[x + 1];
+  // this warp's run [lo, hi) of the row tile's steps
+  int lo = 0, hi = 0, my_end = 0;
+  if (SP > 1) {
+    my_end = warp_scan(2 * ((my_nctl + 1) >> 1) + ((my_nct - my_nctl + 1) >> 1), lane);
+    int total = __shfl_sync(0xffffffffu, my_end, 31);
+    for (int q = d0; q < d1; q += 32)
+      total += __reduce_add_sync(0xffffffffu, q + lane < d1 ? dense[leaf_dblk[q + lane]].nct : 0);
+    lo = (int)((long long)total * sp / SP);
+    hi = (int)((long long)total * (sp + 1) / SP);
+  }
+  // first and last step, among n that weigh w each from position at on, of this warp's run
+  auto run = [&](int at, int n, int w, int& a, int& b) {
+    a = min(n, (max(0, lo - at) + w - 1) / w);
+    b = min(n, (max(0, hi - at) + w - 1) / w);
+  };
   for (int l = 1; l <= depth; ++l) {
-    const int p = __shfl_sync(0xffffffffu, my_p, l - 1);
-    if (p < 0) continue;
+    const int nct = __shfl_sync(0xffffffffu, my_nct, l - 1);
+    if (nct == 0) continue;
+    const int nctl = __shfl_sync(0xffffffffu, my_nctl, l - 1);
+    int la = 0, lb = nctl, ha = nctl, hb = nct;  // this warp's column tiles with and without low parts
+    if (SP > 1) {
+      const int nl = (nctl + 1) >> 1, nh = (nct - nctl + 1) >> 1;
+      const int at = __shfl_sync(0xffffffffu, my_end, l - 1) - 2 * nl - nh;
+      int a, b;
+      run(at, nl, 2, a, b);
+      la = 2 * a;
+      lb = min(nctl, 2 * b);
+      run(at + 2 * nl, nh, 1, a, b);
+      ha = nctl + 2 * a;
+      hb = min(nct, nctl + 2 * b);
+    }
     const long long ou = __shfl_sync(0xffffffffu, my_u, l - 1);
     const long long ol = __shfl_sync(0xffffffffu, my_l, l - 1);
     const long long ot = __shfl_sync(0xffffffffu, my_t, l - 1);
-    const int nct = __shfl_sync(0xffffffffu, my_nct, l - 1);
-    const int nctl = __shfl_sync(0xffffffffu, my_nctl, l - 1);
     const uint4* uh = store + ou * 32 + lane;
     const uint4* ul = store + ol * 32 + lane;
     // tiles with low parts: U (hi + lo) T (hi + lo)
     const uint4* tl = reinterpret_cast<const uint4*>(T + ot) + lane;
 #pragma unroll 2
-    for (int ct = 0; ct < nctl; ct += 2) {
+    for (int ct = la; ct < lb; ct += 2) {
       const bool two = ct + 1 < nctl;
       const uint4 h0 = ld_tile<SH>(uh + ct * 32);
       const uint4 h1 = two ? ld_tile<SH>(uh + (ct + 1) * 32) : z;
@@ -684,8 +720,8 @@ __global__ void __launch_bounds__(32 * WPC, (NH == 1 ? kP2PerSm : kP2PerSm2) / W
     }
     // tiles without: U_hi T_hi
     const uint2* tw = reinterpret_cast<const uint2*>(T + ot + (long long)nctl * 128) + lane;
-#pragma unroll 2
-    for (int ct = nctl; ct < nct; ct += 2) {
+#pragma unroll(SP == 1 ? 2 : 4)
+    for (int ct = ha; ct < hb; ct += 2) {
       const bool two = ct + 1 < nct;
       const uint4 h0 = ld_tile<SH>(uh + ct * 32);
       const uint4 h1 = two ? ld_tile<SH>(uh + (ct + 1) * 32) : z;
@@ -699,42 +735,73 @@ __global__ void __launch_bounds__(32 * WPC, (NH == 1 ? kP2PerSm : kP2PerSm2) / W
       }
     }
   }
-  for (int q = leaf_dptr[x]; q < leaf_dptr[x + 1]; ++q) {
-    const MxDense D = dense[leaf_dblk[q]];
-    const long long rt = G - D.row_tile0;
-    const uint4* dh = store + (D.hi + rt * D.nct) * 32 + lane;
-    const uint4* dl = store + (D.lo + rt * D.nct) * 32 + lane;
-    for (int ct = 0; ct < D.nct; ct += 2) {
-      const uint4 h0 = ld_tile<SH>(dh + ct * 32), h1 = ld_tile<SH>(dh + (ct + 1) * 32);
-      const uint4 l0 = ld_tile<SH>(dl + ct * 32), l1 = ld_tile<SH>(dl + (ct + 1) * 32);
-      const size_t xt = (size_t)(D.col_tile0 + (ct >> 2)) * 128 + (size_t)((ct >> 1) & 1) * 32 + lane;
+  int at = SP > 1 ? __shfl_sync(0xffffffffu, my_end, 31) : 0;
+  for (int q0 = d0; q0 < d1; q0 += 32) {
+    // up to 32 dense blocks' descriptors at once
+    long long my_dh = 0, my_dl = 0;
+    int my_x = 0, my_c = 0, my_e = 0;
+    if (q0 + lane < d1) {
+      const MxDense D = dense[leaf_dblk[q0 + lane]];
+      const long long rt = G - D.row_tile0;
+      my_dh = D.hi + rt * D.nct;
+      my_dl = D.lo + rt * D.nct;
+      my_x = D.col_tile0;
+      my_c = D.nct;
+    }
+    if (SP > 1) my_e = at + warp_scan(my_c, lane);
+    const int nq = min(32, d1 - q0);
+    for (int q = 0; q < nq; ++q) {
+      const int nct = __shfl_sync(0xffffffffu, my_c, q);
+      int ca = 0, cb = nct;  // this warp's column tiles (nct is a multiple of 4)
+      if (SP > 1) {
+        int a, b;
+        run(__shfl_sync(0xffffffffu, my_e, q) - nct, nct >> 1, 2, a, b);
+        ca = 2 * a;
+        cb = 2 * b;
+        if (ca >= cb) continue;
+      }
+      const uint4* dh = store + __shfl_sync(0xffffffffu, my_dh, q) * 32 + lane;
+      const uint4* dl = store + __shfl_sync(0xffffffffu, my_dl, q) * 32 + lane;
+      const int xt0 = __shfl_sync(0xffffffffu, my_x, q);
+#pragma unroll(SP == 1 ? 1 : 2)
+      for (int ct = ca; ct < cb; ct += 2) {
+        const uint4 h0 = ld_tile<SH>(dh + ct * 32), h1 = ld_tile<SH>(dh + (ct + 1) * 32);
+        const uint4 l0 = ld_tile<SH>(dl + ct * 32), l1 = ld_tile<SH>(dl + (ct + 1) * 32);
+        const size_t xt = (size_t)(xt0 + (ct >> 2)) * 128 + (size_t)((ct >> 1) & 1) * 32 + lane;
 #pragma unroll
-      for (int h = 0; h < NH; ++h) {
-        const uint4 xh = __ldg(Xf + h * xh_ + xt), xl = __ldg(Xf + h * xh_ + xt + 64);
-        const uint32_t bh[2][2] = {{xh.x, xh.z}, {xh.y, xh.w}};
-        const uint32_t bl[2][2] = {{xl.x, xl.z}, {xl.y, xl.w}};
-        mx_p2_step(acc[h], h0, h1, l0, l1, bh, bl, true);
+        for (int h = 0; h < NH; ++h) {
+          const uint4 xh = __ldg(Xf + h * xh_ + xt), xl = __ldg(Xf + h * xh_ + xt + 64);
+          const uint32_t bh[2][2] = {{xh.x, xh.z}, {xh.y, xh.w}};
+          const uint32_t bl[2][2] = {{xl.x, xl.z}, {xl.y, xl.w}};
+          mx_p2_step(acc[h], h0, h1, l0, l1, bh, bl, true);
+        }
       }
     }
+    if (SP > 1) at = __shfl_sync(0xffffffffu, my_e, 31);
   }
-  const int base = leaf_off[x] + 32 * (G - leaf_tile0[x]);
-  const int lim = leaf_off[x + 1];
+  const int base = leaf_off[x] + 32 * (G - leaf_tile0[x]), lim = leaf_off[x + 1];
+  // sum i of lane L: half i / 16, rows 16 mt + g (+ 8), column 8 nb + 2 t (+ 1) of C fragment (mt, nb)
+  auto store_y = [&](int i, int L, float v) {
+    const int row = base + 16 * ((i >> 3) & 1) + (L >> 2) + 8 * ((i >> 1) & 1);
+    const int c = 16 * (i >> 4) + 8 * ((i >> 2) & 1) + 2 * (L & 3) + (i & 1);
+    if (row < lim && c < nr) Y[(size_t)c * ldy + (perm ? __ldg(perm + row) : row)] = v;
+  };
+  if (SP == 1) {
 #pragma unroll
-  for (int h = 0; h < NH; ++h)
+    for (int i = 0; i < NA; ++i) store_y(i, lane, acc[i >> 4][(i >> 3) & 1][(i >> 2) & 1][i & 3]);
+  } else {
+    float* mine = red + (size_t)(sp * WPC + pg) * NA * 32;
 #pragma unroll
-    for (int mt = 0; mt < 2; ++mt)
+    for (int i = 0; i < NA; ++i) mine[i * 32 + lane] = acc[i >> 4][(i >> 3) & 1][(i >> 2) & 1][i & 3];
+    __syncthreads();
+    const float* first = red + (size_t)pg * NA * 32;
+    for (int i = sp; i < NA; i += SP) {
+      float v = first[i * 32 + lane];
 #pragma unroll
-      for (int nb = 0; nb < 2; ++nb) {
-        const int ra = base + 16 * mt + g, rb = ra + 8, c = 16 * h + 8 * nb + 2 * t;
-        if (c < nr) {
-          if (ra < lim) Y[(size_t)c * ldy + ra] = acc[h][mt][nb][0];
-          if (rb < lim) Y[(size_t)c * ldy + rb] = acc[h][mt][nb][2];
-        }
-        if (c + 1 < nr) {
-          if (ra < lim) Y[(size_t)(c + 1) * ldy + ra] = acc[h][mt][nb][1];
-          if (rb < lim) Y[(size_t)(c + 1) * ldy + rb] = acc[h][mt][nb][3];
-        }
-      }
+      for (int w = 1; w < SP; ++w) v += first[(w * WPC * NA + i) * 32 + lane];
+      store_y(i, lane, v);
+    }
+  }
 }
 
 // ---- conversion (build time) ------------------------------------------------
@@ -1021,6 +1088,18 @@ hm_status mixed_build(hm_hmatrix_s* h, const std::vector<MxPair>& pairs, const s
   M.store_tiles = tiles;
   HM_TRY(M.store.alloc((size_t)std::max<long long>(tiles, 1) * 32));
   M.h_panels = panels;
+  p1_shape(M.num_tiles, &M.chunk_tiles, &M.group_tiles);
+  // short chunks leave more partials: a matrix whose 16-column pass fits the
+  // allocation-free product's scratch with the longest ones keeps fitting
+  auto pass_floats = [&](int chunk) {
+    long long st = 0;
+    for (const MxPanel& P : panels)
+      if (P.nrt > chunk) st += (long long)((P.nrt + chunk - 1) / chunk) * P.nct;
+    return ((long long)M.num_tiles * (f32 ? 8 : 4) + st) * 128 + t_words;
+  };
+  if (pass_floats(128) <= kNoallocFloats)
+    while (M.chunk_tiles < 128 && pass_floats(M.chunk_tiles) > kNoallocFloats)
+      M.chunk_tiles = std::min(128, 2 * M.chunk_tiles);
   HM_TRY(mixed_schedule(h, M.chunk_tiles, M.group_tiles, M.p1_ring ? 1 : 0, s));
   HM_TRY(upload(M.pan_of, pan_of, s));
   HM_TRY(upload(M.tile_leaf, tile_leaf, s));
@@ -1374,12 +1453,13 @@ hm_status mixed_schedule(hm_hmatrix_s* h, int chunk_tiles, int group_tiles, int 
 }
 
 hm_status mixed_warp_pass(hm_hmatrix_s* h, int nh, int nr, uint4* Xf, float4* S, uint32_t* T, long long xh,
-                          long long sh, long long th, float* Y, int ldy, cudaStream_t s, KernelMarks* km);
+                          long long sh, long long th, float* Y, int ldy, const int* perm, cudaStream_t s,
+                          KernelMarks* km);
 
 hm_status mixed_run_panel(hm_hmatrix_s* h, int nr, const float* X, int ldx, float* Y, int ldy, float* scratch,
-                          cudaStream_t s, KernelMarks* km) {
+                          const int* perm, cudaStream_t s, KernelMarks* km) {
   MxPlan& M = h->mx;
-  if (M.fmt == 1) return fp32_run_panel(h, nr, X, ldx, Y, ldy, scratch, s, km);
+  if (M.fmt == 1) return fp32_run_panel(h, nr, X, ldx, Y, ldy, scratch, perm, s, km);
   if (nr < 1 || nr > 128) return fail(HM_ERR_INVALID, "mixed product: a pass holds 1 to 128 right-hand sides");
   // 16-column parts of this pass: 1, 2, 4 or 8 (the parts past nr are zero)
   const int nh = nr > 64 ? 8 : (nr > 32 ? 4 : (nr > 16 ? 2 : 1));
@@ -1397,16 +1477,17 @@ hm_status mixed_run_panel(hm_hmatrix_s* h, int nr, const float* X, int ldx, floa
   const long long xbytes = 4ll * h->n * 16 * nh;  // the X fragments, hi + lo
   if (M.num_tiles > 0) {
     k_mx_split_x<<<dim3((M.num_tiles + 3) / 4, nh), 128, 0, s>>>(X, ldx, nr, M.num_tiles, M.tile_leaf.p,
-                                                                 M.leaf_tile0.p, leaf_off, Xf, tc ? Xf : nullptr);
+                                                                 M.leaf_tile0.p, leaf_off, perm, Xf, tc ? Xf : nullptr);
     HM_LAUNCH_CHECK();
     if (km) km->mark("k_mx_split_x", 4ll * h->n * nr + xbytes, s);
   }
   if (tc) {
-    HM_TRY(mixed_tc_pass(h, nr, Xf, reinterpret_cast<float*>(S), reinterpret_cast<uint4*>(T), Y, ldy, s, km));
+    HM_TRY(mixed_tc_pass(h, nr, Xf, reinterpret_cast<float*>(S), reinterpret_cast<uint4*>(T), Y, ldy, perm, s,
+                         km));
   } else {
-    HM_TRY(mixed_warp_pass(h, nh, nr, Xf, S, T, xh, sh, th, Y, ldy, s, km));
+    HM_TRY(mixed_warp_pass(h, nh, nr, Xf, S, T, xh, sh, th, Y, ldy, perm, s, km));
   }
-  if (h->diag_fly)  // the diagonal from coordinates, 16 columns at a time
+  if (h->diag_fly)  // the diagonal from coordinates, 16 columns at a time (perm is null then)
     for (int c0 = 0; c0 < nr; c0 += 16)
       HM_TRY(diag_fly_panel(h, std::min(16, nr - c0), X + (size_t)c0 * ldx, ldx, Y + (size_t)c0 * ldy, ldy, s, km));
   return HM_OK;
@@ -1414,7 +1495,8 @@ hm_status mixed_run_panel(hm_hmatrix_s* h, int nr, const float* X, int ldx, floa
 
 // Phases 1 and 2 of a pass on the warp-level MMA kernels (nh parts of 16).
 hm_status mixed_warp_pass(hm_hmatrix_s* h, int nh, int nr, uint4* Xf, float4* S, uint32_t* T, long long xh,
-                          long long sh, long long th, float* Y, int ldy, cudaStream_t s, KernelMarks* km) {
+                          long long sh, long long th, float* Y, int ldy, const int* perm, cudaStream_t s,
+                          KernelMarks* km) {
   MxPlan& M = h->mx;
   const int* leaf_off = h->tree->offsets.p;
   const long long xbytes = 4ll * h->n * 16 * nh;
@@ -1445,20 +1527,29 @@ hm_status mixed_warp_pass(hm_hmatrix_s* h, int nh, int nr, uint4* Xf, float4* S,
     if (km) km->mark("k_mx_reduce", (512ll * M.s_tiles + 512ll * M.nmt) * nh, s);
   }
   if (M.p2_tiles > 0) {
-    const unsigned grid = (unsigned)M.p2_tiles;
-    const int te = M.p2_tile0 + M.p2_tiles;
-#define HM_P2_ARGS                                                                                            \
-  M.p2_tile0, te, h->depth, M.tile_leaf.p, M.leaf_tile0.p, leaf_off, M.pan_of.p, M.panels.p, M.store.p, T,      \
-      M.leaf_dptr.p, M.leaf_dblk.p, M.dense.p, Xf, Y, ldy, nr, xh, th
+    auto p2 = [&](auto nhc, auto wpc, auto spc) {
+      constexpr int NH = decltype(nhc)::value, WPC = decltype(wpc)::value, SP = decltype(spc)::value;
+      k_mx_p2<NH, WPC, SP><<<(unsigned)M.p2_tiles, 32 * WPC * SP, 0, s>>>(
+          M.p2_tile0, M.p2_tile0 + M.p2_tiles, h->depth, M.tile_leaf.p, M.leaf_tile0.p, leaf_off, M.pan_of.p,
+          M.panels.p, M.store.p, T, M.leaf_dptr.p, M.leaf_dblk.p, M.dense.p, Xf, perm, Y, ldy, nr, xh, th);
+    };
+    auto p2_shared = [&](auto nhc) {
+      const int sp = p2_share(M.p2_tiles, 3000);
+      if (sp == 8)
+        p2(nhc, kInt<1>{}, kInt<8>{});
+      else if (sp == 4)
+        p2(nhc, kInt<1>{}, kInt<4>{});
+      else
+        p2(nhc, kInt<1>{}, kInt<1>{});
+    };
     if (nh == 1)
-      k_mx_p2<1, 1><<<grid, 32, 0, s>>>(HM_P2_ARGS);
+      p2_shared(kInt<1>{});
     else if (nh == 2)
-      k_mx_p2<2, 1><<<grid, 32, 0, s>>>(HM_P2_ARGS);
+      p2_shared(kInt<2>{});
     else if (nh == 4)  // two warps of two parts share each row tile's factor tiles
-      k_mx_p2<2, 2><<<grid, 64, 0, s>>>(HM_P2_ARGS);
+      p2(kInt<2>{}, kInt<2>{}, kInt<1>{});
     else  // four warps of two parts
-      k_mx_p2<2, 4><<<grid, 128, 0, s>>>(HM_P2_ARGS);
-#undef HM_P2_ARGS
+      p2(kInt<2>{}, kInt<4>{}, kInt<1>{});
     HM_LAUNCH_CHECK();
     if (km) km->mark("k_mx_p2", M.bytes_p2 + xbytes + 4ll * h->n * nr, s);
   }

@@ -34,6 +34,9 @@ struct hm_hmatrix_s;
 
 namespace hm {
 
+// Scratch of the allocation-free product, in floats (hm_matvec.cu).
+constexpr long long kNoallocFloats = 4ll << 20;
+
 struct MxPanel {
   long long hi1, lo1, hi2, lo2;  // 512-byte tile offsets into MxPlan::store, [row tile][col tile]
   long long s0;                  // first phase-1 output tile (nchunk x nct tiles)
@@ -133,7 +136,7 @@ struct MxPlan {
   std::vector<MxDense> h_dense;           // host copy
   std::vector<MxLoc> h_locs;              // every factor and dense block converted into the panels
   std::vector<std::pair<const float*, int>> loc_index;  // h_locs by key, sorted (built on first use)
-  int chunk_tiles = 128, group_tiles = 8;  // phase-1 unit shape (schedule parameters; measured best at 16 RHS)
+  int chunk_tiles = 128, group_tiles = 8;  // phase-1 unit shape (p1_shape, or the schedule's)
   bool p1_ring = false;                    // phase 1 by persistent warps with a cp.async ring
   int num_sms = 148;
   // 128-column passes (BF16 format) on tcgen05 (hm_mixed_tc.cu): phase-1
@@ -190,7 +193,7 @@ hm_status mixed_build(hm_hmatrix_s* h, const std::vector<MxPair>& pairs, const s
 // the chunk reduction, phase 2 (Y, tree order, nr <= 128 columns).
 struct KernelMarks;
 hm_status mixed_tc_pass(hm_hmatrix_s* h, int nr, const uint4* Xtc, float* S, uint4* Tb, float* Y, int ldy,
-                        cudaStream_t s, KernelMarks* km);
+                        const int* perm, cudaStream_t s, KernelMarks* km);
 
 struct KernelMarks;
 
@@ -203,9 +206,10 @@ hm_status mixed_schedule(hm_hmatrix_s* h, int chunk_tiles, int group_tiles, int 
 // One pass of nr <= 128 right-hand sides in tree order (two, four or eight parts of 16
 // when nr > 16: every factor tile is read once for all of them); scratch holds
 // scratch_floats(h) floats, h = 1, 2, 4 or 8 parts.  km (optional) receives an event
-// after each kernel.
+// after each kernel.  perm (optional; null with diag_fly): X and Y are in the
+// points' original order, tree row i at row perm[i].
 hm_status mixed_run_panel(hm_hmatrix_s* h, int nr, const float* X, int ldx, float* Y, int ldy, float* scratch,
-                          cudaStream_t s, KernelMarks* km);
+                          const int* perm, cudaStream_t s, KernelMarks* km);
 
 // The FP32 values of the BF16 panels: for each (h_locs index, device
 // destination), the factor or dense block rebuilt column-major from its hi
@@ -222,6 +226,27 @@ int mixed_find_loc(hm_hmatrix_s* h, const float* key);
 hm_status fp32_convert(hm_hmatrix_s* h, const std::vector<const float*>& colsrc, const std::vector<MxDense>& dense,
                        cudaStream_t s);
 hm_status fp32_run_panel(hm_hmatrix_s* h, int nr, const float* X, int ldx, float* Y, int ldy, float* scratch,
-                         cudaStream_t s, KernelMarks* km);
+                         const int* perm, cudaStream_t s, KernelMarks* km);
+
+// Phase-1 unit shape of a matrix of `tiles` row tiles.  One warp walks a unit
+// one load latency per row tile, so the tallest unit bounds the phase unless
+// the matrix gives the chip many times more units than it runs at once: with
+// 128 x 8 units phase 1 took 65 us at 8192 points (2-D FP32), 215 us at 60001
+// (mixture) and 310 us at 100003 (FP32); with these shapes, the partials'
+// reduction included, 19, 57 and 182 us.  Above 2^19 points 128 x 8 stays (64
+// x 8 and 128 x 4 are within 2 % of it).
+inline void p1_shape(int tiles, int* chunk, int* group) {
+  *chunk = std::min(128, std::max(8, tiles / 128));
+  *group = tiles < 4096 ? 4 : 8;
+}
+
+// Warps that share one row tile's sources in phase 2 (passes of up to 32
+// right-hand sides).  One warp per row tile fills the chip (28 warps per SM)
+// from about 4000 row tiles on and walks its sources one latency at a time;
+// measured 1 -> 8 warps at 256 row tiles 45 -> 15 us (FP32) and 105 -> 25 us
+// (mixed), 1 -> 4 at 1024 150 -> 60 us (FP32), at 2048 123 -> 84 us (mixed),
+// at 4096 240 -> 204 us (FP32) but 240 -> 291 us (mixed), at 8192 466 -> 488
+// and 282 -> 299 us.  top: the last count at which four warps share.
+inline int p2_share(int row_tiles, int top) { return row_tiles <= 512 ? 8 : row_tiles <= top ? 4 : 1; }
 
 }  // namespace hm

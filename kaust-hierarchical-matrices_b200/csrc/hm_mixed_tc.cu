@@ -413,8 +413,8 @@ __global__ void __launch_bounds__(kP2Threads, 1)
     k_mx_p2_tc(int nblocks, int tile0, int tile_end, const int* __restrict__ step_ptr,
                const P2Step* __restrict__ steps, const uint4* __restrict__ store, const uint4* __restrict__ Tb,
                const uint4* __restrict__ Xtc, const int* __restrict__ tile_leaf,
-               const int* __restrict__ leaf_tile0, const int* __restrict__ leaf_off, float* __restrict__ Y, int ldy,
-               int nr, int* __restrict__ err) {
+               const int* __restrict__ leaf_tile0, const int* __restrict__ leaf_off, const int* __restrict__ perm,
+               float* __restrict__ Y, int ldy, int nr, int* __restrict__ err) {
   extern __shared__ __align__(1024) unsigned char smem[];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const uint32_t sbase = smem_u32(smem);
@@ -598,7 +598,7 @@ __global__ void __launch_bounds__(kP2Threads, 1)
       if (G < tile_end) {
         const int x = tile_leaf[G];
         const int r = leaf_off[x] + 32 * (G - leaf_tile0[x]) + (m & 31);
-        if (r < leaf_off[x + 1]) row = r;
+        if (r < leaf_off[x + 1]) row = perm ? __ldg(perm + r) : r;
       }
       for (int c = 0; c < nchains; ++c) {
         ++chain;
@@ -651,7 +651,7 @@ __global__ void __launch_bounds__(kP2Threads, 1)
 }  // namespace
 
 hm_status mixed_tc_pass(hm_hmatrix_s* h, int nr, const uint4* Xtc, float* S, uint4* Tb, float* Y, int ldy,
-                        cudaStream_t s, KernelMarks* km) {
+                        const int* perm, cudaStream_t s, KernelMarks* km) {
   MxPlan& M = h->mx;
   // the kernels' shared-memory limit, once per device of this process
   static unsigned long long attr_done = 0;
@@ -680,7 +680,7 @@ hm_status mixed_tc_pass(hm_hmatrix_s* h, int nr, const uint4* Xtc, float* S, uin
     const int grid = std::min(M.num_sms, M.p2_blocks);
     k_mx_p2_tc<<<grid, kP2Threads, kP2Smem, s>>>(M.p2_blocks, M.p2_tile0, M.p2_tile0 + M.p2_tiles, M.p2_step_ptr.p,
                                                 M.p2_steps.p, M.store.p, Tb, Xtc, M.tile_leaf.p, M.leaf_tile0.p,
-                                                h->tree->offsets.p, Y, ldy, nr, M.tc_err.p);
+                                                h->tree->offsets.p, perm, Y, ldy, nr, M.tc_err.p);
     HM_LAUNCH_CHECK();
     if (km) km->mark("k_mx_p2_tc", M.bytes_p2 + xbytes + 4ll * h->n * nr, s);
   }

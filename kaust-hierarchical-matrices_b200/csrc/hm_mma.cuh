@@ -89,6 +89,16 @@ __device__ __forceinline__ void mma_bf16(float (&c)[4], uint32_t a0, uint32_t a1
       : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
+// inclusive sum over the lanes up to this one
+__device__ __forceinline__ int warp_scan(int v, int lane) {
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int u = __shfl_up_sync(0xffffffffu, v, o);
+    if (lane >= o) v += u;
+  }
+  return v;
+}
+
 // ---- FP64 m8n8k4 (lane = 4*g + t) ------------------------------------------
 //   A (8x4): a = A[g][t];  B (4x8): b = B[t][g];  C (8x8): c0, c1 = C[g][2t], C[g][2t+1]
 __device__ __forceinline__ void mma_f64(double (&d)[2], double a, double b) {
