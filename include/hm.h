@@ -78,6 +78,13 @@ HM_API const char* hm_last_error(void);
 /* Library version string. */
 HM_API const char* hm_version(void);
 
+/* Device memory.  The library keeps up to 4 GB of device memory that its
+ * objects have released, for the next ones (mapping and unmapping memory costs
+ * a build up to a second).  hm_release_memory waits for the current device and
+ * hands that memory back; memory in use is not touched.  An allocation of the
+ * library that fails does the same and tries again. */
+HM_API hm_status hm_release_memory(void);
+
 /* --- points ------------------------------------------------------------- */
 
 /* generateDataset (src/generateDataset.cu:15-19): d_points[i] for i < n*d is

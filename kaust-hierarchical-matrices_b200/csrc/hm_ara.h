@@ -1,9 +1,9 @@
 // hm_ara.h -- what the stages of the batched ARA build share: the problems of
 // a batch, their state, and the launchers of the per-block stages.
 //
-// Workspace layout of a problem (working precision W): Q (m x k), Y (m x s)
-// and B (n x k), column-major with the row count rounded up to 4 (ara_ld), so
-// that every column starts on a 16-byte boundary; the padding rows are zero.
+// Workspace of a problem (working precision W): Q (m x k), Y (m x s) and B
+// (n x k), column-major with the row count rounded up to 4 (ara_ld), so that
+// every column starts on a 16-byte boundary; the padding rows are zero.
 #pragma once
 #include <vector>
 
@@ -21,7 +21,9 @@ struct Prob {
   int kmax;
   int level;
   int u, v;
-  long long qoff, yoff, boff;  // workspace offsets (elements)
+  int gid;                     // its number among the problems that were listed with it (the sample's stream)
+  int qcap;                    // columns Q has room for now (<= kmax)
+  void *q, *y, *b;             // Q, Y, B in the working precision
   double tscale2;              // (this block's tolerance / the build's)^2: 1, or the level schedule's
 };
 
@@ -59,8 +61,7 @@ hm_status orth_plan(const std::vector<Prob>& probs, OrthPlan* plan, cudaStream_t
 // against Q, tested (est = ||Y'||^2 / bs <= thresh2 tscale2 ||A||^2), and
 // otherwise orthonormalised and appended to Q.
 template <typename W>
-hm_status orth_round(const OrthPlan& plan, const Prob* probs, ProbState* st, W* ws, int bs, double thresh2,
-                     cudaStream_t s);
+hm_status orth_round(const OrthPlan& plan, const Prob* probs, ProbState* st, int bs, double thresh2, cudaStream_t s);
 
 // ---- truncation (hm_trunc.cu) --------------------------------------------------
 constexpr int kTruncMax = 128;  // widest basis the SVD truncation handles (wider: kept as sampled)
@@ -77,14 +78,14 @@ struct TruncWork {
 // truncation and BF16 rounding budgets relative to ||A||_F^2.
 template <typename W>
 hm_status trunc_rank(const std::vector<Prob>& bp, const std::vector<ProbState>& hst, const Prob* probs, ProbState* st,
-                     const W* ws, double tol2, double rbudget, TruncWork* tw, cudaStream_t s);
+                     double tol2, double rbudget, TruncWork* tw, cudaStream_t s);
 
 // U = Q W_r and V = B W_r of the problems with dst_u >= 0, FP32, column-major
 // without padding.  rows, cols: the batch's 64-row tiles (problem, tile) over
 // the blocks' rows and columns.
 template <typename W>
-hm_status trunc_pack(const Prob* probs, const ProbState* st, const W* ws, const TruncWork& tw, const int2* rows,
-                     size_t nrows, const int2* cols, size_t ncols, const long long* dst_u, const long long* dst_v,
+hm_status trunc_pack(const Prob* probs, const ProbState* st, const TruncWork& tw, const int2* rows, size_t nrows,
+                     const int2* cols, size_t ncols, const long long* dst_u, const long long* dst_v,
                      float* dst, cudaStream_t s);
 
 }  // namespace hm

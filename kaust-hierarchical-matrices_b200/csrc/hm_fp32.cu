@@ -458,7 +458,8 @@ __global__ void k_fp_conv_dense(const MxDense* __restrict__ dense, const long lo
 
 }  // namespace
 
-hm_status fp32_convert(hm_hmatrix_s* h, const std::vector<const float*>& colsrc, const std::vector<MxDense>& dense,
+// colsrc (device): see k_fp_conv_panels
+hm_status fp32_convert(hm_hmatrix_s* h, const float* const* colsrc, const std::vector<MxDense>& dense,
                        cudaStream_t s) {
   MxPlan& M = h->mx;
   const std::vector<MxPanel>& panels = M.h_panels;
@@ -470,16 +471,12 @@ hm_status fp32_convert(hm_hmatrix_s* h, const std::vector<const float*>& colsrc,
       start[p] = tot;
       tot += (long long)panels[p].nrt * panels[p].nct;
     }
-    DevBuf<const float*> dcol;
     DevBuf<long long> dstart;
-    HM_TRY(dcol.alloc(std::max<size_t>(colsrc.size(), 1)));
     HM_TRY(dstart.alloc(np));
-    if (!colsrc.empty())
-      HM_CUDA(cudaMemcpyAsync(dcol.p, colsrc.data(), sizeof(const float*) * colsrc.size(), cudaMemcpyHostToDevice, s));
     HM_CUDA(cudaMemcpyAsync(dstart.p, start.data(), sizeof(long long) * np, cudaMemcpyHostToDevice, s));
     if (tot > 0) {
       k_fp_conv_panels<<<(unsigned)((tot * 32 + 255) / 256), 256, 0, s>>>(
-          M.panels.p, dstart.p, np, tot, dcol.p, M.tile_leaf.p, M.leaf_tile0.p, h->tree->offsets.p, M.store.p);
+          M.panels.p, dstart.p, np, tot, colsrc, M.tile_leaf.p, M.leaf_tile0.p, h->tree->offsets.p, M.store.p);
       HM_LAUNCH_CHECK();
     }
     HM_CUDA(cudaStreamSynchronize(s));

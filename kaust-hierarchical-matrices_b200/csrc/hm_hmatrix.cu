@@ -45,6 +45,7 @@ constexpr int kTR = 64;        // rows of a KMM tile
 constexpr int kTC = 64;        // columns per KMM chunk
 constexpr int kKmmThreads = 256;
 constexpr int kColGroup = 128; // projection columns per sketch launch
+constexpr int kQCols = 64;     // basis columns a problem starts with room for
 template <typename W>
 struct KmmArgs {
   const Prob* probs;
@@ -58,7 +59,6 @@ struct KmmArgs {
   int bs;
   uint32_t seed;
   int round;
-  W* ws;              // workspace (Y, Q, B) in the ARA's working precision
 };
 
 // ---------------------------------------------------------------------------
@@ -88,8 +88,8 @@ __global__ void __launch_bounds__(kKmmThreads) k_kmm(KmmArgs<W> a) {
   const int rbase = a.mode ? P.c0 : P.r0;
   const int cbase = a.mode ? P.r0 : P.c0;
   const int ldo = ara_ld(mr), ldq = ara_ld(P.m);
-  W* out = a.ws + (a.mode ? P.boff : P.yoff) + (size_t)col0 * ldo;
-  const W* Q = a.ws + P.qoff + (size_t)col0 * ldq;  // mode 1: W = Q (m x k)
+  W* out = reinterpret_cast<W*>(a.mode ? P.b : P.y) + (size_t)col0 * ldo;
+  const W* Q = reinterpret_cast<const W*>(P.q) + (size_t)col0 * ldq;  // mode 1: W = Q (m x k)
   const int nslab = s <= 32 ? 1 : (s <= 64 ? 2 : 4);
   const int ncg = 4 / nslab;
   const int t = threadIdx.x, r = t & 63, q = t >> 6;
@@ -119,7 +119,7 @@ __global__ void __launch_bounds__(kKmmThreads) k_kmm(KmmArgs<W> a) {
       W w = W(0);
       if (j < nc && cc < s) {
         if (a.mode == 0)
-          w = (W)gauss_at(a.seed, (uint32_t)it.x, (uint32_t)j, (uint32_t)(a.round * kMaxBs + cc));
+          w = (W)gauss_at(a.seed, (uint32_t)P.gid, (uint32_t)j, (uint32_t)(a.round * kMaxBs + cc));
         else
           w = Q[(size_t)cc * ldq + j];
       }
@@ -216,7 +216,6 @@ struct KmmFastArgs {
   const uint4* qt;          // projection: {hi b0, hi b1, lo b0, lo b1} of Q, per problem
   const long long* qpoff;   // per problem (batch index), 16-byte words
   int col0;                 // projection: first basis column of this launch
-  float* ws;
 };
 
 __device__ __forceinline__ float ex2_approx(float x) {
@@ -269,7 +268,7 @@ __global__ void __launch_bounds__(128) k_kmm_fast(KmmFastArgs a) {
   const int rbase = MODE ? P.c0 : P.r0;
   const int cbase = MODE ? P.r0 : P.c0;
   const int ld = ara_ld(mr);
-  float* out = a.ws + (MODE ? P.boff : P.yoff) + (size_t)col0 * ld;
+  float* out = reinterpret_cast<float*>(MODE ? P.b : P.y) + (size_t)col0 * ld;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
   const int ra = it.y * kTR + warp * 16 + g, rb = ra + 8;
   const bool ra_ok = ra < mr, rb_ok = rb < mr;
@@ -420,14 +419,13 @@ __global__ void k_omega_pack(uint2* om, int ksteps, int bs, int nt_tot, uint32_t
 // Q (m x k, column-major, ld m) of each problem in fragment order, hi and lo
 // (see KmmFastArgs): k-steps over the rows padded to whole coordinate chunks,
 // column tiles over k padded to 8.
-__global__ void k_pack_q(const Prob* probs, const ProbState* st, const float* ws, const long long* qpoff,
-                         uint4* qt) {
+__global__ void k_pack_q(const Prob* probs, const ProbState* st, const long long* qpoff, uint4* qt) {
   const Prob P = probs[blockIdx.x];
   const int k = st[blockIdx.x].k;
   if (k <= 0) return;
   const int ntq = (k + 7) >> 3;
   const int ksteps = (P.m + kCC - 1) / kCC * (kCC / 16);
-  const float* Q = ws + P.qoff;
+  const float* Q = reinterpret_cast<const float*>(P.q);
   uint4* q = qt + qpoff[blockIdx.x];
   for (int e = threadIdx.x; e < ksteps * ntq * 32; e += blockDim.x) {
     const int lane = e & 31, g = lane >> 2, t = lane & 3;
@@ -488,6 +486,19 @@ void launch_kmm_fast(int d, int kind, int mode, int nt, unsigned grid, cudaStrea
 // ---------------------------------------------------------------------------
 // dense blocks
 // ---------------------------------------------------------------------------
+struct QMove {  // a basis that moves to wider storage
+  const void* from;
+  long long to, count;  // elements
+};
+
+template <typename W>
+__global__ void k_move_q(const QMove* __restrict__ moves, W* __restrict__ base) {
+  const QMove m = moves[blockIdx.x];
+  const W* from = reinterpret_cast<const W*>(m.from);
+  for (long long e = blockIdx.y * blockDim.x + threadIdx.x; e < m.count; e += (long long)gridDim.y * blockDim.x)
+    base[m.to + e] = from[e];
+}
+
 struct DenseItem {
   int r0, m, c0, n;
   long long off;
@@ -631,7 +642,6 @@ hm_status hmatrix_build(hm_kdtree t, hm_structure s, const double* d_points, con
   // ---- batches bounded by the workspace budget -----------------------------
   size_t freeb = 0, totb = 0;
   HM_CUDA(cudaMemGetInfo(&freeb, &totb));
-  const size_t budget_bytes = std::min<size_t>(freeb / 4, (size_t)24 << 30);
   // per-problem results that survive the batch: rank (-1: stored dense, -2:
   // split into its child blocks), low-part columns, and the factor location.
   // A problem that misses the tolerance at its rank cap above the leaf level
@@ -662,7 +672,6 @@ hm_status hmatrix_build(hm_kdtree t, hm_structure s, const double* d_points, con
   const bool fp64 = opt.tol < 5e-6;
   auto batch_loop = [&](auto tag) -> hm_status {
     using W = decltype(tag);
-    const size_t budget_elems = budget_bytes / sizeof(W);
     HM_CUDA(cudaFuncSetAttribute(k_kmm<W>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kmm_smem<W>()));
     // The specialised sketch kernels draw a double-width first sample (the
     // generation of the kernel block, not its product with the sample, is
@@ -674,41 +683,45 @@ hm_status hmatrix_build(hm_kdtree t, hm_structure s, const double* d_points, con
     const bool fastW = kTensorW && t->d <= 3;
     const int bs_first = fastW ? std::min(2 * bs, kMaxBs) : bs;  // round 0 columns
     const int wmax = std::max(bs_first, bs);                      // widest sample
-    // greedy batches under the workspace budget; one workspace for all of
-    // them (child blocks of split problems come in later batches, whose
-    // workspace is no larger unless a batch of them packs tighter)
-    auto next_batch = [&](long long ps, size_t* wsz_out) {
+    // Greedy batches.  A problem starts with room for kQCols basis columns and
+    // its sample; the few that need more move to wider storage when they do
+    // (below), and B is allocated at its exact width after the rounds.  The
+    // budget, an eighth of all problems' need between kBatchMin and kBatchMax,
+    // gives every launch enough blocks and keeps what is mapped and unmapped
+    // per build small (mapping a GB takes 0.2 to 100 ms on a shared host).
+    // Problems listed together share one first-round width, whatever the batch.
+    constexpr size_t kBatchMin = size_t(1) << 30, kBatchMax = size_t(12) << 30;
+    auto need_of = [&](const Prob& P) {
+      return ((size_t)ara_ld(P.m) * (std::min(P.kmax, kQCols) + wmax) + (size_t)ara_ld(P.n) * kMaxBs) * sizeof(W);
+    };
+    size_t budget = 0;
+    int gen_bs0 = 0;  // first-round columns of the problems listed last
+    long long gen_end = 0;
+    auto next_batch = [&](long long ps) {
+      if (ps >= gen_end) {
+        gen_end = (long long)probs.size();
+        size_t all = 0;
+        gen_bs0 = bs_first;  // as wide as every block's rank cap allows
+        for (long long i = ps; i < gen_end; ++i) {
+          probs[i].gid = (int)(i - ps);
+          all += need_of(probs[i]);
+          if (probs[i].kmax < gen_bs0) gen_bs0 = std::max(bs, probs[i].kmax / 8 * 8);
+        }
+        budget = std::min(std::max(all / 8, kBatchMin), std::min<size_t>(freeb / 8, kBatchMax));
+      }
       long long pe = ps;
-      size_t wsz = 0;
-      while (pe < (long long)probs.size()) {
-        const Prob& P = probs[pe];
-        const size_t lm = ara_ld(P.m), ln = ara_ld(P.n);
-        size_t need = lm * (P.kmax + wmax) + lm * wmax + ln * (P.kmax + wmax);
-        if (pe > ps && wsz + need > budget_elems) break;
-        wsz += need;
+      size_t sz = 0;
+      while (pe < gen_end) {
+        const size_t need = need_of(probs[pe]);
+        if (pe > ps && sz + need > budget) break;
+        sz += need;
         ++pe;
       }
-      *wsz_out = wsz;
       return pe;
     };
-    size_t ws_max = 1;
-    for (long long ps = pstart; ps < (long long)probs.size();) {
-      size_t w = 0;
-      ps = next_batch(ps, &w);
-      ws_max = std::max(ws_max, w);
-    }
-    DevBuf<W> ws;
-    {
-      hm_status st0 = ws.alloc(ws_max);
-      if (st0) return st0;
-    }
+    DevBuf<W> ws, wb;  // Q and Y; B (kept from batch to batch)
     while (pstart < (long long)probs.size()) {
-      size_t wsz = 0;
-      const long long pend = next_batch(pstart, &wsz);
-      if (wsz > ws.n) {
-        hm_status st0 = ws.alloc(wsz);
-        if (st0) return st0;
-      }
+      const long long pend = next_batch(pstart);
       const int nb = (int)(pend - pstart);
       tr.mark("batch begin", stream, nb, 0);
       std::vector<Prob> bp(probs.begin() + pstart, probs.begin() + pend);
@@ -716,14 +729,22 @@ hm_status hmatrix_build(hm_kdtree t, hm_structure s, const double* d_points, con
       std::vector<int2> items_rows, items_cols;
       for (int i = 0; i < nb; ++i) {
         Prob& P = bp[i];
-        P.qoff = (long long)off;
-        off += (size_t)ara_ld(P.m) * (P.kmax + wmax);
-        P.yoff = (long long)off;
-        off += (size_t)ara_ld(P.m) * wmax;
-        P.boff = (long long)off;
-        off += (size_t)ara_ld(P.n) * (P.kmax + wmax);
+        P.qcap = std::min(P.kmax, kQCols);
+        off += (size_t)ara_ld(P.m) * (P.qcap + wmax);
         for (int tt = 0; tt * kTR < P.m; ++tt) items_rows.push_back(make_int2(i, tt));
         for (int tt = 0; tt * kTR < P.n; ++tt) items_cols.push_back(make_int2(i, tt));
+      }
+      if (off > ws.n) {
+        hm_status st0 = ws.alloc(off);
+        if (st0) return st0;
+      }
+      off = 0;
+      for (int i = 0; i < nb; ++i) {
+        Prob& P = bp[i];
+        P.q = ws.p + off;
+        off += (size_t)ara_ld(P.m) * P.qcap;
+        P.y = ws.p + off;
+        off += (size_t)ara_ld(P.m) * wmax;
       }
       DevBuf<Prob> dprobs;
       DevBuf<ProbState> dst;
@@ -753,7 +774,6 @@ hm_status hmatrix_build(hm_kdtree t, hm_structure s, const double* d_points, con
       ka.kp = h->kp;
       ka.bs = bs;
       ka.seed = (uint32_t)(opt.seed ^ (opt.seed >> 32)) ^ 0x5bd1e995u;
-      ka.ws = ws.p;
       OrthPlan orth;
       if ((st = orth_plan<W>(bp, &orth, stream))) return st;
       // FP32 working precision and d <= 3: specialised tensor-core sketch
@@ -762,10 +782,7 @@ hm_status hmatrix_build(hm_kdtree t, hm_structure s, const double* d_points, con
       const bool fast = kTensor && t->d <= 3;
       KmmFastArgs kf{};
       DevBuf<uint2> om2;
-      // round 0 columns: as wide as every block's rank cap allows
-      int bs0 = bs_first;
-      for (const Prob& P : bp)
-        if (P.kmax < bs0) bs0 = std::max(bs, P.kmax / 8 * 8);
+      const int bs0 = gen_bs0;
       const int bs8 = (bs0 + 7) & ~7;
       int om_rows2 = 0;
       if (fast) {
@@ -792,10 +809,10 @@ hm_status hmatrix_build(hm_kdtree t, hm_structure s, const double* d_points, con
         kf.bs = bs;
         kf.om = om2.p;
         kf.om_nt = bs8 / 8;
-        kf.ws = reinterpret_cast<float*>(ws.p);
       }
       tr.mark("batch setup", stream, nb, 0);
       const int max_rounds = kMaxCols / bs + 2;
+      std::vector<DevBuf<W>> grown;  // wider bases, until the end of the batch
       for (int round = 0; round < max_rounds; ++round) {
         // sample columns: double width in the first round and again from the
         // fourth on (the blocks still active by then are the high-rank ones;
@@ -803,6 +820,34 @@ hm_status hmatrix_build(hm_kdtree t, hm_structure s, const double* d_points, con
         // wider rounds mean fewer of them; earlier, a wider basis would cost
         // more in the projection than it saves)
         const int rbs = fast && round != 1 && round != 2 ? bs0 : bs;
+        // active bases without room for this round's columns move to storage
+        // of twice the width (at most their cap)
+        {
+          std::vector<QMove> moves;
+          size_t more = 0;
+          for (int i = 0; i < nb; ++i) {
+            Prob& P = bp[i];
+            const int k = hst[i].k;
+            if (!hst[i].active || k + rbs <= P.qcap || P.qcap >= P.kmax) continue;
+            P.qcap = std::min(P.kmax, std::max(2 * P.qcap, k + rbs));
+            moves.push_back(QMove{P.q, (long long)more, (long long)ara_ld(P.m) * k});
+            more += (size_t)ara_ld(P.m) * P.qcap;
+          }
+          if (!moves.empty()) {
+            grown.emplace_back();
+            if ((st = grown.back().alloc_async(more, stream))) return st;
+            W* base = grown.back().p;
+            size_t j = 0;
+            for (int i = 0; i < nb && j < moves.size(); ++i)
+              if (bp[i].q == moves[j].from) bp[i].q = base + moves[j++].to;
+            DevBuf<QMove> dm;
+            if ((st = dm.alloc_async(moves.size(), stream))) return st;
+            HM_CUDA(cudaMemcpyAsync(dm.p, moves.data(), sizeof(QMove) * moves.size(), cudaMemcpyHostToDevice, stream));
+            k_move_q<W><<<dim3((unsigned)moves.size(), 8), 256, 0, stream>>>(dm.p, base);
+            HM_LAUNCH_CHECK();
+            HM_CUDA(cudaMemcpyAsync(dprobs.p, bp.data(), sizeof(Prob) * nb, cudaMemcpyHostToDevice, stream));
+          }
+        }
         if (fast) {
           k_omega_pack<<<592, 256, 0, stream>>>(om2.p, om_rows2 / 8, rbs, bs8 / 8, ka.seed, round);
           HM_LAUNCH_CHECK();
@@ -819,7 +864,7 @@ hm_status hmatrix_build(hm_kdtree t, hm_structure s, const double* d_points, con
         }
         HM_LAUNCH_CHECK();
         tr.mark("  round sketch", stream, round, 1);
-        if ((st = orth_round<W>(orth, dprobs.p, dst.p, ws.p, rbs, thresh2, stream))) return st;
+        if ((st = orth_round<W>(orth, dprobs.p, dst.p, rbs, thresh2, stream))) return st;
         tr.mark("  round orth", stream, round, 2);
         HM_CUDA(cudaMemcpyAsync(hst.data(), dst.p, sizeof(ProbState) * nb, cudaMemcpyDeviceToHost, stream));
         HM_CUDA(cudaStreamSynchronize(stream));
@@ -829,6 +874,17 @@ hm_status hmatrix_build(hm_kdtree t, hm_structure s, const double* d_points, con
       }
       tr.mark("sample rounds", stream, nb, 2);
       // B = A^T Q
+      {
+        size_t bsz = 0;
+        for (int i = 0; i < nb; ++i) bsz += (size_t)ara_ld(bp[i].n) * hst[i].k;
+        if (bsz > wb.n && (st = wb.alloc(bsz))) return st;
+        bsz = 0;
+        for (int i = 0; i < nb; ++i) {
+          bp[i].b = wb.p + bsz;
+          bsz += (size_t)ara_ld(bp[i].n) * hst[i].k;
+        }
+        HM_CUDA(cudaMemcpyAsync(dprobs.p, bp.data(), sizeof(Prob) * nb, cudaMemcpyHostToDevice, stream));
+      }
       DevBuf<uint4> qt;
       DevBuf<long long> dqpoff;
       DevBuf<int2> dcls;
@@ -844,7 +900,7 @@ hm_status hmatrix_build(hm_kdtree t, hm_structure s, const double* d_points, con
           return st;
         tr.mark("  q table alloc (MB)", stream, (long long)(qw * 16 >> 20), 3);
         HM_CUDA(cudaMemcpyAsync(dqpoff.p, qpoff.data(), sizeof(long long) * nb, cudaMemcpyHostToDevice, stream));
-        k_pack_q<<<nb, 256, 0, stream>>>(dprobs.p, dst.p, reinterpret_cast<const float*>(ws.p), dqpoff.p, qt.p);
+        k_pack_q<<<nb, 256, 0, stream>>>(dprobs.p, dst.p, dqpoff.p, qt.p);
         HM_LAUNCH_CHECK();
         tr.mark("  q pack", stream, nb, 3);
         kf.qt = qt.p;
@@ -900,7 +956,7 @@ hm_status hmatrix_build(hm_kdtree t, hm_structure s, const double* d_points, con
       // 0.15 tol^2 of BF16 rounding (mixed form)
       const bool mixed = opt.precision == HM_PREC_MIXED;
       TruncWork tw;
-      if ((st = trunc_rank<W>(bp, hst, dprobs.p, dst.p, ws.p, (mixed ? 0.35 : 0.45) * opt.tol * opt.tol,
+      if ((st = trunc_rank<W>(bp, hst, dprobs.p, dst.p, (mixed ? 0.35 : 0.45) * opt.tol * opt.tol,
                               mixed ? 0.15 * opt.tol * opt.tol : 0.0, &tw, stream)))
         return st;
       HM_CUDA(cudaMemcpyAsync(hst.data(), dst.p, sizeof(ProbState) * nb, cudaMemcpyDeviceToHost, stream));
@@ -982,8 +1038,8 @@ hm_status hmatrix_build(hm_kdtree t, hm_structure s, const double* d_points, con
       HM_CUDA(cudaMemcpyAsync(ddu.p, du.data(), sizeof(long long) * nb, cudaMemcpyHostToDevice, stream));
       HM_CUDA(cudaMemcpyAsync(ddv.p, dv.data(), sizeof(long long) * nb, cudaMemcpyHostToDevice, stream));
       static_assert(kTR == 64, "trunc_pack's tiles are the sketch's row tiles");
-      if ((st = trunc_pack<W>(dprobs.p, dst.p, ws.p, tw, drows.p, items_rows.size(), dcols.p, items_cols.size(), ddu.p,
-                              ddv.p, chunk.p, stream)))
+      if ((st = trunc_pack<W>(dprobs.p, dst.p, tw, drows.p, items_rows.size(), dcols.p, items_cols.size(), ddu.p, ddv.p,
+                              chunk.p, stream)))
         return st;
       if (!dens.empty()) {
         if ((st = ddi.alloc_async(dens.size(), stream))) return st;
@@ -1109,7 +1165,8 @@ hm_status hmatrix_build(hm_kdtree t, hm_structure s, const double* d_points, con
     for (long long i = 0; i < nprob; ++i) {
       if (rank[i] <= 0) continue;
       const Prob& P = probs[i];
-      mp.push_back(MxPair{P.level, P.r0, P.m, P.c0, P.n, rank[i], std::min(rhis[i], rank[i]), fu[i], fv[i]});
+      mp.push_back(
+          MxPair{P.level, P.r0, P.m, P.c0, P.n, rank[i], std::min(rhis[i], rank[i]), fu[i], fv[i], P.v, P.u});
     }
     std::vector<MxDenseIn> md;
     for (const DenseBlock& db : h->h_dense) md.push_back(MxDenseIn{db.r0, db.m, db.c0, db.n, db.D});

@@ -67,24 +67,44 @@ struct PhaseTrace {
   }
 };
 
+// ---- device memory (hm_memory.cu) ---------------------------------------------
+// Blocks below kPoolMax come from a pool of the library's own (one per device),
+// about 5 us each once its memory is mapped; larger ones from cudaMalloc.
+// Mapping and unmapping is what costs: cudaMalloc + cudaFree take 0.7 ms at 80
+// MB and 12 ms at 11 GB as a median and up to 1 s on a shared host, the
+// stream-ordered pool 6.5 ms/GB each way, and with no memory kept at least 0.25
+// ms for every allocation after a synchronisation.  (A 2^17-point build spent
+// 75 of its 200 ms there.)  The pool keeps at most kPoolKeep bytes that are not
+// in use, a fortieth of the device's memory; hm_release_memory hands them
+// back, and so does an allocation that fails.  Safe from any thread.
+constexpr size_t kPoolMax = size_t(1) << 30, kPoolKeep = size_t(4) << 30;
+// On the current device (*dev): usable on every stream on return; in the order of s.
+cudaError_t dev_alloc(void** p, size_t bytes, int* dev);
+cudaError_t dev_alloc_async(void** p, size_t bytes, cudaStream_t s, int* dev);
+void dev_free(void* p, size_t bytes, int dev);  // after all work of the device, as cudaFree
+void dev_free_async(void* p, size_t bytes, cudaStream_t s, int dev);
+
 // ---- device buffer RAII -----------------------------------------------------
-// Long-lived buffers use cudaMalloc; temporaries of a build step pass a stream
-// and come from the stream-ordered pool (cudaMallocAsync / cudaFreeAsync), so
-// freeing them neither synchronises the device nor returns memory to the OS.
+// alloc: long-lived buffers.  alloc_async: temporaries of a build step, used
+// and released in the order of one stream.
 template <typename T>
 struct DevBuf {
   T* p = nullptr;
   size_t n = 0;
   cudaStream_t s = nullptr;
   bool async = false;
+  int dev = 0;
   DevBuf() = default;
   DevBuf(const DevBuf&) = delete;
   DevBuf& operator=(const DevBuf&) = delete;
-  DevBuf(DevBuf&& o) noexcept : p(o.p), n(o.n), s(o.s), async(o.async) { o.p = nullptr; o.n = 0; }
+  DevBuf(DevBuf&& o) noexcept : p(o.p), n(o.n), s(o.s), async(o.async), dev(o.dev) {
+    o.p = nullptr;
+    o.n = 0;
+  }
   DevBuf& operator=(DevBuf&& o) noexcept {
     if (this != &o) {
       release();
-      p = o.p; n = o.n; s = o.s; async = o.async;
+      p = o.p; n = o.n; s = o.s; async = o.async; dev = o.dev;
       o.p = nullptr; o.n = 0;
     }
     return *this;
@@ -94,38 +114,34 @@ struct DevBuf {
     release();
     async = false;
     if (count == 0) return HM_OK;
-    cudaError_t e = cudaMalloc(reinterpret_cast<void**>(&p), count * sizeof(T));
-    if (e != cudaSuccess) {
-      p = nullptr;
-      cudaGetLastError();
-      return fail(HM_ERR_NOMEM, "cudaMalloc of " + std::to_string(count * sizeof(T)) +
-                                    " bytes failed: " + cudaGetErrorString(e));
-    }
-    n = count;
-    return HM_OK;
+    return take(dev_alloc(reinterpret_cast<void**>(&p), count * sizeof(T), &dev), count);
   }
   hm_status alloc_async(size_t count, cudaStream_t stream) {
     release();
     async = true;
     s = stream;
     if (count == 0) return HM_OK;
-    cudaError_t e = cudaMallocAsync(reinterpret_cast<void**>(&p), count * sizeof(T), stream);
+    return take(dev_alloc_async(reinterpret_cast<void**>(&p), count * sizeof(T), stream, &dev), count);
+  }
+  void release() {
+    if (p) {
+      if (async) dev_free_async(p, n * sizeof(T), s, dev);
+      else dev_free(p, n * sizeof(T), dev);
+    }
+    p = nullptr;
+    n = 0;
+  }
+
+ private:
+  hm_status take(cudaError_t e, size_t count) {
     if (e != cudaSuccess) {
       p = nullptr;
       cudaGetLastError();
-      return fail(HM_ERR_NOMEM, "cudaMallocAsync of " + std::to_string(count * sizeof(T)) +
+      return fail(HM_ERR_NOMEM, "device allocation of " + std::to_string(count * sizeof(T)) +
                                     " bytes failed: " + cudaGetErrorString(e));
     }
     n = count;
     return HM_OK;
-  }
-  void release() {
-    if (p) {
-      if (async) cudaFreeAsync(p, s);
-      else cudaFree(p);
-    }
-    p = nullptr;
-    n = 0;
   }
 };
 

@@ -390,6 +390,28 @@ hm_status matvec_plan_build(hm_hmatrix h, int nrhs_cap, cudaStream_t stream) {
   nrhs_cap = 16;
   P.nrhs_cap = nrhs_cap;
   P.num_leaves = nleaf;
+  // projection scratch of one pass, for whichever product runs (the mixed
+  // form's panels: passes of up to 128 right-hand sides; the FP32 form's
+  // panels or per-block kernels: 16)
+  auto vectors = [&](long long scratch) -> hm_status {
+    HM_TRY(P.T.alloc(std::max<long long>(scratch, 1)));
+    HM_TRY(P.Xp.alloc((size_t)h->n * pass_width(h)));
+    return P.Yp.alloc((size_t)h->n * pass_width(h));
+  };
+  if (h->mx.enabled) {
+    // the panel products have their plan (mixed_build); the lists below serve
+    // the per-block kernels, and a schedule that selects those builds them
+    P.lr.release();
+    P.p1.release();
+    P.multi.release();
+    P.groups.release();
+    P.leaf_ptr.release();
+    P.leaf_blk.release();
+    P.dense.release();
+    P.leaf_dptr.release();
+    P.leaf_dblk.release();
+    return vectors(h->mx.scratch_floats(h->mx.fmt == 0 ? 8 : 1));
+  }
   // device block list: blocks of rank above 128 become pieces of at most
   // 128 columns (U and V sliced alike), whose products add up
   std::vector<LRBlock> lr;
@@ -491,14 +513,7 @@ hm_status matvec_plan_build(hm_hmatrix h, int nrhs_cap, cudaStream_t stream) {
   HM_TRY(P.dense.alloc(std::max<size_t>(h->h_dense.size(), 1)));
   HM_TRY(P.leaf_dptr.alloc(nleaf + 1));
   HM_TRY(P.leaf_dblk.alloc(dblk.size()));
-  // projection scratch of one pass, for whichever product runs (the mixed
-  // form's panels: passes of up to 128 right-hand sides; the FP32 form's
-  // panels or per-block kernels: 16)
-  const long long scratch =
-      h->mx.enabled ? h->mx.scratch_floats(h->mx.fmt == 0 ? 8 : 1) : tk + part;
-  HM_TRY(P.T.alloc(std::max<long long>(scratch, 1)));
-  HM_TRY(P.Xp.alloc((size_t)h->n * pass_width(h)));
-  HM_TRY(P.Yp.alloc((size_t)h->n * pass_width(h)));
+  HM_TRY(vectors(tk + part));
   auto up = [&](void* dst, const void* src, size_t bytes) -> hm_status {
     if (bytes) HM_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, stream));
     return HM_OK;

@@ -894,6 +894,61 @@ __global__ void k_mx_conv_dense(const MxDense* __restrict__ dense, const long lo
   store[(D.lo + (long long)rt * D.nct + ct) * 32 + lane] = l;
 }
 
+// A stored pair's columns in the panels: factor columns fu, fv at panel columns
+// bu + ., bv + . (the first kl of them from colL on, the others from colH on).
+struct PairColumns {
+  const float *fu, *fv;
+  long long bu, bv;
+  int m, n, k, kl;
+  int colL_u, colH_u, colL_v, colH_v;
+};
+
+// Column sources and the projection's column map, one warp per pair: Y_u += fu
+// (fv^T X_v) and Y_v += fv (fu^T X_u), so the two columns are each other's mirror.
+__global__ void k_pair_columns(const PairColumns* __restrict__ pairs, int npairs, const float** __restrict__ colsrc,
+                               int* __restrict__ mirror) {
+  const int i = (int)(((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+  if (i >= npairs) return;
+  const PairColumns q = pairs[i];
+  for (int c = threadIdx.x & 31; c < q.k; c += 32) {
+    const long long cu = q.bu + (c < q.kl ? q.colL_u + c : q.colH_u + c - q.kl);
+    const long long cv = q.bv + (c < q.kl ? q.colL_v + c : q.colH_v + c - q.kl);
+    colsrc[cu] = q.fu + (size_t)c * q.m;
+    colsrc[cv] = q.fv + (size_t)c * q.n;
+    mirror[cv] = (int)cu;
+    mirror[cu] = (int)cv;
+  }
+}
+
+// Where each column's projection goes (MxPlan::tslot, and tslot_tc in the BF16
+// format): the position of its mirror column, or of itself for a padding column.
+__global__ void k_tslot(const MxPanel* __restrict__ panels, int np, const int* __restrict__ mirror, long long ncols,
+                        bool f32, int* __restrict__ tslot, int2* __restrict__ tslot_tc) {
+  const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (c >= ncols) return;
+  const int m = mirror[c];
+  const long long e = m >= 0 ? m : c;
+  if (f32) {  // the destination's global column (its T words follow from it)
+    tslot[c] = m >= 0 ? (int)e : -1 - (int)e;
+    return;
+  }
+  int lo = 0, hi = np - 1;  // the panel of column e
+  while (lo < hi) {
+    const int mid = (lo + hi + 1) >> 1;
+    if (panels[mid].t0 * 8 <= e)
+      lo = mid;
+    else
+      hi = mid - 1;
+  }
+  const MxPanel& P = panels[lo];
+  const int l = (int)(e - P.t0 * 8), j = l >> 3, cc = l & 7;
+  // (word << 1) | no-low-part
+  const int own = (int)(t_word(P.tw0, P.nctl, l) << 1) | (j >= P.nctl ? 1 : 0);
+  tslot[c] = m >= 0 ? own : -1 - own;
+  const int2 tc = make_int2((int)((P.tb0 + j) * 8 + cc), j < P.nctl ? (int)((P.tb0 + P.nct + j) * 8 + cc) : -1);
+  tslot_tc[c] = m >= 0 ? tc : make_int2(-1 - tc.x, tc.y);
+}
+
 template <class T>
 hm_status upload(DevBuf<T>& b, const std::vector<T>& v, cudaStream_t s) {
   HM_TRY(b.alloc(std::max<size_t>(v.size(), 1)));
@@ -952,39 +1007,51 @@ hm_status mixed_build(hm_hmatrix_s* h, const std::vector<MxPair>& pairs, const s
   struct Side {
     int pair, side;  // side 0: fu (row cluster), 1: fv (column cluster)
   };
-  std::vector<std::vector<Side>> members;
-  std::vector<int> plevel, pcl;
+  std::vector<int> plevel, pcl, first(1, 0);  // first: members per panel, then their prefix sums
   std::vector<int> panel_u(pairs.size(), -1), panel_v(pairs.size(), -1);
   for (size_t i = 0; i < pairs.size(); ++i) {
     const MxPair& q = pairs[i];
     if (q.k <= 0) continue;
     for (int side = 0; side < 2; ++side) {
-      const int a = side ? cluster_of(q.level, q.c0, q.n) : cluster_of(q.level, q.r0, q.m);
+      int a = side ? q.cv : q.cu;
+      if (a < 0) a = side ? cluster_of(q.level, q.c0, q.n) : cluster_of(q.level, q.r0, q.m);
       const size_t id = ((size_t)1 << q.level) - 1 + a;
       if (pan_of[id] < 0) {
-        pan_of[id] = (int)members.size();
-        members.emplace_back();
+        pan_of[id] = (int)plevel.size();
+        first.push_back(0);
         plevel.push_back(q.level);
         pcl.push_back(a);
       }
-      members[pan_of[id]].push_back(Side{(int)i, side});
+      ++first[pan_of[id] + 1];
       (side ? panel_v : panel_u)[i] = pan_of[id];
     }
   }
-  const int np = (int)members.size();
+  const int np = (int)plevel.size();
+  for (int p = 0; p < np; ++p) first[p + 1] += first[p];
+  std::vector<Side> members(first[np]);  // panel p's at [first[p], first[p + 1]), in pair order
+  {
+    std::vector<int> at(first.begin(), first.end() - 1);
+    for (size_t i = 0; i < pairs.size(); ++i) {
+      if (panel_u[i] < 0) continue;
+      members[at[panel_u[i]]++] = Side{(int)i, 0};
+      members[at[panel_v[i]]++] = Side{(int)i, 1};
+    }
+  }
   std::vector<MxPanel> panels(np);
   std::vector<int> colL_u(pairs.size()), colH_u(pairs.size()), colL_v(pairs.size()), colH_v(pairs.size());
   long long tiles = 0, t_tiles = 0, t_words = 0, t_blocks = 0;
   for (int p = 0; p < np; ++p) {
     long long sl = 0, sh_ = 0;
-    for (const Side& m : members[p]) {
+    for (int e = first[p]; e < first[p + 1]; ++e) {
+      const Side& m = members[e];
       const int kl = f32 ? 0 : pairs[m.pair].khi;
       sl += kl;
       sh_ += pairs[m.pair].k - kl;
     }
     const int KL = (int)((sl + 7) / 8 * 8), KH = (int)((sh_ + 7) / 8 * 8);
     long long al = 0, ah = KL;
-    for (const Side& m : members[p]) {
+    for (int e = first[p]; e < first[p + 1]; ++e) {
+      const Side& m = members[e];
       const MxPair& q = pairs[m.pair];
       const int kl = f32 ? 0 : q.khi;
       (m.side ? colL_v : colL_u)[m.pair] = (int)al;
@@ -1019,23 +1086,14 @@ hm_status mixed_build(hm_hmatrix_s* h, const std::vector<MxPair>& pairs, const s
   // column sources and the projection's column map
   if ((long long)t_tiles * 8 > 0x7fffffffll || (!f32 && t_words >= (1ll << 30)))
     return fail(HM_ERR_UNSUPPORTED, "panel form: too many factor columns");
-  std::vector<const float*> colsrc((size_t)t_tiles * 8, nullptr);
-  std::vector<int> mirror((size_t)t_tiles * 8, -1);  // partner column (an involution)
+  std::vector<PairColumns> pcols;
+  pcols.reserve(pairs.size());
   long long bytes_lr = 0;
   for (size_t i = 0; i < pairs.size(); ++i) {
     const MxPair& q = pairs[i];
     if (q.k <= 0) continue;
-    const int pu = panel_u[i], pv = panel_v[i];
-    const long long bu = panels[pu].t0 * 8, bv = panels[pv].t0 * 8;
-    const int kl = f32 ? 0 : q.khi;
-    for (int c = 0; c < q.k; ++c) {
-      const int cu = c < kl ? colL_u[i] + c : colH_u[i] + c - kl;
-      const int cv = c < kl ? colL_v[i] + c : colH_v[i] + c - kl;
-      colsrc[bu + cu] = q.fu + (size_t)c * q.m;
-      colsrc[bv + cv] = q.fv + (size_t)c * q.n;
-      mirror[bv + cv] = (int)(bu + cu);  // Y_u += fu (fv^T X_v)
-      mirror[bu + cu] = (int)(bv + cv);  // Y_v += fv (fu^T X_u)
-    }
+    pcols.push_back(PairColumns{q.fu, q.fv, panels[panel_u[i]].t0 * 8, panels[panel_v[i]].t0 * 8, q.m, q.n, q.k,
+                                f32 ? 0 : q.khi, colL_u[i], colH_u[i], colL_v[i], colH_v[i]});
     bytes_lr += f32 ? 4ll * (q.m + q.n) * q.k : 2ll * (q.m + q.n) * (q.k + q.khi);
   }
   std::vector<MxLoc> locs;
@@ -1104,28 +1162,30 @@ hm_status mixed_build(hm_hmatrix_s* h, const std::vector<MxPair>& pairs, const s
   HM_TRY(upload(M.pan_of, pan_of, s));
   HM_TRY(upload(M.tile_leaf, tile_leaf, s));
   HM_TRY(upload(M.leaf_tile0, leaf_tile0, s));
-  // BF16 format: (word << 1) | no-low-part of the destination; FP32 format:
-  // the destination's global column (its T words follow from it)
-  std::vector<int> own(mirror.size()), tslot(mirror.size());
-  for (const MxPanel& P : panels)
-    for (int c = 0; c < P.nct * 8; ++c)
-      own[P.t0 * 8 + c] = f32 ? (int)(P.t0 * 8 + c)
-                              : (int)(t_word(P.tw0, P.nctl, c) << 1) | ((c >> 3) >= P.nctl ? 1 : 0);
-  for (size_t c = 0; c < mirror.size(); ++c) tslot[c] = mirror[c] >= 0 ? own[mirror[c]] : -1 - own[c];
-  HM_TRY(upload(M.tslot, tslot, s));
+  const size_t ncols = (size_t)t_tiles * 8;
+  DevBuf<const float*> colsrc;  // per panel column: its factor column, null for padding
+  {
+    DevBuf<PairColumns> dpc;
+    DevBuf<int> mirror;  // partner column (an involution), -1 for padding
+    HM_TRY(upload(dpc, pcols, s));
+    HM_TRY(colsrc.alloc(std::max<size_t>(ncols, 1)));
+    HM_TRY(mirror.alloc(std::max<size_t>(ncols, 1)));
+    HM_TRY(M.tslot.alloc(std::max<size_t>(ncols, 1)));
+    HM_TRY(M.tslot_tc.alloc(f32 ? 1 : std::max<size_t>(ncols, 1)));
+    if (ncols > 0) {
+      HM_CUDA(cudaMemsetAsync(colsrc.p, 0, sizeof(const float*) * ncols, s));
+      HM_CUDA(cudaMemsetAsync(mirror.p, 0xff, sizeof(int) * ncols, s));
+      k_pair_columns<<<(unsigned)((pcols.size() * 32 + 255) / 256), 256, 0, s>>>(dpc.p, (int)pcols.size(), colsrc.p,
+                                                                               mirror.p);
+      HM_LAUNCH_CHECK();
+      k_tslot<<<(unsigned)((ncols + 255) / 256), 256, 0, s>>>(M.panels.p, np, mirror.p, (long long)ncols, f32,
+                                                            M.tslot.p, M.tslot_tc.p);
+      HM_LAUNCH_CHECK();
+    }
+    HM_CUDA(cudaStreamSynchronize(s));
+  }
   if (!f32) {
-    // 128-column passes on tcgen05: the T blocks' column map, and phase 2's
-    // blocks of 4 row tiles with their sources
-    std::vector<int2> own_tc(mirror.size()), tslot_tc(mirror.size());
-    for (const MxPanel& P : panels)
-      for (int c = 0; c < P.nct * 8; ++c) {
-        const int j = c >> 3, cc = c & 7;
-        own_tc[P.t0 * 8 + c] = make_int2((int)((P.tb0 + j) * 8 + cc),
-                                         j < P.nctl ? (int)((P.tb0 + P.nct + j) * 8 + cc) : -1);
-      }
-    for (size_t c = 0; c < mirror.size(); ++c)
-      tslot_tc[c] = mirror[c] >= 0 ? own_tc[mirror[c]] : make_int2(-1 - own_tc[c].x, own_tc[c].y);
-    HM_TRY(upload(M.tslot_tc, tslot_tc, s));
+    // 128-column passes on tcgen05: phase 2's blocks of 4 row tiles with their sources
     std::vector<P2Step> steps;
     std::vector<int> step_ptr(1, 0);
     const int tend = M.p2_tile0 + M.p2_tiles;
@@ -1188,12 +1248,11 @@ hm_status mixed_build(hm_hmatrix_s* h, const std::vector<MxPair>& pairs, const s
   M.bytes_p2 = bytes_lr + bytes_dense;
 
   if (f32) {
-    HM_TRY(fp32_convert(h, colsrc, dense, s));
+    HM_TRY(fp32_convert(h, colsrc.p, dense, s));
     HM_CUDA(cudaStreamSynchronize(s));
     M.enabled = true;
     return HM_OK;
   }
-  DevBuf<const float*> dcol;
   DevBuf<long long> dstart;
   if (np > 0) {
     std::vector<long long> start(np);
@@ -1202,11 +1261,10 @@ hm_status mixed_build(hm_hmatrix_s* h, const std::vector<MxPair>& pairs, const s
       start[p] = tot;
       tot += (long long)panels[p].nrt * panels[p].nct;
     }
-    HM_TRY(upload(dcol, colsrc, s));
     HM_TRY(upload(dstart, start, s));
     if (tot > 0) {
       k_mx_conv_panels<<<(unsigned)((tot * 32 + 255) / 256), 256, 0, s>>>(
-          M.panels.p, dstart.p, np, tot, dcol.p, M.tile_leaf.p, M.leaf_tile0.p, h->tree->offsets.p, M.store.p);
+          M.panels.p, dstart.p, np, tot, colsrc.p, M.tile_leaf.p, M.leaf_tile0.p, h->tree->offsets.p, M.store.p);
       HM_LAUNCH_CHECK();
     }
     HM_CUDA(cudaStreamSynchronize(s));

@@ -176,6 +176,7 @@ struct MxPair {  // one stored low-rank pair (u rows, v columns) = fu fv^T, and 
   int level, r0, m, c0, n, k, khi;
   const float* fu;  // m x k, column-major
   const float* fv;  // n x k, column-major
+  int cu = -1, cv = -1;  // row and column cluster at that level (-1: found from the rows)
 };
 
 struct MxDenseIn {
@@ -223,8 +224,7 @@ int mixed_find_loc(hm_hmatrix_s* h, const float* key);
 
 // The FP32 format (hm_fp32.cu): tile conversion of the panels and dense
 // blocks, and one pass of nr <= 16 right-hand sides.
-hm_status fp32_convert(hm_hmatrix_s* h, const std::vector<const float*>& colsrc, const std::vector<MxDense>& dense,
-                       cudaStream_t s);
+hm_status fp32_convert(hm_hmatrix_s* h, const float* const* colsrc, const std::vector<MxDense>& dense, cudaStream_t s);
 hm_status fp32_run_panel(hm_hmatrix_s* h, int nr, const float* X, int ldx, float* Y, int ldy, float* scratch,
                          const int* perm, cudaStream_t s, KernelMarks* km);
 

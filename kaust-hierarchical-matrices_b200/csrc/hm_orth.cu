@@ -77,7 +77,6 @@ struct OrthArgs {
   const Prob* probs;
   ProbState* st;
   const int* ids;
-  void* ws;
   int bs;
   int kcap;
   double thresh2;
@@ -177,8 +176,8 @@ __global__ void __launch_bounds__(NT) k_orth(OrthArgs a) {
   const int row0 = min(ld, rank * slice), rows = min(ld, row0 + slice) - row0;
   const int nch = max(1, (rows + RW - 1) / RW);
   const bool resident = nch == 1;
-  W* Q = reinterpret_cast<W*>(a.ws) + P.qoff + row0;
-  W* Y = reinterpret_cast<W*>(a.ws) + P.yoff + row0;
+  W* Q = reinterpret_cast<W*>(P.q) + row0;
+  W* Y = reinterpret_cast<W*>(P.y) + row0;
   const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
   const int cgi = t & 7;
   int k = S.k;
@@ -573,11 +572,11 @@ hm_status orth_plan(const std::vector<Prob>& probs, OrthPlan* plan, cudaStream_t
 }
 
 template <typename W>
-hm_status orth_round(const OrthPlan& plan, const Prob* probs, ProbState* st, W* ws, int bs, double thresh2,
+hm_status orth_round(const OrthPlan& plan, const Prob* probs, ProbState* st, int bs, double thresh2,
                      cudaStream_t s) {
   constexpr int kTall = tall_rows<W>();
   for (const OrthPlan::Class& c : plan.classes) {
-    OrthArgs a{probs, st, plan.ids.p + c.first, ws, bs, c.kcap, thresh2};
+    OrthArgs a{probs, st, plan.ids.p + c.first, bs, c.kcap, thresh2};
     if (c.cluster > 1)
       HM_TRY((launch<W, 256, kTall, true>(c, a, s)));
     else if (c.rows <= 64)
@@ -592,7 +591,7 @@ hm_status orth_round(const OrthPlan& plan, const Prob* probs, ProbState* st, W* 
 
 template hm_status orth_plan<float>(const std::vector<Prob>&, OrthPlan*, cudaStream_t);
 template hm_status orth_plan<double>(const std::vector<Prob>&, OrthPlan*, cudaStream_t);
-template hm_status orth_round<float>(const OrthPlan&, const Prob*, ProbState*, float*, int, double, cudaStream_t);
-template hm_status orth_round<double>(const OrthPlan&, const Prob*, ProbState*, double*, int, double, cudaStream_t);
+template hm_status orth_round<float>(const OrthPlan&, const Prob*, ProbState*, int, double, cudaStream_t);
+template hm_status orth_round<double>(const OrthPlan&, const Prob*, ProbState*, int, double, cudaStream_t);
 
 }  // namespace hm

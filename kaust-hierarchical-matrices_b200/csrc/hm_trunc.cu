@@ -59,8 +59,8 @@ struct Row4 {  // four consecutive rows of one column
 // (upper triangle).
 template <typename W, int KT, int NW>
 __global__ void __launch_bounds__(32 * NW) k_gram(const int2* __restrict__ items, const Prob* __restrict__ probs,
-                                                  const ProbState* __restrict__ st, const W* __restrict__ ws,
-                                                  const long long* __restrict__ goff, double* __restrict__ G) {
+                                                  const ProbState* __restrict__ st, const long long* __restrict__ goff,
+                                                  double* __restrict__ G) {
   constexpr int RS = KT == 128 ? 32 : 64;  // rows staged at a time
   constexpr int LD = RS + 4;               // a half-warp's 4 columns x 4 rows fall into 16 banks
   constexpr int NT = 32 * NW;
@@ -71,7 +71,7 @@ __global__ void __launch_bounds__(32 * NW) k_gram(const int2* __restrict__ items
   const Prob P = probs[it.x];
   const int k = st[it.x].k, ld = ara_ld(P.n);
   const int row0 = it.y * kGramRows, row1 = min(ld, row0 + kGramRows);
-  const W* B = ws + P.boff;
+  const W* B = reinterpret_cast<const W*>(P.b);
   const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
   const int nt = (k + 7) >> 3, ntiles = nt * (nt + 1) / 2;
   // this warp's tiles (a <= b), numbered row by row of the upper triangle
@@ -408,16 +408,16 @@ __global__ void __launch_bounds__(4 * KT) k_eig(const int* __restrict__ ids, con
 // are one 256-byte run of a basis column.
 template <typename W, int SIDE>
 __global__ void __launch_bounds__(128) k_pack(const int2* __restrict__ items, const Prob* __restrict__ probs,
-                                              const ProbState* __restrict__ st, const W* __restrict__ ws,
-                                              const long long* __restrict__ woff, const float* __restrict__ Wr,
-                                              const long long* __restrict__ at, float* __restrict__ dst) {
+                                              const ProbState* __restrict__ st, const long long* __restrict__ woff,
+                                              const float* __restrict__ Wr, const long long* __restrict__ at,
+                                              float* __restrict__ dst) {
   __shared__ __align__(16) float wsh[kTruncMax * 32];  // [k][32]
   const int2 it = items[blockIdx.x];
   const int p = it.x, k = st[p].k, r = st[p].r;
   if (at[p] < 0 || r <= 0) return;
   const Prob P = probs[p];
   const int rows = SIDE ? P.n : P.m, ld = ara_ld(rows);
-  const W* src = ws + (SIDE ? P.boff : P.qoff);
+  const W* src = reinterpret_cast<const W*>(SIDE ? P.b : P.q);
   float* out = dst + at[p];
   const int t = threadIdx.x;
   if (k > kTruncMax) {  // kept as sampled (W_r = I)
@@ -477,11 +477,11 @@ constexpr size_t eig_smem() {
 }
 
 template <typename W, int KT, int NW>
-hm_status launch_gram(const int2* items, size_t count, const Prob* probs, const ProbState* st, const W* ws,
+hm_status launch_gram(const int2* items, size_t count, const Prob* probs, const ProbState* st,
                       const long long* goff, double* G, cudaStream_t s) {
   if (!count) return HM_OK;
   HM_CUDA(cudaFuncSetAttribute(k_gram<W, KT, NW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gram_smem<KT>()));
-  k_gram<W, KT, NW><<<(unsigned)count, 32 * NW, gram_smem<KT>(), s>>>(items, probs, st, ws, goff, G);
+  k_gram<W, KT, NW><<<(unsigned)count, 32 * NW, gram_smem<KT>(), s>>>(items, probs, st, goff, G);
   HM_LAUNCH_CHECK();
   return HM_OK;
 }
@@ -506,7 +506,7 @@ hm_status upload(DevBuf<T>& d, const std::vector<T>& v, cudaStream_t s) {
 
 template <typename W>
 hm_status trunc_rank(const std::vector<Prob>& bp, const std::vector<ProbState>& hst, const Prob* probs, ProbState* st,
-                     const W* ws, double tol2, double rbudget, TruncWork* tw, cudaStream_t s) {
+                     double tol2, double rbudget, TruncWork* tw, cudaStream_t s) {
   const size_t nb = bp.size();
   std::vector<long long> goff(nb, 0), woff(nb, 0);
   std::vector<int2> items[3];
@@ -543,11 +543,11 @@ hm_status trunc_rank(const std::vector<Prob>& bp, const std::vector<ProbState>& 
   HM_TRY(G.alloc_async(std::max<size_t>(gtot, 1), s));
   HM_TRY(tw->w.alloc_async(std::max<size_t>(wtot, 1), s));
   const int2* it = ditems.p;
-  HM_TRY((launch_gram<W, 32, 4>(it, items[0].size(), probs, st, ws, dgoff.p, G.p, s)));
+  HM_TRY((launch_gram<W, 32, 4>(it, items[0].size(), probs, st, dgoff.p, G.p, s)));
   it += items[0].size();
-  HM_TRY((launch_gram<W, 64, 4>(it, items[1].size(), probs, st, ws, dgoff.p, G.p, s)));
+  HM_TRY((launch_gram<W, 64, 4>(it, items[1].size(), probs, st, dgoff.p, G.p, s)));
   it += items[1].size();
-  HM_TRY((launch_gram<W, 128, 8>(it, items[2].size(), probs, st, ws, dgoff.p, G.p, s)));
+  HM_TRY((launch_gram<W, 128, 8>(it, items[2].size(), probs, st, dgoff.p, G.p, s)));
   const int* id = dids.p;
   // the widest first: their CTAs run the longest
   HM_TRY(launch_eig<128>(id + ids[0].size() + ids[1].size(), ids[2].size(), probs, st, dgoff.p, G.p, *tw, tol2, rbudget, s));
@@ -557,24 +557,23 @@ hm_status trunc_rank(const std::vector<Prob>& bp, const std::vector<ProbState>& 
 }
 
 template <typename W>
-hm_status trunc_pack(const Prob* probs, const ProbState* st, const W* ws, const TruncWork& tw, const int2* rows,
-                     size_t nrows, const int2* cols, size_t ncols, const long long* dst_u, const long long* dst_v,
+hm_status trunc_pack(const Prob* probs, const ProbState* st, const TruncWork& tw, const int2* rows, size_t nrows,
+                     const int2* cols, size_t ncols, const long long* dst_u, const long long* dst_v,
                      float* dst, cudaStream_t s) {
-  if (nrows) k_pack<W, 0><<<(unsigned)nrows, 128, 0, s>>>(rows, probs, st, ws, tw.woff.p, tw.w.p, dst_u, dst);
+  if (nrows) k_pack<W, 0><<<(unsigned)nrows, 128, 0, s>>>(rows, probs, st, tw.woff.p, tw.w.p, dst_u, dst);
   HM_LAUNCH_CHECK();
-  if (ncols) k_pack<W, 1><<<(unsigned)ncols, 128, 0, s>>>(cols, probs, st, ws, tw.woff.p, tw.w.p, dst_v, dst);
+  if (ncols) k_pack<W, 1><<<(unsigned)ncols, 128, 0, s>>>(cols, probs, st, tw.woff.p, tw.w.p, dst_v, dst);
   HM_LAUNCH_CHECK();
   return HM_OK;
 }
 
 template hm_status trunc_rank<float>(const std::vector<Prob>&, const std::vector<ProbState>&, const Prob*, ProbState*,
-                                     const float*, double, double, TruncWork*, cudaStream_t);
+                                     double, double, TruncWork*, cudaStream_t);
 template hm_status trunc_rank<double>(const std::vector<Prob>&, const std::vector<ProbState>&, const Prob*, ProbState*,
-                                      const double*, double, double, TruncWork*, cudaStream_t);
-template hm_status trunc_pack<float>(const Prob*, const ProbState*, const float*, const TruncWork&, const int2*, size_t,
-                                     const int2*, size_t, const long long*, const long long*, float*, cudaStream_t);
-template hm_status trunc_pack<double>(const Prob*, const ProbState*, const double*, const TruncWork&, const int2*,
-                                      size_t, const int2*, size_t, const long long*, const long long*, float*,
-                                      cudaStream_t);
+                                      double, double, TruncWork*, cudaStream_t);
+template hm_status trunc_pack<float>(const Prob*, const ProbState*, const TruncWork&, const int2*, size_t, const int2*,
+                                     size_t, const long long*, const long long*, float*, cudaStream_t);
+template hm_status trunc_pack<double>(const Prob*, const ProbState*, const TruncWork&, const int2*, size_t, const int2*,
+                                      size_t, const long long*, const long long*, float*, cudaStream_t);
 
 }  // namespace hm

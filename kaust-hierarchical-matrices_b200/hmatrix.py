@@ -154,6 +154,12 @@ def version():
     return lib().hm_version().decode()
 
 
+def release_memory():
+    """Hand back the device memory that the library keeps for its next objects
+    (hm_release_memory); objects in use are not touched."""
+    _check(lib().hm_release_memory())
+
+
 def generate_dataset(n, d, seed=1234, out=None, stream=None):
     """Points in SoA layout p[dim*n + i] (float64 CUDA tensor of n*d)."""
     import torch
