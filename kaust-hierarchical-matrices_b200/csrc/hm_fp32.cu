@@ -504,7 +504,7 @@ hm_status fp32_convert(hm_hmatrix_s* h, const float* const* colsrc, const std::v
 // One pass of nr <= 16 right-hand sides in tree order; scratch holds
 // scratch_floats(1) floats: X fragments, chunk partials, T.
 hm_status fp32_run_panel(hm_hmatrix_s* h, int nr, const float* X, int ldx, float* Y, int ldy, float* scratch,
-                         const int* perm, cudaStream_t s, KernelMarks* km) {
+                         const int* permx, const int* permy, cudaStream_t s, KernelMarks* km) {
   MxPlan& M = h->mx;
   if (nr < 1 || nr > 16) return fail(HM_ERR_INVALID, "FP32 panel product: a pass holds 1 to 16 right-hand sides");
   uint4* Xf = reinterpret_cast<uint4*>(scratch);
@@ -514,7 +514,7 @@ hm_status fp32_run_panel(hm_hmatrix_s* h, int nr, const float* X, int ldx, float
   const long long xbytes = 4ll * h->n * 16 * 2;  // the X fragments, hi + lo
   if (M.num_tiles > 0) {
     k_fp_split_x<<<(M.num_tiles + 3) / 4, 128, 0, s>>>(X, ldx, nr, M.num_tiles, M.tile_leaf.p, M.leaf_tile0.p,
-                                                       leaf_off, perm, Xf);
+                                                       leaf_off, permx, Xf);
     HM_LAUNCH_CHECK();
     if (km) km->mark("k_fp_split_x", 4ll * h->n * nr + xbytes, s);
   }
@@ -534,7 +534,7 @@ hm_status fp32_run_panel(hm_hmatrix_s* h, int nr, const float* X, int ldx, float
       constexpr int NB = decltype(nb)::value, SP = decltype(sp)::value;
       k_fp_p2<NB, SP><<<(unsigned)M.p2_tiles, 32 * SP, 0, s>>>(
           M.p2_tile0, M.p2_tile0 + M.p2_tiles, h->depth, M.tile_leaf.p, M.leaf_tile0.p, leaf_off, M.pan_of.p,
-          M.panels.p, M.store.p, T, M.leaf_dptr.p, M.leaf_dblk.p, M.dense.p, Xf, perm, Y, ldy, nr);
+          M.panels.p, M.store.p, T, M.leaf_dptr.p, M.leaf_dblk.p, M.dense.p, Xf, permy, Y, ldy, nr);
     };
     auto p2_shared = [&](auto nb) {
       const int sp = p2_share(M.p2_tiles, 6000);
@@ -552,7 +552,7 @@ hm_status fp32_run_panel(hm_hmatrix_s* h, int nr, const float* X, int ldx, float
     HM_LAUNCH_CHECK();
     if (km) km->mark("k_fp_p2", M.bytes_p2 + xbytes + 4ll * h->n * nr, s);
   }
-  if (h->diag_fly) HM_TRY(diag_fly_panel(h, nr, X, ldx, Y, ldy, s, km));  // (perm is null then)
+  if (h->diag_fly) HM_TRY(diag_fly_panel(h, nr, X, ldx, Y, ldy, s, km));  // (no permutation then)
   return HM_OK;
 }
 

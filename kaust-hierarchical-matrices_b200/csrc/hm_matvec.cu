@@ -257,24 +257,21 @@ __global__ void __launch_bounds__(32 * kWarpsPerCta) k_p2(const int2* groups, in
   }
 }
 
-__global__ void k_gather_rows(const float* X, int ldx, const int* perm, int n, int nrhs, float* Xp) {
-  long long tot = (long long)n * nrhs;
-  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < tot;
-       e += (long long)gridDim.x * blockDim.x) {
-    int i = (int)(e % n), c = (int)(e / n);
-    Xp[(size_t)c * n + i] = X[(size_t)c * ldx + perm[i]];
-  }
+// Tree order <-> original order, one column after another (blockIdx.y), so
+// that the column being scattered stays in L2 until its sectors are whole.
+__global__ void k_gather_rows(const float* __restrict__ X, int ldx, const int* __restrict__ perm, int n,
+                              float* __restrict__ Xp) {
+  const size_t c = blockIdx.y;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+    Xp[c * n + i] = X[c * ldx + perm[i]];
 }
 
-__global__ void k_scatter_rows(const float* Yp, const int* perm, int n, int nrhs, float* Y, int ldy) {
-  long long tot = (long long)n * nrhs;
-  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < tot;
-       e += (long long)gridDim.x * blockDim.x) {
-    int i = (int)(e % n), c = (int)(e / n);
-    Y[(size_t)c * ldy + perm[i]] = Yp[(size_t)c * n + i];
-  }
+__global__ void k_scatter_rows(const float* __restrict__ Yp, const int* __restrict__ perm, int n,
+                               float* __restrict__ Y, int ldy) {
+  const size_t c = blockIdx.y;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+    Y[c * ldy + perm[i]] = Yp[c * n + i];
 }
-
 
 // FP64 vectors of the reference's interface: X (double, ldx; rows gathered
 // through perm when perm != null) narrowed into Xp (float, ld n) ...
@@ -354,9 +351,9 @@ __global__ void __launch_bounds__(kFlyT) k_diag_fly(const int* __restrict__ leaf
 // One pass of nr <= pass_width(h) right-hand sides (X, Y in tree order); T:
 // projection scratch (FP32 form: 16 x kpad per block, then the chunk
 // partials; mixed form: see mixed_run_panel).
-hm_status run_panel(hm_hmatrix h, int nr, const float* X, int ldx, float* Y, int ldy, float* T, const int* perm,
-                    cudaStream_t s, KernelMarks* km) {
-  if (h->mx.enabled) return mixed_run_panel(h, nr, X, ldx, Y, ldy, T, perm, s, km);
+hm_status run_panel(hm_hmatrix h, int nr, const float* X, int ldx, float* Y, int ldy, float* T, const int* permx,
+                    const int* permy, cudaStream_t s, KernelMarks* km) {
+  if (h->mx.enabled) return mixed_run_panel(h, nr, X, ldx, Y, ldy, T, permx, permy, s, km);
   MatvecPlan& P = h->plan;
   float* Tpart = T + P.t_floats;
   if (P.num_p1 > 0) {
@@ -549,22 +546,33 @@ hm_status hmatvec(hm_hmatrix h, int trans, int nrhs, const float* X, int ldx, fl
     int ldxt = ldx;
     float* Yt = Yout;
     int ldyt = ldy;
-    // the panel products read X and write Y through the permutation; the
-    // others (and diagonal blocks from coordinates, which read X after Y is
-    // written) work on permuted copies
-    const bool fused = h->mx.enabled && !h->diag_fly;
-    const int* perm = original_order && fused ? h->tree->perm.p : nullptr;
-    if (original_order && !fused) {
-      k_gather_rows<<<592, 256, 0, stream>>>(Xin, ldx, h->tree->perm.p, n, nr, P.Xp.p);
+    // The panel products read X through the permutation, and write Y through
+    // it while Y is small (24 MB): single words scattered by all row tiles at
+    // once leave L2 as partial sectors when Y is larger, and a pass that
+    // scatters one column after another is cheaper.  Measured, fused against
+    // the extra pass, over the product in tree order: 2^18 points x 16
+    // right-hand sides +22 against +40 us, 10^6 x 16 +288 against +173 us,
+    // 2^18 x 128 (tcgen05) +750 against +315 us.  The per-block kernels, and
+    // diagonal blocks from coordinates, which read X after Y is written, work
+    // on permuted copies.
+    const bool fuse_x = h->mx.enabled && !h->diag_fly;
+    const bool fuse_y = fuse_x && (long long)n * nr <= (6ll << 20) && nr <= 64;
+    const int* perm = h->tree->perm.p;
+    const dim3 grid((unsigned)std::max(1, std::min((n + 255) / 256, 1184)), (unsigned)nr);
+    if (original_order && !fuse_x) {
+      k_gather_rows<<<grid, 256, 0, stream>>>(Xin, ldx, perm, n, P.Xp.p);
       HM_LAUNCH_CHECK();
       Xt = P.Xp.p;
       ldxt = n;
+    }
+    if (original_order && !fuse_y) {
       Yt = P.Yp.p;
       ldyt = n;
     }
-    HM_TRY(run_panel(h, nr, Xt, ldxt, Yt, ldyt, P.T.p, perm, stream, nullptr));
-    if (original_order && !fused) {
-      k_scatter_rows<<<592, 256, 0, stream>>>(P.Yp.p, h->tree->perm.p, n, nr, Yout, ldy);
+    HM_TRY(run_panel(h, nr, Xt, ldxt, Yt, ldyt, P.T.p, original_order && fuse_x ? perm : nullptr,
+                     original_order && fuse_y ? perm : nullptr, stream, nullptr));
+    if (original_order && !fuse_y) {
+      k_scatter_rows<<<grid, 256, 0, stream>>>(P.Yp.p, perm, n, Yout, ldy);
       HM_LAUNCH_CHECK();
     }
     c0 += nr;
@@ -589,7 +597,7 @@ hm_status hmatvec_f64(hm_hmatrix h, int trans, int nrhs, const double* X, int ld
     const int nr = std::min(pass_width(h), nrhs - c0);
     k_narrow_rows<<<592, 256, 0, stream>>>(X + (size_t)c0 * ldx, ldx, perm, n, nr, P.Xp.p);
     HM_LAUNCH_CHECK();
-    HM_TRY(run_panel(h, nr, P.Xp.p, n, P.Yp.p, n, P.T.p, nullptr, stream, nullptr));
+    HM_TRY(run_panel(h, nr, P.Xp.p, n, P.Yp.p, n, P.T.p, nullptr, nullptr, stream, nullptr));
     k_widen_rows<<<592, 256, 0, stream>>>(P.Yp.p, perm, n, nr, Y + (size_t)c0 * ldy, ldy);
     HM_LAUNCH_CHECK();
     c0 += nr;
@@ -664,7 +672,7 @@ hm_status timed_panel(hm_hmatrix h, int nr, const float* X, int ldx, float* Y, i
   for (auto& x : km->ev) HM_CUDA(cudaEventCreate(&x));
   km->n = 0;
   HM_CUDA(cudaEventRecord(km->ev[0], s));
-  HM_TRY(run_panel(h, nr, X, ldx, Y, ldy, h->plan.T.p, nullptr, s, km));
+  HM_TRY(run_panel(h, nr, X, ldx, Y, ldy, h->plan.T.p, nullptr, nullptr, s, km));
   HM_CUDA(cudaEventSynchronize(km->ev[km->n]));
   return HM_OK;
 }
@@ -700,7 +708,8 @@ extern "C" hm_status hm_hmatvec_noalloc(hm_hmatrix h, int nrhs, const float* X, 
     // the scratch keeps the previous call's contents, which need no clearing:
     // every scratch word the pass reads (X fragments, chunk partials,
     // projections, padding columns as zeros) is written earlier in the pass
-    HM_TRY(hm::run_panel(h, nr, X + (size_t)c0 * ldx, ldx, Y + (size_t)c0 * ldy, ldy, T, nullptr, s, nullptr));
+    HM_TRY(hm::run_panel(h, nr, X + (size_t)c0 * ldx, ldx, Y + (size_t)c0 * ldy, ldy, T, nullptr, nullptr, s,
+                         nullptr));
     c0 += nr;
   }
   return HM_OK;

@@ -30,6 +30,8 @@
 // each short chain of MMAs goes into a zeroed temporary that is added to the
 // running FP32 sum with an ordinary FADD.
 #include <algorithm>
+#include <functional>
+#include <queue>
 #include <type_traits>
 #include <vector>
 
@@ -892,6 +894,15 @@ __global__ void k_mx_conv_dense(const MxDense* __restrict__ dense, const long lo
   split_bf16x2(val(g + 24, cbase), val(g + 24, cbase + 1), h.w, l.w);
   store[(D.hi + (long long)rt * D.nct + ct) * 32 + lane] = h;
   store[(D.lo + (long long)rt * D.nct + ct) * 32 + lane] = l;
+  // the P1 copy: lane (g, t) holds column 8 (g / 2) + 2 (ct % 4) + g % 2 of the
+  // 32-column tile at rows 2t, 2t+1, 2t+8, .. (k_mx_conv_panels' order)
+  const int c1 = leaf_off[y] + 32 * (GC - leaf_tile0[y]) - D.c0 + 8 * (g >> 1) + 2 * (ct & 3) + (g & 1);
+  split_bf16x2(val(2 * t, c1), val(2 * t + 1, c1), h.x, l.x);
+  split_bf16x2(val(2 * t + 8, c1), val(2 * t + 9, c1), h.y, l.y);
+  split_bf16x2(val(2 * t + 16, c1), val(2 * t + 17, c1), h.z, l.z);
+  split_bf16x2(val(2 * t + 24, c1), val(2 * t + 25, c1), h.w, l.w);
+  store[(D.hi1 + (long long)rt * D.nct + ct) * 32 + p1_slot(lane)] = h;
+  store[(D.lo1 + (long long)rt * D.nct + ct) * 32 + p1_slot(lane)] = l;
 }
 
 // A stored pair's columns in the panels: factor columns fu, fv at panel columns
@@ -947,6 +958,27 @@ __global__ void k_tslot(const MxPanel* __restrict__ panels, int np, const int* _
   tslot[c] = m >= 0 ? own : -1 - own;
   const int2 tc = make_int2((int)((P.tb0 + j) * 8 + cc), j < P.nctl ? (int)((P.tb0 + P.nct + j) * 8 + cc) : -1);
   tslot_tc[c] = m >= 0 ? tc : make_int2(-1 - tc.x, tc.y);
+}
+
+// Items in row order dealt to `ctas` CTAs, each to the one with the least work
+// so far: equal shares, and at any time the CTAs work on nearby rows.
+std::vector<int> deal(const std::vector<long long>& cost, int ctas, std::vector<int>* ptr) {
+  using Load = std::pair<long long, int>;
+  std::priority_queue<Load, std::vector<Load>, std::greater<Load>> least;
+  for (int c = 0; c < ctas; ++c) least.push({0, c});
+  std::vector<int> of(cost.size());
+  ptr->assign(ctas + 1, 0);
+  for (size_t i = 0; i < cost.size(); ++i) {
+    const Load l = least.top();
+    least.pop();
+    of[i] = l.second;
+    ++(*ptr)[l.second + 1];
+    least.push({l.first + cost[i], l.second});
+  }
+  for (int c = 0; c < ctas; ++c) (*ptr)[c + 1] += (*ptr)[c];
+  std::vector<int> at(ptr->begin(), ptr->end() - 1), order(cost.size());
+  for (size_t i = 0; i < cost.size(); ++i) order[at[of[i]]++] = (int)i;
+  return order;
 }
 
 template <class T>
@@ -1111,6 +1143,7 @@ hm_status mixed_build(hm_hmatrix_s* h, const std::vector<MxPair>& pairs, const s
   std::vector<MxDense> dense;
   std::vector<std::vector<int>> leaf_d(nleaf);
   long long bytes_dense = 0;
+  M.tc_dense_tiles = 0;
   for (const MxDenseIn& di : dense_in) {
     if (di.m <= 0 || di.n <= 0) continue;
     int xs, xe, ys, ye;
@@ -1129,7 +1162,14 @@ hm_status mixed_build(hm_hmatrix_s* h, const std::vector<MxPair>& pairs, const s
     D.hi = tiles;
     tiles += (long long)D.nrt * D.nct * tu;
     D.lo = tiles;
-    if (!f32) tiles += (long long)D.nrt * D.nct;
+    if (!f32) {
+      const long long nt = (long long)D.nrt * D.nct;
+      tiles += nt;
+      D.hi1 = tiles;
+      D.lo1 = tiles + nt;
+      tiles += 2 * nt;
+      M.tc_dense_tiles += 2 * nt;
+    }
     for (int x = xs; x < xe; ++x) leaf_d[x].push_back((int)dense.size());
     locs.push_back(MxLoc{di.D, 1, (int)dense.size(), di.m, di.n, 0, 0, 0});
     dense.push_back(D);
@@ -1144,7 +1184,9 @@ hm_status mixed_build(hm_hmatrix_s* h, const std::vector<MxPair>& pairs, const s
 
   // ---- upload and convert ----------------------------------------------------
   M.store_tiles = tiles;
-  HM_TRY(M.store.alloc((size_t)std::max<long long>(tiles, 1) * 32));
+  M.zero_tile = tiles;
+  HM_TRY(M.store.alloc((size_t)(tiles + 8) * 32));
+  HM_CUDA(cudaMemsetAsync(M.store.p + tiles * 32, 0, 8 * 512, s));
   M.h_panels = panels;
   p1_shape(M.num_tiles, &M.chunk_tiles, &M.group_tiles);
   // short chunks leave more partials: a matrix whose 16-column pass fits the
@@ -1194,11 +1236,11 @@ hm_status mixed_build(hm_hmatrix_s* h, const std::vector<MxPair>& pairs, const s
       const MxPanel& P = panels[p];
       const long long rb = G0 - P.tile0;  // the panel's row tile of the block's tile 0
       for (int j0 = 0; j0 < P.nctl; j0 += 4)
-        steps.push_back(P2Step{P.hi2 + rb * P.nct + j0, P.lo2 + rb * P.nctl + j0, (P.tb0 + j0) * 128,
+        steps.push_back(P2Step{P.hi1 + rb * P.nct + j0, P.lo1 + rb * P.nctl + j0, (P.tb0 + j0) * 128,
                                (P.tb0 + P.nct + j0) * 128, P.nct, P.nctl,
                                0 | (std::min(4, P.nctl - j0) << 2) | (mask << 8), 0});
       for (int j0 = P.nctl; j0 < P.nct; j0 += 8)
-        steps.push_back(P2Step{P.hi2 + rb * P.nct + j0, -1, (P.tb0 + j0) * 128, -1, P.nct, 0,
+        steps.push_back(P2Step{P.hi1 + rb * P.nct + j0, -1, (P.tb0 + j0) * 128, -1, P.nct, 0,
                                1 | (std::min(8, P.nct - j0) << 2) | (mask << 8), 0});
     };
     for (int G0 = M.p2_tile0; G0 < tend; G0 += 4) {
@@ -1219,7 +1261,7 @@ hm_status mixed_build(hm_hmatrix_s* h, const std::vector<MxPair>& pairs, const s
           const MxDense& D = dense[dblk[q]];
           const long long rb = G0 - D.row_tile0;
           for (int j0 = 0; j0 < D.nct; j0 += 4)
-            steps.push_back(P2Step{D.hi + rb * D.nct + j0, D.lo + rb * D.nct + j0,
+            steps.push_back(P2Step{D.hi1 + rb * D.nct + j0, D.lo1 + rb * D.nct + j0,
                                    (long long)(D.col_tile0 + j0 / 4) * 1024, (long long)(D.col_tile0 + j0 / 4) * 1024 + 512,
                                    D.nct, D.nct, 2 | (4 << 2) | (mask_of(k, k2) << 8), 0});
         }
@@ -1231,6 +1273,13 @@ hm_status mixed_build(hm_hmatrix_s* h, const std::vector<MxPair>& pairs, const s
     HM_TRY(upload(M.p2_steps, steps, s));
     HM_TRY(upload(M.p2_step_ptr, step_ptr, s));
     M.p2_blocks = (int)step_ptr.size() - 1;
+    std::vector<long long> cost(M.p2_blocks);
+    for (int b = 0; b < M.p2_blocks; ++b) cost[b] = step_ptr[b + 1] - step_ptr[b] + 4;
+    std::vector<int> ptr;
+    M.p2_ctas = std::min(M.num_sms, M.p2_blocks);
+    const std::vector<int> order = deal(cost, std::max(1, M.p2_ctas), &ptr);
+    HM_TRY(upload(M.p2_cta_ptr, ptr, s));
+    HM_TRY(upload(M.p2_cta_blocks, order, s));
   }
   HM_TRY(upload(M.dense, dense, s));
   HM_TRY(upload(M.leaf_dptr, dptr, s));
@@ -1479,15 +1528,24 @@ hm_status mixed_schedule(hm_hmatrix_s* h, int chunk_tiles, int group_tiles, int 
       }
     }
     // in row order (the larger unit first among those that start on the same
-    // row tile): the CTAs, each walking every gridDim-th unit, then work on
-    // nearby rows at every level at once, and X's image of those rows is
-    // read from HBM about once for all levels (it stays in L2 between them)
+    // row tile), then dealt to the CTAs: they work on nearby rows at every
+    // level at once, and X's image of those rows is read from HBM about once
+    // for all levels (it stays in L2 between them)
     std::stable_sort(tcu.begin(), tcu.end(), [](const TcUnit& a, const TcUnit& b) {
       return a.xtile != b.xtile ? a.xtile < b.xtile : a.nrt > b.nrt;
     });
     int dev = 0;
     HM_CUDA(cudaGetDevice(&dev));
     HM_CUDA(cudaDeviceGetAttribute(&M.num_sms, cudaDevAttrMultiProcessorCount, dev));
+    std::vector<long long> cost(tcu.size());
+    for (size_t i = 0; i < tcu.size(); ++i) cost[i] = ((tcu[i].flags & 1) ? tcu[i].nrt : (tcu[i].nrt + 1) / 2) + 2;
+    std::vector<int> ptr;
+    M.tc_ctas = std::min<int>(M.num_sms, (int)tcu.size());
+    const std::vector<int> order = deal(cost, std::max(1, M.tc_ctas), &ptr);
+    std::vector<TcUnit> dealt(tcu.size());
+    for (size_t i = 0; i < order.size(); ++i) dealt[i] = tcu[order[i]];
+    tcu.swap(dealt);
+    HM_TRY(upload(M.tc_ptr, ptr, s));
     if (!M.tc_err.p) {
       HM_TRY(M.tc_err.alloc(1));
       HM_CUDA(cudaMemsetAsync(M.tc_err.p, 0, sizeof(int), s));
@@ -1515,9 +1573,9 @@ hm_status mixed_warp_pass(hm_hmatrix_s* h, int nh, int nr, uint4* Xf, float4* S,
                           KernelMarks* km);
 
 hm_status mixed_run_panel(hm_hmatrix_s* h, int nr, const float* X, int ldx, float* Y, int ldy, float* scratch,
-                          const int* perm, cudaStream_t s, KernelMarks* km) {
+                          const int* permx, const int* permy, cudaStream_t s, KernelMarks* km) {
   MxPlan& M = h->mx;
-  if (M.fmt == 1) return fp32_run_panel(h, nr, X, ldx, Y, ldy, scratch, perm, s, km);
+  if (M.fmt == 1) return fp32_run_panel(h, nr, X, ldx, Y, ldy, scratch, permx, permy, s, km);
   if (nr < 1 || nr > 128) return fail(HM_ERR_INVALID, "mixed product: a pass holds 1 to 128 right-hand sides");
   // 16-column parts of this pass: 1, 2, 4 or 8 (the parts past nr are zero)
   const int nh = nr > 64 ? 8 : (nr > 32 ? 4 : (nr > 16 ? 2 : 1));
@@ -1535,17 +1593,16 @@ hm_status mixed_run_panel(hm_hmatrix_s* h, int nr, const float* X, int ldx, floa
   const long long xbytes = 4ll * h->n * 16 * nh;  // the X fragments, hi + lo
   if (M.num_tiles > 0) {
     k_mx_split_x<<<dim3((M.num_tiles + 3) / 4, nh), 128, 0, s>>>(X, ldx, nr, M.num_tiles, M.tile_leaf.p,
-                                                                 M.leaf_tile0.p, leaf_off, perm, Xf, tc ? Xf : nullptr);
+                                                                 M.leaf_tile0.p, leaf_off, permx, Xf, tc ? Xf : nullptr);
     HM_LAUNCH_CHECK();
     if (km) km->mark("k_mx_split_x", 4ll * h->n * nr + xbytes, s);
   }
   if (tc) {
-    HM_TRY(mixed_tc_pass(h, nr, Xf, reinterpret_cast<float*>(S), reinterpret_cast<uint4*>(T), Y, ldy, perm, s,
-                         km));
+    HM_TRY(mixed_tc_pass(h, nr, Xf, reinterpret_cast<float*>(S), reinterpret_cast<uint4*>(T), Y, ldy, s, km));
   } else {
-    HM_TRY(mixed_warp_pass(h, nh, nr, Xf, S, T, xh, sh, th, Y, ldy, perm, s, km));
+    HM_TRY(mixed_warp_pass(h, nh, nr, Xf, S, T, xh, sh, th, Y, ldy, permy, s, km));
   }
-  if (h->diag_fly)  // the diagonal from coordinates, 16 columns at a time (perm is null then)
+  if (h->diag_fly)  // the diagonal from coordinates, 16 columns at a time (no permutation then)
     for (int c0 = 0; c0 < nr; c0 += 16)
       HM_TRY(diag_fly_panel(h, std::min(16, nr - c0), X + (size_t)c0 * ldx, ldx, Y + (size_t)c0 * ldy, ldy, s, km));
   return HM_OK;

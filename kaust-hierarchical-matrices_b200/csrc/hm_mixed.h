@@ -78,7 +78,7 @@ struct TcUnit {
 // A rows of the block's tiles that the source does not cover (mask bit k
 // clear) are zero.
 struct P2Step {
-  long long a_hi, a_lo;  // P2 tile (512-byte units) of the block's tile 0 at the step's first column tile
+  long long a_hi, a_lo;  // P1 tile (512-byte units) of the block's tile 0 at the step's first column tile
   long long b_hi, b_lo;  // 16-byte offset of B: T blocks (kinds 0, 1) or X's image (kind 2)
   int a_stride, a_stride_lo;  // tiles per row tile of the source (hi, lo)
   int info;                   // kind | column tiles << 2 | mask << 8
@@ -87,6 +87,8 @@ struct P2Step {
 
 struct MxDense {  // a dense block in P2 order, hi + lo, [row tile][col tile]
   long long hi, lo;
+  long long hi1, lo1;        // BF16 format: a copy in P1 order for 128-column passes; column tile 4 i + c holds
+                             // columns 32 i + 8 (g / 2) + 2 c + g % 2, g = 0..7 (X's image's K order)
   int row_tile0, col_tile0;  // global row tiles of its row and column clusters
   int nrt, nct;              // nct: 8-column tiles, a multiple of 4
   int r0, c0, m, n;
@@ -109,6 +111,8 @@ struct MxPlan {
   int fmt = 0;           // tile format: 0 BF16 hi + lo (mixed form), 1 FP32 in TF32 fragment order (FP32 form)
   DevBuf<uint4> store;  // all BF16 tiles
   long long store_tiles = 0;
+  long long zero_tile = 0;   // eight zero tiles past the last one
+  long long tc_dense_tiles = 0;  // the dense blocks' P1 copies, read by 128-column passes only
   DevBuf<MxPanel> panels;
   int num_panels = 0;
   DevBuf<int> pan_of;      // heap-ordered cluster (2^l - 1 + a) -> panel or -1
@@ -150,12 +154,15 @@ struct MxPlan {
   int tc_chunk_tiles = 32;         // row tiles per tcgen05 phase-1 unit
   DevBuf<int2> mtiles_tc;          // (panel, column tile) of panels of several tcgen05 row chunks
   long long nmt_tc = 0, s_tiles_tc = 0;
-  DevBuf<TcUnit> tc_units;
-  int num_tc_units = 0;
+  DevBuf<TcUnit> tc_units;  // CTA c's units at [tc_ptr[c], tc_ptr[c + 1])
+  DevBuf<int> tc_ptr;
+  int num_tc_units = 0, tc_ctas = 0;
   DevBuf<int2> tslot_tc;
   DevBuf<P2Step> p2_steps;
   DevBuf<int> p2_step_ptr;
   int p2_blocks = 0;
+  DevBuf<int> p2_cta_ptr, p2_cta_blocks;  // CTA c's blocks: p2_cta_blocks[p2_cta_ptr[c] .. p2_cta_ptr[c + 1])
+  int p2_ctas = 0;
   DevBuf<int> tc_err;  // set when a bounded wait of those kernels gave up
   bool tc_pass(int halves) const { return wide_tc && fmt == 0 && halves == 8; }
   // scratch of one 16-column panel of right-hand sides, in floats: X
@@ -194,7 +201,7 @@ hm_status mixed_build(hm_hmatrix_s* h, const std::vector<MxPair>& pairs, const s
 // the chunk reduction, phase 2 (Y, tree order, nr <= 128 columns).
 struct KernelMarks;
 hm_status mixed_tc_pass(hm_hmatrix_s* h, int nr, const uint4* Xtc, float* S, uint4* Tb, float* Y, int ldy,
-                        const int* perm, cudaStream_t s, KernelMarks* km);
+                        cudaStream_t s, KernelMarks* km);
 
 struct KernelMarks;
 
@@ -207,10 +214,10 @@ hm_status mixed_schedule(hm_hmatrix_s* h, int chunk_tiles, int group_tiles, int 
 // One pass of nr <= 128 right-hand sides in tree order (two, four or eight parts of 16
 // when nr > 16: every factor tile is read once for all of them); scratch holds
 // scratch_floats(h) floats, h = 1, 2, 4 or 8 parts.  km (optional) receives an event
-// after each kernel.  perm (optional; null with diag_fly): X and Y are in the
+// after each kernel.  permx, permy (null with diag_fly): X, resp. Y, is in the
 // points' original order, tree row i at row perm[i].
 hm_status mixed_run_panel(hm_hmatrix_s* h, int nr, const float* X, int ldx, float* Y, int ldy, float* scratch,
-                          const int* perm, cudaStream_t s, KernelMarks* km);
+                          const int* permx, const int* permy, cudaStream_t s, KernelMarks* km);
 
 // The FP32 values of the BF16 panels: for each (h_locs index, device
 // destination), the factor or dense block rebuilt column-major from its hi
@@ -226,7 +233,7 @@ int mixed_find_loc(hm_hmatrix_s* h, const float* key);
 // blocks, and one pass of nr <= 16 right-hand sides.
 hm_status fp32_convert(hm_hmatrix_s* h, const float* const* colsrc, const std::vector<MxDense>& dense, cudaStream_t s);
 hm_status fp32_run_panel(hm_hmatrix_s* h, int nr, const float* X, int ldx, float* Y, int ldy, float* scratch,
-                         const int* perm, cudaStream_t s, KernelMarks* km);
+                         const int* permx, const int* permy, cudaStream_t s, KernelMarks* km);
 
 // Phase-1 unit shape of a matrix of `tiles` row tiles.  One warp walks a unit
 // one load latency per row tile, so the tallest unit bounds the phase unless

@@ -20,15 +20,25 @@
 // Columns with low parts take three products per tile (V_hi X_hi, V_hi X_lo,
 // V_lo X_hi), one row tile per step; the others one, two row tiles per step.
 //
-// Warp roles, no CTA-wide barrier in the loop: warp 0 lane 0 copies each
-// step into one of six 32 KB stages (bulk copies, counted in bytes on the
-// stage's "full" mbarrier); warp 1 lane 0 waits for it, issues the step's
-// MMAs and commits them to the stage's "empty" mbarrier; chains of four steps
-// go into one of four TMEM accumulators (128 columns each), committed to its
-// "ready" mbarrier; warps 2-5 (TMEM lanes 32 (w % 4) ..) read a ready accumulator
-// out (tcgen05.ld), add it to their FP32 sums with round-to-nearest adds,
-// and release it.  The tensor core's own sums do not round to nearest, so the
-// chains are kept short: 24 MMAs for columns with low parts, a drift far
+// Warp roles, no CTA-wide barrier in the loop: two copy warps take the steps in
+// turn, each lane one bulk copy into one of six 32 KB stages (counted in bytes
+// on the stage's "full" mbarrier); one lane of the MMA warp waits for it, issues
+// the step's MMAs and commits them to the stage's "empty" mbarrier; chains of
+// four steps go into one of four TMEM accumulators (128 columns each), committed
+// to its "ready" mbarrier; four drain warps (TMEM lanes 32 (w % 4) ..) read a
+// ready accumulator out (tcgen05.ld), add it to their FP32 sums with
+// round-to-nearest adds, and release it.  Units and blocks are dealt to the CTAs
+// in row order, each to the least loaded, and every role holds 32 descriptors at
+// a time, one per lane.
+// What bounds it: instructions.  A step's MMAs take about 400 clocks, but with
+// one copy warp laying out and issuing a phase-2 step's 10-20 copies took 1600
+// clocks, and issuing its MMAs from a loop over K 730; copying 16 bytes per
+// step, three stages or chains of 16 steps changed nothing.  Two copy warps
+// (four, or 8 and 16 drain warps, take issue slots from the MMA warp: 8-20 %
+// slower), straight-line MMA code and 32 descriptors per load give, at 131072
+// mixture points, 0.31 ms for phase 1 (0.38 before) and 0.36 ms for phase 2
+// (1.15 with A rearranged word by word, 0.60 with one copy warp).
+// The tensor core's own sums do not round to nearest, so the chains are kept short: 24 MMAs for columns with low parts, a drift far
 // below the BF16 hi + lo rounding of T.  At a unit's end each drain thread
 // stores its column (its TMEM lane): as T (into the mirror column's slots,
 // split hi + lo or hi only) when the panel is projected in one row chunk,
@@ -45,14 +55,16 @@
 //
 // Phase 2 (k_mx_p2_tc): one CTA per SM walks blocks of 4 row tiles (128
 // rows), D (128 rows x 128 right-hand sides) += U T per ancestor panel and
-// D X per dense block, M = 128, N = 128.  A = the factor tiles as stored (P2
-// order: lane (g,t) holds rows g + 8 w, w = 0..3, at columns 2t, 2t+1), each
-// 4-byte word copied by cp.async to its row of the core-matrix image; rows of
-// the block's tiles that a source does not cover are zero.  Dense blocks take
-// their columns in X's row order rho so that B is X's image of the column
-// cluster's tile.  Panels' columns with low parts take three products per 16
-// columns, 32 columns per step; the others one per 16 columns, 64 per step;
-// dense blocks three per 16 columns, 32 per step.
+// D X per dense block, M = 128, N = 128.  A = the P1 tiles of phase 1 again,
+// read as an M-major operand: a tile's column is 32 rows in 64 contiguous
+// bytes, so the K-major image of V^T is the M-major image of U and the copy
+// engine moves it as it is; the rows of D come out in the tiles' order rho and
+// go to their place at the store.  (Rearranging the other tile order by 4-byte
+// cp.async with 27 copy warps took 1.15 ms at 131072 mixture points.)  Dense blocks keep a copy in the
+// same order for these passes, their columns in X's row order rho so that B
+// is X's image of the column cluster's tile.  Panels' columns with low parts
+// take three products per 16 columns, 32 columns per step; the others one per
+// 16 columns, 64 per step; dense blocks three per 16 columns, 32 per step.
 #include "hm_hmatrix.h"
 #include "hm_mixed.h"
 #include "hm_mma.cuh"
@@ -69,7 +81,11 @@ constexpr uint32_t kIdescBmn = tc_idesc_bf16(128, 128) | (1u << 16);  // B MN-ma
 constexpr int kP1Stages = 6;
 constexpr int kP1Bufs = 4;       // TMEM accumulators of 128 columns (all 512)
 constexpr int kP1Chain = 4;      // steps per MMA chain
-constexpr int kP1Threads = 192;  // copy warp 0, MMA warp 1, drain warps 2-5
+constexpr int kDrainWarps = 4;  // drain warps of either phase (a multiple of 4: one per 32 TMEM lanes)
+constexpr int kDrainCols = 512 / kDrainWarps;        // right-hand sides per drain warp
+constexpr int kCopyWarps = 2;  // copy warp w takes every kCopyWarps-th step from w on
+constexpr int kMmaWarp = kCopyWarps, kDrainWarp0 = kCopyWarps + 1;
+constexpr int kTcThreads = 32 * (kDrainWarp0 + kDrainWarps);
 // shared memory: stages, then mbarriers full[S], empty[S], ready[B], free[B],
 // done; then the TMEM address and the abort flag
 constexpr int kP1BarBytes = 8 * (2 * kP1Stages + 2 * kP1Bufs + 1);
@@ -94,34 +110,36 @@ __device__ __forceinline__ void split8(const float* v, uint4& hi, uint4& lo) {
 
 // Drain thread m (the unit's column m, its TMEM lane) of a finished unit: T
 // or the chunk's partial S (column c of S tile i at floats 128 (8 i + c)),
-// all 128 right-hand sides.
-__device__ __forceinline__ void p1_store(const TcUnit& U, const float (&acc)[128], const int2* __restrict__ tslot_tc,
-                                         float* __restrict__ S, uint4* __restrict__ Tb, int m) {
+// right-hand sides R0 .. R0 + 8 NQ - 1.
+template <int NQ>
+__device__ __forceinline__ void p1_store(long long out_tile, int nct, int flags, const float (&acc)[8 * NQ], int q0,
+                                         int2 e, float* __restrict__ S, uint4* __restrict__ Tb, int m) {
   const int jt = m >> 3, c = m & 7;
-  if (jt >= U.nct) return;
-  if (U.flags & 2) {
-    const int2 e = __ldg(tslot_tc + (U.out + jt) * 8 + c);
+  if (jt >= nct) return;
+  if (flags & 2) {
     const bool pad = e.x < 0;  // a padding column: zeros into its own slots
     const long long hp = pad ? -1 - (long long)e.x : e.x;
     const uint4 z = make_uint4(0u, 0u, 0u, 0u);
 #pragma unroll
-    for (int q = 0; q < 16; ++q) {
+    for (int q = 0; q < NQ; ++q) {
       uint4 hi, lo;
       split8(acc + 8 * q, hi, lo);
-      Tb[tb_word(hp, q)] = pad ? z : hi;
-      if (e.y >= 0) Tb[tb_word(e.y, q)] = pad ? z : lo;
+      Tb[tb_word(hp, q0 + q)] = pad ? z : hi;
+      if (e.y >= 0) Tb[tb_word(e.y, q0 + q)] = pad ? z : lo;
     }
   } else {
-    float4* out = reinterpret_cast<float4*>(S + ((U.out + jt) * 8 + c) * 128);
+    float4* out = reinterpret_cast<float4*>(S + ((out_tile + jt) * 8 + c) * 128) + 2 * q0;
 #pragma unroll
-    for (int q = 0; q < 32; ++q) out[q] = make_float4(acc[4 * q], acc[4 * q + 1], acc[4 * q + 2], acc[4 * q + 3]);
+    for (int q = 0; q < 2 * NQ; ++q) out[q] = make_float4(acc[4 * q], acc[4 * q + 1], acc[4 * q + 2], acc[4 * q + 3]);
   }
 }
 
-__device__ __forceinline__ int p1_step_tiles(const TcUnit& U, int r) { return (U.flags & 1) ? 1 : min(2, U.nrt - r); }
+__device__ __forceinline__ int p1_step_tiles(int flags, int left) { return (flags & 1) ? 1 : min(2, left); }
 
-__global__ void __launch_bounds__(kP1Threads, 1)
-    k_mx_p1_tc(const TcUnit* __restrict__ units, int nunits, const uint4* __restrict__ store,
+// CTA c's units are [cta_ptr[c], cta_ptr[c + 1]).  Every role holds 32 units'
+// descriptors at a time, one per lane.
+__global__ void __launch_bounds__(kTcThreads, 1)
+    k_mx_p1_tc(const TcUnit* __restrict__ units, const int* __restrict__ cta_ptr, const uint4* __restrict__ store,
                const uint4* __restrict__ Xtc, const int2* __restrict__ tslot_tc, float* __restrict__ S,
                uint4* __restrict__ Tb, int* __restrict__ err) {
   extern __shared__ __align__(1024) unsigned char smem[];
@@ -138,7 +156,7 @@ __global__ void __launch_bounds__(kP1Threads, 1)
     }
     for (int i = 0; i < kP1Bufs; ++i) {
       mbar_init(ready + 8u * i, 1);
-      mbar_init(freeb + 8u * i, 128);
+      mbar_init(freeb + 8u * i, kDrainWarps);
     }
     mbar_init(done, 1);
     *abort_flag = 0;
@@ -152,162 +170,188 @@ __global__ void __launch_bounds__(kP1Threads, 1)
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *reinterpret_cast<volatile uint32_t*>(slot);
-  const int stride = gridDim.x;
+  const int u0 = cta_ptr[blockIdx.x], u1 = cta_ptr[blockIdx.x + 1];
   bool failed = false;
   auto give_up = [&]() {
     failed = true;
     *abort_flag = 1;
   };
 
-  if (warp == 0) {
-    if (lane == 0) {  // ---- producer: bulk copies of each step
-      long long j = 0;
-      int u = blockIdx.x;
-      TcUnit U;
-      if (u < nunits) U = units[u];
-      while (u < nunits && !failed) {
-        TcUnit nxt;
-        if (u + stride < nunits) nxt = units[u + stride];
-        const bool lo = U.flags & 1;
-        const uint32_t abytes = (uint32_t)U.nct * 512u;
-        for (int r = 0; r < U.nrt;) {
-          const int nt = p1_step_tiles(U, r), s = (int)(j % kP1Stages);
-          if (j >= kP1Stages &&
-              !mbar_wait_or(empty + 8u * s, (uint32_t)(((j - kP1Stages) / kP1Stages) & 1), abort_flag)) {
-            give_up();
-            break;
-          }
-          const uint32_t base = sbase + (uint32_t)(s * kTcStage), bar = full + 8u * s;
-          mbar_arrive_expect_tx(bar, (uint32_t)nt * (abytes + 8192u) + (lo ? abytes + 8192u : 0u));
-          for (int k = 0; k < nt; ++k) {
-            bulk_g2s(base + (uint32_t)(k * 8192), store + (U.vhi + (long long)(r + k) * U.shi) * 32, abytes, bar);
-            bulk_g2s(base + 16384u + (uint32_t)(k * 8192), Xtc + (size_t)(U.xtile + r + k) * 1024, 8192u, bar);
-          }
-          if (lo) {
-            bulk_g2s(base + 8192u, store + (U.vlo + (long long)r * U.slo) * 32, abytes, bar);
-            bulk_g2s(base + 24576u, Xtc + (size_t)(U.xtile + r) * 1024 + 512, 8192u, bar);
-          }
-          r += nt;
-          ++j;
-        }
-        u += stride;
-        U = nxt;
-      }
-      // every copy issued has landed before the CTA ends (bounded)
-      for (long long jj = j > kP1Stages ? j - kP1Stages : 0; jj < j; ++jj)
-        mbar_wait(full + 8u * (uint32_t)(jj % kP1Stages), (uint32_t)((jj / kP1Stages) & 1), 1000000000ull);
-    }
-  } else if (warp == 1) {
-    if (lane == 0) {  // ---- MMA issuer
-      const uint64_t adesc0 = tc_sdesc_sw64(sbase, 512), bdesc0 = tc_sdesc(sbase, 2048, 128);
-      long long j = 0;
-      int chain = -1;
-      int u = blockIdx.x;
-      TcUnit U;
-      if (u < nunits) U = units[u];
-      while (u < nunits && !failed) {
-        TcUnit nxt;
-        if (u + stride < nunits) nxt = units[u + stride];
-        const bool lo = U.flags & 1;
-        int in_chain = 0;
-        for (int r = 0; r < U.nrt && !failed;) {
-          const int nt = p1_step_tiles(U, r), s = (int)(j % kP1Stages);
-          if (in_chain == 0) {
-            ++chain;
-            if (chain >= kP1Bufs && !mbar_wait_or(freeb + 8u * (uint32_t)(chain % kP1Bufs),
-                                                  (uint32_t)((chain / kP1Bufs - 1) & 1), abort_flag)) {
-              give_up();
+  if (warp < kCopyWarps) {  // ---- producers: one copy per lane
+    // lanes 0, 1: A_hi of row tile r + lane; 2, 3: X_hi; 4: A_lo; 5: X_lo
+    long long j = 0, last = -1;
+    for (int ub = u0; ub < u1 && !failed; ub += 32) {
+      TcUnit W{};
+      if (ub + lane < u1) W = units[ub + lane];
+      const int nu = min(32, u1 - ub);
+      for (int i = 0; i < nu && !failed; ++i) {
+        const int nrt = __shfl_sync(0xffffffffu, W.nrt, i), flags = __shfl_sync(0xffffffffu, W.flags, i);
+        const bool lo = flags & 1;
+        const int per = lo ? 1 : 2, nsteps = (nrt + per - 1) / per;
+        const int first = (int)((warp - j) & (kCopyWarps - 1));  // this warp's first step of the unit
+        if (first < nsteps) {
+          const long long vhi = __shfl_sync(0xffffffffu, W.vhi, i), vlo = __shfl_sync(0xffffffffu, W.vlo, i);
+          const int shi = __shfl_sync(0xffffffffu, W.shi, i), slo = __shfl_sync(0xffffffffu, W.slo, i);
+          const int nct = __shfl_sync(0xffffffffu, W.nct, i), xtile = __shfl_sync(0xffffffffu, W.xtile, i);
+          const uint32_t abytes = (uint32_t)nct * 512u;
+          // this lane's copy: of the step's row tile k, from src0 + tile * step
+          const int k = lo ? 0 : lane & 1;
+          const bool is_x = lane == 2 || lane == 3 || lane == 5;
+          const uint4* src0 = is_x ? Xtc + (size_t)xtile * 1024 + (lane == 5 ? 512 : 0)
+                                   : store + (lane < 2 ? vhi : vlo) * 32;
+          const long long adv = is_x ? 1024 : (long long)(lane < 2 ? shi : slo) * 32;
+          const uint32_t dst = (is_x ? 16384u : 0u) + (uint32_t)((lane < 4 ? lane & 1 : 1) * 8192);
+          const uint32_t size = is_x ? 8192u : abytes;
+          const bool mine = lo ? (lane == 0 || lane == 2 || lane == 4 || lane == 5) : lane < 4;
+          for (int st = first; st < nsteps; st += kCopyWarps) {
+            const long long js = j + st;
+            const int s = (int)(js % kP1Stages), r = st * per, nt = min(per, nrt - r);
+            const uint32_t base = sbase + (uint32_t)(s * kTcStage), bar = full + 8u * s;
+            int ok = 1;
+            if (lane == 0) {
+              if (js >= kP1Stages &&
+                  !mbar_wait_or(empty + 8u * s, (uint32_t)(((js - kP1Stages) / kP1Stages) & 1), abort_flag)) {
+                give_up();
+                ok = 0;
+              } else {
+                mbar_arrive_expect_tx(bar, (uint32_t)(lo ? 2 : nt) * (abytes + 8192u));
+              }
+            }
+            if (!__shfl_sync(0xffffffffu, ok, 0)) {
+              failed = true;
               break;
             }
+            if (mine && k < nt) bulk_g2s(base + dst, src0 + (r + k) * adv, size, bar);
+            last = js;
           }
-          if (!mbar_wait_or(full + 8u * s, (uint32_t)((j / kP1Stages) & 1), abort_flag)) {
+        }
+        j += nsteps;
+      }
+    }
+    // Every step's MMAs wait for its copies, so these have landed when the MMAs
+    // are done; after a wait that gave up, the copies this warp may still have
+    // in flight are waited for here (bounded).
+    if (failed && lane == 0)
+      for (long long js = last; js >= 0 && js > last - kP1Stages; js -= kCopyWarps)
+        mbar_wait(full + 8u * (uint32_t)(js % kP1Stages), (uint32_t)((js / kP1Stages) & 1), kWaitClocks / 8);
+    __syncwarp();
+  } else if (warp == kMmaWarp) {  // ---- MMA issuer (lane 0; the others hold descriptors)
+    const uint64_t adesc0 = tc_sdesc_sw64(sbase, 512), bdesc0 = tc_sdesc(sbase, 2048, 128);
+    long long j = 0;
+    int chain = -1;
+    for (int ub = u0; ub < u1 && !failed; ub += 32) {
+      int w_nrt = 0, w_flags = 0;
+      if (ub + lane < u1) w_nrt = units[ub + lane].nrt, w_flags = units[ub + lane].flags;
+      const int nu = min(32, u1 - ub);
+      for (int i = 0; i < nu && !failed; ++i) {
+        const int nrt = __shfl_sync(0xffffffffu, w_nrt, i), flags = __shfl_sync(0xffffffffu, w_flags, i);
+        const bool lo = flags & 1;
+        int in_chain = 0;
+        for (int r = 0; r < nrt && !failed;) {
+          const int nt = p1_step_tiles(flags, nrt - r), s = (int)(j % kP1Stages);
+          if (in_chain == 0) ++chain;
+          if (lane == 0) {
+            if (in_chain == 0 && chain >= kP1Bufs &&
+                !mbar_wait_or(freeb + 8u * (uint32_t)(chain % kP1Bufs), (uint32_t)((chain / kP1Bufs - 1) & 1),
+                              abort_flag))
+              give_up();
+            if (!failed && !mbar_wait_or(full + 8u * s, (uint32_t)((j / kP1Stages) & 1), abort_flag)) give_up();
+            if (!failed) {
+              tc_fence_after();
+              // descriptors of this stage; an offset of o bytes adds o >> 4 to the start address field
+              const uint64_t da = adesc0 + (uint64_t)((s * kTcStage) >> 4),
+                             db = bdesc0 + (uint64_t)((s * kTcStage) >> 4);
+              const uint32_t d = tmem + (uint32_t)((chain % kP1Bufs) * 128);
+              uint32_t acc = in_chain == 0 ? 0u : 1u;
+              if (lo) {
+#pragma unroll
+                for (int p = 0; p < 3; ++p) {  // V_hi X_hi, V_hi X_lo, V_lo X_hi
+                  const uint32_t pa = p == 2 ? 8192u : 0u, pb = p == 1 ? 24576u : 16384u;
+#pragma unroll
+                  for (int q = 0; q < 2; ++q) {
+                    tc_mma_bf16(d, da + ((pa + (uint32_t)(q * 32)) >> 4), db + ((pb + (uint32_t)(q * 4096)) >> 4),
+                                kIdesc, acc);
+                    acc = 1u;
+                  }
+                }
+              } else {
+                for (int k = 0; k < nt; ++k)
+#pragma unroll
+                  for (int q = 0; q < 2; ++q) {
+                    tc_mma_bf16(d, da + ((uint32_t)(k * 8192 + q * 32) >> 4),
+                                db + ((16384u + (uint32_t)(k * 8192 + q * 4096)) >> 4), kIdesc, acc);
+                    acc = 1u;
+                  }
+              }
+              tc_commit(empty + 8u * s);
+            }
+          }
+          failed = __shfl_sync(0xffffffffu, failed, 0);
+          r += nt;
+          ++j;
+          if (r >= nrt || ++in_chain == kP1Chain) {
+            if (lane == 0 && !failed) tc_commit(ready + 8u * (uint32_t)(chain % kP1Bufs));
+            in_chain = 0;
+          }
+        }
+      }
+    }
+    if (lane == 0) tc_commit(done);  // arrives once every MMA issued above is done
+  } else {  // ---- drain warps: TMEM lanes 32 (warp % 4) .., kDrainCols right-hand sides each
+    const int m = (warp & 3) * 32 + lane, h = (warp - kDrainWarp0) >> 2;
+    const uint32_t mine = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(h * kDrainCols);
+    float acc[kDrainCols];
+#pragma unroll
+    for (int i = 0; i < kDrainCols; ++i) acc[i] = 0.f;
+    int chain = -1;
+    for (int ub = u0; ub < u1 && !failed; ub += 32) {
+      long long w_out = 0;
+      int w_nct = 0, w_nrt = 0, w_flags = 0;
+      if (ub + lane < u1) {
+        const TcUnit& W = units[ub + lane];
+        w_out = W.out, w_nct = W.nct, w_nrt = W.nrt, w_flags = W.flags;
+      }
+      const int nu = min(32, u1 - ub);
+      for (int i = 0; i < nu && !failed; ++i) {
+        const long long out = __shfl_sync(0xffffffffu, w_out, i);
+        const int nct = __shfl_sync(0xffffffffu, w_nct, i), nrt = __shfl_sync(0xffffffffu, w_nrt, i);
+        const int flags = __shfl_sync(0xffffffffu, w_flags, i);
+        // the column's slots, fetched while the unit's steps run
+        int2 e = make_int2(-1, -1);
+        if ((flags & 2) && (m >> 3) < nct) e = __ldg(tslot_tc + (out + (m >> 3)) * 8 + (m & 7));
+        const int nsteps = (flags & 1) ? nrt : (nrt + 1) / 2;
+        const int nchains = (nsteps + kP1Chain - 1) / kP1Chain;
+        for (int c = 0; c < nchains; ++c) {
+          ++chain;
+          const uint32_t b = (uint32_t)(chain % kP1Bufs);
+          if (!warp_wait_or(ready + 8u * b, (uint32_t)((chain / kP1Bufs) & 1), abort_flag)) {
             give_up();
             break;
           }
           tc_fence_after();
-          // descriptors of this stage; an offset of o bytes adds o >> 4 to the start address field
-          const uint64_t da = adesc0 + (uint64_t)((s * kTcStage) >> 4), db = bdesc0 + (uint64_t)((s * kTcStage) >> 4);
-          const uint32_t d = tmem + (uint32_t)((chain % kP1Bufs) * 128);
-          uint32_t acc = in_chain == 0 ? 0u : 1u;
-          if (lo) {
 #pragma unroll
-            for (int p = 0; p < 3; ++p) {  // V_hi X_hi, V_hi X_lo, V_lo X_hi
-              const uint32_t pa = p == 2 ? 8192u : 0u, pb = p == 1 ? 24576u : 16384u;
+          for (int q = 0; q < kDrainCols / 32; ++q) {
+            uint32_t v[32];
+            tc_ld32(mine + b * 128u + (uint32_t)(q * 32), v);
+            tc_wait_ld();
 #pragma unroll
-              for (int q = 0; q < 2; ++q) {
-                tc_mma_bf16(d, da + ((pa + (uint32_t)(q * 32)) >> 4), db + ((pb + (uint32_t)(q * 4096)) >> 4), kIdesc,
-                            acc);
-                acc = 1u;
-              }
-            }
-          } else {
-            for (int k = 0; k < nt; ++k)
-#pragma unroll
-              for (int q = 0; q < 2; ++q) {
-                tc_mma_bf16(d, da + ((uint32_t)(k * 8192 + q * 32) >> 4),
-                            db + ((16384u + (uint32_t)(k * 8192 + q * 4096)) >> 4), kIdesc, acc);
-                acc = 1u;
-              }
+            for (int k = 0; k < 32; ++k) acc[q * 32 + k] += __uint_as_float(v[k]);
           }
-          tc_commit(empty + 8u * s);
-          r += nt;
-          ++j;
-          if (r >= U.nrt || ++in_chain == kP1Chain) {
-            tc_commit(ready + 8u * (uint32_t)(chain % kP1Bufs));
-            in_chain = 0;
-          }
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(freeb + 8u * b);
         }
-        u += stride;
-        U = nxt;
+        if (failed) break;
+        p1_store<kDrainCols / 8>(out, nct, flags, acc, h * (kDrainCols / 8), e, S, Tb, m);
+#pragma unroll
+        for (int k = 0; k < kDrainCols; ++k) acc[k] = 0.f;
       }
-    }
-    if (lane == 0) tc_commit(done);  // arrives once every MMA issued above is done
-  } else {  // ---- drain warps 2-5: TMEM lanes 32 (warp % 4) ..
-    const int m = (warp & 3) * 32 + lane;
-    const uint32_t my_lanes = (uint32_t)((warp & 3) * 32) << 16;
-    float acc[128];
-#pragma unroll
-    for (int i = 0; i < 128; ++i) acc[i] = 0.f;
-    int chain = -1;
-    int u = blockIdx.x;
-    TcUnit U;
-    if (u < nunits) U = units[u];
-    while (u < nunits && !failed) {
-      TcUnit nxt;
-      if (u + stride < nunits) nxt = units[u + stride];
-      const int nsteps = (U.flags & 1) ? U.nrt : (U.nrt + 1) / 2;
-      const int nchains = (nsteps + kP1Chain - 1) / kP1Chain;
-      for (int c = 0; c < nchains; ++c) {
-        ++chain;
-        const uint32_t b = (uint32_t)(chain % kP1Bufs);
-        if (!mbar_wait_or(ready + 8u * b, (uint32_t)((chain / kP1Bufs) & 1), abort_flag)) {
-          give_up();
-          break;
-        }
-        tc_fence_after();
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          uint32_t v[32];
-          tc_ld32(tmem + my_lanes + b * 128u + (uint32_t)(q * 32), v);
-          tc_wait_ld();
-#pragma unroll
-          for (int i = 0; i < 32; ++i) acc[q * 32 + i] += __uint_as_float(v[i]);
-        }
-        tc_fence_before();
-        mbar_arrive(freeb + 8u * b);
-      }
-      if (failed) break;
-      p1_store(U, acc, tslot_tc, S, Tb, m);
-#pragma unroll
-      for (int i = 0; i < 128; ++i) acc[i] = 0.f;
-      u += stride;
-      U = nxt;
     }
   }
   if (failed) atomicExch(err, 1);
   // the tensor memory is released once every MMA is done (thread 0 waits,
   // bounded; the others wait at the barrier)
-  if (tid == 0 && !mbar_wait(done, 0, 10000000000ull)) atomicExch(err, 1);
+  if (tid == 0 && !mbar_wait(done, 0, 5 * kWaitClocks)) atomicExch(err, 1);
   tc_fence_before();
   __syncthreads();
   if (warp == 0) {
@@ -351,69 +395,29 @@ __global__ void k_mx_reduce_tc(const int2* __restrict__ mtiles, long long nmt, c
 }
 
 // ---- phase 2 ------------------------------------------------------------------
-// Warp roles as in phase 1, with 27 copy warps and four drain warps that keep
-// the running sums in tensor memory: A (the factor tiles in
-// P2 order) is rearranged word by word into its core-matrix image by
-// cp.async (4 bytes, any destination); B (T blocks, X's image) comes by bulk
-// copies from producer thread 0.  A producer thread's copies of step j are
-// fenced to the async proxy and announced on the stage's "full" mbarrier
-// kP2Delay steps later, once they have landed (cp.async.wait_group), so that
-// producers do not wait on their own copies.
-// Stage layout (bytes): kind 0: A_hi 0, A_lo 8192, B_hi 16384, B_lo 24576
-// (K blocks of 8 columns 2048 apart); kind 1: A_hi 0, B_hi 16384 (8 K
-// blocks); kind 2: as kind 0, with X's image as B; kind 3: zero A at 0 and B
-// at 16384 (one K chunk).  A: row m = 32 k + g + 8 w at 16 g + 128 (4 k + w)
-// (K-major, SBO 128, LBO 2048); B: T blocks MN-major (right-hand side n at
-// 2 (n % 8) + 128 (n / 8), column c at 16 c; SBO 128, LBO 2048), X's image
-// K-major (n at 16 (n % 8) + 128 (n / 8); SBO 128, LBO 2048).
+// Warp roles as in phase 1.  Stage layout (bytes): kinds 0, 2, 3: A_hi 0 (row
+// tile k at 2048 k), A_lo 8192, B_hi 16384, B_lo 24576; kind 1: A_hi 0 (row
+// tile k at 4096 k), B_hi 16384 (8 K blocks).  A: column tiles as stored (P1
+// order), 512 bytes each, M-major with the 64-byte swizzle: 32 rows of a
+// column are 64 contiguous bytes, the row tiles (LBO) and the groups of 8
+// columns (512 = SBO) apart; row i of a tile is rho(i / 8, i % 8).  B: T blocks
+// MN-major (right-hand side n at 2 (n % 8) + 128 (n / 8), column c at 16 c;
+// SBO 128, LBO 2048), X's image K-major (n at 16 (n % 8) + 128 (n / 8); SBO
+// 128, LBO 2048).  Row tiles outside a step's mask, the odd last column tile
+// of a step and kind 3's operands are copied from the store's zero tiles.
 constexpr int kP2Stages = 6;
-constexpr int kP2Bufs = 2;        // TMEM chain accumulators (columns 0-255); running sums at 256-383
+constexpr int kP2Bufs = 4;       // TMEM accumulators of 128 columns (all 512)
 constexpr int kP2Chain = 4;      // steps per MMA chain
-constexpr int kP2Delay = 3;      // steps between a producer's copies and its arrival
-constexpr int kP2CopyWarps = 27;
-constexpr int kP2Producers = 32 * kP2CopyWarps;  // threads of the copy warps 0-26
-constexpr int kP2Threads = 1024;                 // copy warps 0-26, MMA warp 27, drain warps 28-31
 constexpr int kP2BarBytes = 8 * (2 * kP2Stages + 2 * kP2Bufs + 1);
 constexpr size_t kP2Smem = (size_t)kP2Stages * kTcStage + kP2BarBytes + 16;
+constexpr uint32_t kIdescAmn = kIdesc | (1u << 15);      // A MN-major
+constexpr uint32_t kIdescABmn = kIdescBmn | (1u << 15);  // A and B MN-major
 
-__device__ __forceinline__ void cpa4(uint32_t saddr, const void* g) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(saddr), "l"(g) : "memory");
-}
-__device__ __forceinline__ void cpa4_zero(uint32_t saddr, const void* g) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, 0;\n" ::"r"(saddr), "l"(g) : "memory");
-}
-
-// A's image of the block's 4 row tiles x nk K blocks (column tiles j0 + jj),
-// word W of the tiles per copy thread (tile W / 128, jj-major; word W % 128):
-// word w of lane (g, t) of tile (k, jj) = rows g + 8 w of row tile k at
-// columns 2t, 2t+1 -> 16 g + 128 (4 k + w) + (DENSE ? 4 jj + 2048 t : 4 t +
-// 2048 jj).  Rows of tiles outside the mask, and K blocks cnt .. nk - 1, are
-// zero.  (Measured: more copy warps raise the rate; fewer instructions per
-// copy with fewer warps, or 16-byte zeroing of whole masked row tiles, did not.)
-template <bool DENSE>
-__device__ __forceinline__ void p2_copy_a(uint32_t base, const uint4* __restrict__ store, long long a0, int stride,
-                                          int mask, int cnt, int nk, int pt) {
-  for (int W = pt; W < 512 * nk; W += kP2Producers) {
-    const int it = W >> 7, wi = W & 127, jj = it >> 2, k = it & 3;
-    const int lane = wi >> 2, w = wi & 3, g = lane >> 2, t = lane & 3;
-    const uint32_t dst = base + (uint32_t)(g * 16 + (4 * k + w) * 128) +
-                         (DENSE ? (uint32_t)(4 * jj + t * 2048) : (uint32_t)(4 * t + jj * 2048));
-    if (((mask >> k) & 1) && jj < cnt)
-      cpa4(dst, reinterpret_cast<const uint32_t*>(store + (a0 + (long long)k * stride + jj) * 32) + wi);
-    else
-      cpa4_zero(dst, store);
-  }
-}
-// zero 2 KB blocks [from, to) of a B image at base (16 bytes per copy)
-__device__ __forceinline__ void p2_zero_blocks(uint32_t base, int from, int to, const void* any, int pt) {
-  for (int u = pt + 128 * from; u < 128 * to; u += kP2Producers) cpa16_zero(base + (uint32_t)(u * 16), any);
-}
-
-__global__ void __launch_bounds__(kP2Threads, 1)
-    k_mx_p2_tc(int nblocks, int tile0, int tile_end, const int* __restrict__ step_ptr,
-               const P2Step* __restrict__ steps, const uint4* __restrict__ store, const uint4* __restrict__ Tb,
-               const uint4* __restrict__ Xtc, const int* __restrict__ tile_leaf,
-               const int* __restrict__ leaf_tile0, const int* __restrict__ leaf_off, const int* __restrict__ perm,
+__global__ void __launch_bounds__(kTcThreads, 1)
+    k_mx_p2_tc(const int* __restrict__ cta_ptr, const int* __restrict__ cta_blocks, int tile0, int tile_end,
+               const int* __restrict__ step_ptr, const P2Step* __restrict__ steps, const uint4* __restrict__ store, long long zero_tile,
+               const uint4* __restrict__ Tb, const uint4* __restrict__ Xtc, const int* __restrict__ tile_leaf,
+               const int* __restrict__ leaf_tile0, const int* __restrict__ leaf_off,
                float* __restrict__ Y, int ldy, int nr, int* __restrict__ err) {
   extern __shared__ __align__(1024) unsigned char smem[];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -424,234 +428,215 @@ __global__ void __launch_bounds__(kP2Threads, 1)
   volatile int* abort_flag = reinterpret_cast<volatile int*>(slot + 1);
   if (tid == 0) {
     for (int i = 0; i < kP2Stages; ++i) {
-      mbar_init(full + 8u * i, kP2Producers + 1);  // copy threads, plus thread 0's expect_tx (bulk copies)
+      mbar_init(full + 8u * i, 1);  // thread 0's expect_tx (bulk copies)
       mbar_init(empty + 8u * i, 1);
     }
     for (int i = 0; i < kP2Bufs; ++i) {
       mbar_init(ready + 8u * i, 1);
-      mbar_init(freeb + 8u * i, 128);
+      mbar_init(freeb + 8u * i, kDrainWarps);
     }
     mbar_init(done, 1);
     *abort_flag = 0;
     mbar_init_fence();
   }
   if (warp == 0) {
-    tmem_alloc(smem_u32(slot), 512);
+    tmem_alloc(smem_u32(slot), 128 * kP2Bufs);
     tmem_relinquish();
   }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *reinterpret_cast<volatile uint32_t*>(slot);
-  const int stride = gridDim.x;
+  const int b0 = cta_ptr[blockIdx.x], b1 = cta_ptr[blockIdx.x + 1];
   bool failed = false;
   auto give_up = [&]() {
     failed = true;
     *abort_flag = 1;
   };
 
-  if (warp < kP2CopyWarps) {  // ---- producers
-    const int pt = tid;
-    long long j = 0, arrived = 0;  // steps issued; steps announced
-    for (int b = blockIdx.x; b < nblocks && !failed; b += stride) {
-      const int e = step_ptr[b + 1];
-      P2Step st_next = steps[step_ptr[b]];  // the next step's descriptor, loaded a step ahead
-      for (int i = step_ptr[b]; i < e; ++i) {
-        const P2Step st = st_next;
-        if (i + 1 < e) st_next = steps[i + 1];
-        const int s = (int)(j % kP2Stages);
-        if (j >= kP2Stages &&
-            !mbar_wait_or(empty + 8u * s, (uint32_t)(((j - kP2Stages) / kP2Stages) & 1), abort_flag)) {
-          give_up();
+  if (warp < kCopyWarps) {  // ---- producers: one copy per lane
+    // lanes 0-3: A_hi of row tile k; 4-7: A_lo; 8-11, 12-15: their odd last
+    // column tiles (zeros); 16, 17: B_hi, B_lo; 18, 19: their odd last blocks
+    const uint4* zero = store + zero_tile * 32;
+    const int k = lane & 3;
+    const bool is_b = lane >= 16, is_pad = is_b ? lane >= 18 : lane >= 8;
+    const bool is_lo = is_b ? lane & 1 : (lane >> 2) & 1;
+    const uint32_t dst0 = (is_b ? 16384u : 0u) + (is_lo ? 8192u : 0u);
+    long long j = 0, last = -1;
+    for (int bi = b0; bi < b1 && !failed; ++bi) {
+      const int b = cta_blocks[bi], i0 = step_ptr[b], ns = step_ptr[b + 1] - i0;
+      P2Step W{};  // this warp's next 32 steps, one per lane
+      const int first = (int)((warp - j) & (kCopyWarps - 1));
+      for (int q = 0, st = first; st < ns; ++q, st += kCopyWarps) {
+        const int at = q & 31;
+        if (at == 0 && st + kCopyWarps * lane < ns) W = steps[i0 + st + kCopyWarps * lane];
+        const long long a_hi = __shfl_sync(0xffffffffu, W.a_hi, at), a_lo = __shfl_sync(0xffffffffu, W.a_lo, at);
+        const long long b_hi = __shfl_sync(0xffffffffu, W.b_hi, at), b_lo = __shfl_sync(0xffffffffu, W.b_lo, at);
+        const int s_hi = __shfl_sync(0xffffffffu, W.a_stride, at), s_lo = __shfl_sync(0xffffffffu, W.a_stride_lo, at);
+        const int info = __shfl_sync(0xffffffffu, W.info, at);
+        const long long js = j + st;
+        const int s = (int)(js % kP2Stages);
+        const int kind = info & 3, mask = info >> 8;
+        const int cnt = kind == 3 ? 2 : (info >> 2) & 15, odd = cnt & 1;
+        const bool lo = kind == 0 || kind == 2;
+        const uint32_t base = sbase + (uint32_t)(s * kTcStage), bar = full + 8u * s;
+        const uint32_t rs = kind == 1 ? 4096u : 2048u;
+        const uint32_t ahi = (uint32_t)(512 * cnt), bhi = kind == 2 ? 8192u : (uint32_t)(2048 * cnt);
+        const uint32_t whole = is_b ? bhi : ahi;
+        const uint32_t dst = dst0 + (is_b ? 0u : (uint32_t)k * rs) + (is_pad ? whole : 0u);
+        const uint32_t size = is_pad ? (is_b ? 2048u : 512u) : whole;
+        const bool mine = lane < 20 && (lo || !is_lo) && (odd || !is_pad);
+        const uint4* src = is_b ? (kind == 2 ? Xtc : Tb) + (is_lo ? b_lo : b_hi)
+                                : store + (is_lo ? a_lo + (long long)k * s_lo : a_hi + (long long)k * s_hi) * 32;
+        if (is_pad || kind == 3 || (!is_b && !((mask >> k) & 1))) src = zero;
+        int ok = 1;
+        if (lane == 0) {
+          if (js >= kP2Stages &&
+              !mbar_wait_or(empty + 8u * s, (uint32_t)(((js - kP2Stages) / kP2Stages) & 1), abort_flag)) {
+            give_up();
+            ok = 0;
+          } else {
+            const uint32_t part = 4u * ahi + bhi + (odd ? 4096u : 0u);  // 4 row tiles and B, and the odd zeros
+            mbar_arrive_expect_tx(bar, lo ? 2u * part : part);
+          }
+        }
+        if (!__shfl_sync(0xffffffffu, ok, 0)) {
+          failed = true;
           break;
         }
-        const int kind = st.info & 3, cnt = (st.info >> 2) & 15, mask = st.info >> 8;
-        const int nk = (cnt + 1) & ~1;
-        const uint32_t base = sbase + (uint32_t)(s * kTcStage), bar = full + 8u * s;
-        if (pt == 0) {  // B by bulk copies
-          if (kind == 0) {
-            mbar_arrive_expect_tx(bar, (uint32_t)(2 * cnt * 2048));
-            bulk_g2s(base + 16384u, Tb + st.b_hi, (uint32_t)(cnt * 2048), bar);
-            bulk_g2s(base + 24576u, Tb + st.b_lo, (uint32_t)(cnt * 2048), bar);
-          } else if (kind == 1) {
-            mbar_arrive_expect_tx(bar, (uint32_t)(cnt * 2048));
-            bulk_g2s(base + 16384u, Tb + st.b_hi, (uint32_t)(cnt * 2048), bar);
-          } else if (kind == 2) {
-            mbar_arrive_expect_tx(bar, 16384u);
-            bulk_g2s(base + 16384u, Xtc + st.b_hi, 8192u, bar);
-            bulk_g2s(base + 24576u, Xtc + st.b_lo, 8192u, bar);
-          } else {
-            mbar_arrive(bar);
-          }
-        }
-        if (kind == 0) {
-          p2_copy_a<false>(base, store, st.a_hi, st.a_stride, mask, cnt, nk, pt);
-          p2_copy_a<false>(base + 8192u, store, st.a_lo, st.a_stride_lo, mask, cnt, nk, pt);
-          p2_zero_blocks(base + 16384u, cnt, nk, store, pt);
-          p2_zero_blocks(base + 24576u, cnt, nk, store, pt);
-        } else if (kind == 1) {
-          p2_copy_a<false>(base, store, st.a_hi, st.a_stride, mask, cnt, nk, pt);
-          p2_zero_blocks(base + 16384u, cnt, nk, store, pt);
-        } else if (kind == 2) {
-          p2_copy_a<true>(base, store, st.a_hi, st.a_stride, mask, 4, 4, pt);
-          p2_copy_a<true>(base + 8192u, store, st.a_lo, st.a_stride_lo, mask, 4, 4, pt);
-        } else {
-          p2_zero_blocks(base, 0, 2, store, pt);
-          p2_zero_blocks(base + 16384u, 0, 2, store, pt);
-        }
-        cpa_commit();
-        ++j;
-        if (j - 1 >= kP2Delay) {  // announce step j - 1 - kP2Delay: its copies have landed
-          cpa_wait<kP2Delay>();
-          fence_proxy_async_smem();
-          mbar_arrive(full + 8u * (uint32_t)(arrived % kP2Stages));
-          ++arrived;
-        }
+        if (mine) bulk_g2s(base + dst, src, size, bar);
+        last = js;
       }
+      j += ns;
     }
-    cpa_wait<0>();
-    fence_proxy_async_smem();
-    for (; arrived < j; ++arrived) mbar_arrive(full + 8u * (uint32_t)(arrived % kP2Stages));
-    // the bulk copies issued have landed before the CTA ends (bounded)
-    if (pt == 0)
-      for (long long jj = j > kP2Stages ? j - kP2Stages : 0; jj < j; ++jj)
-        mbar_wait(full + 8u * (uint32_t)(jj % kP2Stages), (uint32_t)((jj / kP2Stages) & 1), 1000000000ull);
-  } else if (warp == kP2CopyWarps) {  // ---- MMA issuer
-    if (lane == 0) {
-      const uint64_t desc0 = tc_sdesc(sbase, 2048, 128);  // A, T blocks and X's image: SBO 128, LBO 2048
-      long long j = 0;
-      int chain = -1;
-      for (int b = blockIdx.x; b < nblocks && !failed; b += stride) {
-        const int e = step_ptr[b + 1];
-        int in_chain = 0;
-        int info_next = steps[step_ptr[b]].info;
-        for (int i = step_ptr[b]; i < e; ++i) {
-          const int info = info_next;
-          if (i + 1 < e) info_next = steps[i + 1].info;
-          const int s = (int)(j % kP2Stages);
-          if (in_chain == 0) {
-            ++chain;
-            if (chain >= kP2Bufs && !mbar_wait_or(freeb + 8u * (uint32_t)(chain % kP2Bufs),
-                                                  (uint32_t)((chain / kP2Bufs - 1) & 1), abort_flag)) {
-              give_up();
-              break;
-            }
-          }
-          if (!mbar_wait_or(full + 8u * s, (uint32_t)((j / kP2Stages) & 1), abort_flag)) {
-            give_up();
-            break;
-          }
-          tc_fence_after();
-          const uint64_t ds = desc0 + (uint64_t)((s * kTcStage) >> 4);  // this stage's start
-          const uint32_t d = tmem + (uint32_t)((chain % kP2Bufs) * 128);
-          uint32_t acc = in_chain == 0 ? 0u : 1u;
-          const int kind = info & 3, cnt = (info >> 2) & 15, nq = (cnt + 1) >> 1;
-          const uint32_t idesc = kind == 2 ? kIdesc : kIdescBmn;  // T blocks are MN-major, X's image K-major
-          auto mma = [&](uint32_t a, uint32_t bb) {
-            tc_mma_bf16(d, ds + (a >> 4), ds + (bb >> 4), idesc, acc);
-            acc = 1u;
-          };
-          if (kind == 0) {
-            for (int q = 0; q < nq; ++q) {
-              const uint32_t o = (uint32_t)(q * 4096);
-              mma(o, 16384u + o);
-              mma(o, 24576u + o);
-              mma(8192u + o, 16384u + o);
-            }
-          } else if (kind == 1) {
-            for (int q = 0; q < nq; ++q) mma((uint32_t)(q * 4096), 16384u + (uint32_t)(q * 4096));
-          } else if (kind == 2) {
-#pragma unroll
-            for (int q = 0; q < 2; ++q) {
-              const uint32_t o = (uint32_t)(q * 4096);
-              mma(o, 16384u + o);
-              mma(o, 24576u + o);
-              mma(8192u + o, 16384u + o);
-            }
-          } else {
-            mma(0u, 16384u);
-          }
-          tc_commit(empty + 8u * s);
-          ++j;
-          if (i + 1 == e || ++in_chain == kP2Chain) {
-            tc_commit(ready + 8u * (uint32_t)(chain % kP2Bufs));
-            in_chain = 0;
-          }
-        }
-      }
-      tc_commit(done);  // arrives once every MMA issued above is done
-    }
-  } else {  // ---- drain warps 28-31: TMEM lanes 32 (warp % 4) .., row m of the block
-    // Each chain is added to the block's running sums kept in tensor memory
-    // (columns 256-383: read, FP32 round-to-nearest add, write back); the last
-    // chain's sums go to Y.  Few registers per thread (at most 64 in a CTA of
-    // 32 warps), so that 27 warps can copy.
-    const int m = (warp & 3) * 32 + lane;
-    const uint32_t my_lanes = (uint32_t)((warp & 3) * 32) << 16;
-    const uint32_t tsum = tmem + my_lanes + 256u;
+    // Every step's MMAs wait for its copies, so these have landed when the MMAs
+    // are done; after a wait that gave up, the copies this warp may still have
+    // in flight are waited for here (bounded).
+    if (failed && lane == 0)
+      for (long long js = last; js >= 0 && js > last - kP2Stages; js -= kCopyWarps)
+        mbar_wait(full + 8u * (uint32_t)(js % kP2Stages), (uint32_t)((js / kP2Stages) & 1), kWaitClocks / 8);
+    __syncwarp();
+  } else if (warp == kMmaWarp) {  // ---- MMA issuer (lane 0; the others hold descriptors)
+    const uint64_t adesc0 = tc_sdesc_sw64_mn(sbase, 2048, 512), adesc1 = tc_sdesc_sw64_mn(sbase, 4096, 512);
+    const uint64_t bdesc0 = tc_sdesc(sbase, 2048, 128);  // T blocks and X's image: SBO 128, LBO 2048
+    long long j = 0;
     int chain = -1;
-    for (int b = blockIdx.x; b < nblocks && !failed; b += stride) {
+    for (int bi = b0; bi < b1 && !failed; ++bi) {
+      const int b = cta_blocks[bi], e = step_ptr[b + 1];
+      int in_chain = 0, w_info = 0;
+      for (int i0 = step_ptr[b], i = i0; i < e && !failed; ++i) {
+        const int at = (i - i0) & 31;
+        if (at == 0 && i + lane < e) w_info = steps[i + lane].info;
+        const int info = __shfl_sync(0xffffffffu, w_info, at);
+        const int s = (int)(j % kP2Stages);
+        if (in_chain == 0) ++chain;
+        if (lane == 0) {
+          if (in_chain == 0 && chain >= kP2Bufs &&
+              !mbar_wait_or(freeb + 8u * (uint32_t)(chain % kP2Bufs), (uint32_t)((chain / kP2Bufs - 1) & 1),
+                            abort_flag))
+            give_up();
+          if (!failed && !mbar_wait_or(full + 8u * s, (uint32_t)((j / kP2Stages) & 1), abort_flag)) give_up();
+          if (!failed) {
+            tc_fence_after();
+            const int kind = info & 3, cnt = (info >> 2) & 15, nq = kind == 3 ? 1 : (cnt + 1) >> 1;
+            // this stage's start; an offset of o bytes adds o >> 4 to the start address field
+            const uint64_t off = (uint64_t)((s * kTcStage) >> 4);
+            const uint64_t da = (kind == 1 ? adesc1 : adesc0) + off, db = bdesc0 + off;
+            const uint32_t d = tmem + (uint32_t)((chain % kP2Bufs) * 128);
+            uint32_t acc = in_chain == 0 ? 0u : 1u;
+            const uint32_t idesc = kind == 2 ? kIdescAmn : kIdescABmn;  // T blocks are MN-major, X's image K-major
+            // 16 columns at a time: two column tiles (1024 bytes of A), two K blocks (4096 of B at 16384)
+            if (kind == 1) {
+#pragma unroll
+              for (int q = 0; q < 4; ++q)
+                if (q < nq) tc_mma_bf16(d, da + q * 64, db + (1024 + q * 256), kIdescABmn, q ? 1u : acc);
+            } else {
+#pragma unroll
+              for (int q = 0; q < 2; ++q)
+                if (q < nq) {
+                  tc_mma_bf16(d, da + q * 64, db + (1024 + q * 256), idesc, q ? 1u : acc);  // U_hi T_hi
+                  if (kind != 3) {
+                    tc_mma_bf16(d, da + q * 64, db + (1536 + q * 256), idesc, 1u);        // U_hi T_lo
+                    tc_mma_bf16(d, da + (512 + q * 64), db + (1024 + q * 256), idesc, 1u);  // U_lo T_hi
+                  }
+                }
+            }
+            tc_commit(empty + 8u * s);
+          }
+        }
+        failed = __shfl_sync(0xffffffffu, failed, 0);
+        ++j;
+        if (i + 1 == e || ++in_chain == kP2Chain) {
+          if (lane == 0 && !failed) tc_commit(ready + 8u * (uint32_t)(chain % kP2Bufs));
+          in_chain = 0;
+        }
+      }
+    }
+    if (lane == 0) tc_commit(done);  // arrives once every MMA issued above is done
+  } else {  // ---- drain warps: TMEM lanes 32 (warp % 4) .., a row of the block and kDrainCols columns each
+    const int m = (warp & 3) * 32 + lane, h = (warp - kDrainWarp0) >> 2;
+    const int in_tile = 8 * ((lane & 7) >> 1) + 2 * (lane >> 3) + (lane & 1);  // rho(lane / 8, lane % 8)
+    const uint32_t mine = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(h * kDrainCols);
+    float acc[kDrainCols];
+#pragma unroll
+    for (int i = 0; i < kDrainCols; ++i) acc[i] = 0.f;
+    int chain = -1;
+    for (int bi = b0; bi < b1 && !failed; ++bi) {
+      const int b = cta_blocks[bi];
       const int nsteps = step_ptr[b + 1] - step_ptr[b];
       const int nchains = (nsteps + kP2Chain - 1) / kP2Chain;
       const int G = tile0 + 4 * b + (m >> 5);
       int row = -1;
       if (G < tile_end) {
         const int x = tile_leaf[G];
-        const int r = leaf_off[x] + 32 * (G - leaf_tile0[x]) + (m & 31);
-        if (r < leaf_off[x + 1]) row = perm ? __ldg(perm + r) : r;
+        const int r = leaf_off[x] + 32 * (G - leaf_tile0[x]) + in_tile;
+        if (r < leaf_off[x + 1]) row = r;
       }
       for (int c = 0; c < nchains; ++c) {
         ++chain;
         const uint32_t bb = (uint32_t)(chain % kP2Bufs);
-        if (!mbar_wait_or(ready + 8u * bb, (uint32_t)((chain / kP2Bufs) & 1), abort_flag)) {
+        if (!warp_wait_or(ready + 8u * bb, (uint32_t)((chain / kP2Bufs) & 1), abort_flag)) {
           give_up();
           break;
         }
         tc_fence_after();
-        const bool first = c == 0, last = c + 1 == nchains;
-        float* yq = Y + (row >= 0 ? row : 0);
-#pragma unroll 1
-        for (int q = 0; q < 8; ++q, yq += (size_t)16 * ldy) {
-          uint32_t v[16];
-          tc_ld16(tmem + my_lanes + bb * 128u + (uint32_t)(q * 16), v);
-          if (!first) {
-            uint32_t sm[16];
-            tc_ld16(tsum + (uint32_t)(q * 16), sm);
-            tc_wait_ld();
 #pragma unroll
-            for (int e = 0; e < 16; ++e) v[e] = __float_as_uint(__uint_as_float(v[e]) + __uint_as_float(sm[e]));
-          } else {
-            tc_wait_ld();
-          }
-          if (!last) {
-            tc_st16(tsum + (uint32_t)(q * 16), v);
-          } else if (row >= 0) {
-            float* y = yq;
+        for (int q = 0; q < kDrainCols / 32; ++q) {
+          uint32_t v[32];
+          tc_ld32(mine + bb * 128u + (uint32_t)(q * 32), v);
+          tc_wait_ld();
 #pragma unroll
-            for (int e = 0; e < 16; ++e, y += ldy)
-              if (q * 16 + e < nr) *y = __uint_as_float(v[e]);
-          }
+          for (int i = 0; i < 32; ++i) acc[q * 32 + i] += __uint_as_float(v[i]);
         }
-        if (!last) tc_wait_st();
         tc_fence_before();
-        mbar_arrive(freeb + 8u * bb);
+        __syncwarp();
+        if (lane == 0) mbar_arrive(freeb + 8u * bb);
       }
+      if (failed) break;
+      if (row >= 0) {
+        float* y = Y + (size_t)(h * kDrainCols) * ldy + row;
+#pragma unroll
+        for (int i = 0; i < kDrainCols; ++i, y += ldy)
+          if (h * kDrainCols + i < nr) *y = acc[i];
+      }
+#pragma unroll
+      for (int i = 0; i < kDrainCols; ++i) acc[i] = 0.f;
     }
   }
   if (failed) atomicExch(err, 1);
-  if (tid == 0 && !mbar_wait(done, 0, 10000000000ull)) atomicExch(err, 1);
+  if (tid == 0 && !mbar_wait(done, 0, 5 * kWaitClocks)) atomicExch(err, 1);
   tc_fence_before();
   __syncthreads();
   if (warp == 0) {
     tc_fence_after();
-    tmem_dealloc(tmem, 512);
+    tmem_dealloc(tmem, 128 * kP2Bufs);
   }
 }
 
 }  // namespace
 
 hm_status mixed_tc_pass(hm_hmatrix_s* h, int nr, const uint4* Xtc, float* S, uint4* Tb, float* Y, int ldy,
-                        const int* perm, cudaStream_t s, KernelMarks* km) {
+                        cudaStream_t s, KernelMarks* km) {
   MxPlan& M = h->mx;
   // the kernels' shared-memory limit, once per device of this process
   static unsigned long long attr_done = 0;
@@ -664,8 +649,7 @@ hm_status mixed_tc_pass(hm_hmatrix_s* h, int nr, const uint4* Xtc, float* S, uin
   }
   const long long xbytes = 4ll * h->n * 128;  // X's image: hi + lo of 128 right-hand sides
   if (M.num_tc_units > 0) {
-    const int grid = std::min(M.num_sms, M.num_tc_units);
-    k_mx_p1_tc<<<grid, kP1Threads, kP1Smem, s>>>(M.tc_units.p, M.num_tc_units, M.store.p, Xtc, M.tslot_tc.p, S, Tb,
+    k_mx_p1_tc<<<M.tc_ctas, kTcThreads, kP1Smem, s>>>(M.tc_units.p, M.tc_ptr.p, M.store.p, Xtc, M.tslot_tc.p, S, Tb,
                                                 M.tc_err.p);
     HM_LAUNCH_CHECK();
     if (km) km->mark("k_mx_p1_tc", M.bytes_p1 + xbytes, s);
@@ -677,10 +661,9 @@ hm_status mixed_tc_pass(hm_hmatrix_s* h, int nr, const uint4* Xtc, float* S, uin
     if (km) km->mark("k_mx_reduce_tc", 4096ll * M.s_tiles_tc + 4096ll * M.nmt_tc, s);
   }
   if (M.p2_blocks > 0) {
-    const int grid = std::min(M.num_sms, M.p2_blocks);
-    k_mx_p2_tc<<<grid, kP2Threads, kP2Smem, s>>>(M.p2_blocks, M.p2_tile0, M.p2_tile0 + M.p2_tiles, M.p2_step_ptr.p,
-                                                M.p2_steps.p, M.store.p, Tb, Xtc, M.tile_leaf.p, M.leaf_tile0.p,
-                                                h->tree->offsets.p, perm, Y, ldy, nr, M.tc_err.p);
+    k_mx_p2_tc<<<M.p2_ctas, kTcThreads, kP2Smem, s>>>(M.p2_cta_ptr.p, M.p2_cta_blocks.p, M.p2_tile0,
+                                                M.p2_tile0 + M.p2_tiles, M.p2_step_ptr.p, M.p2_steps.p, M.store.p, M.zero_tile, Tb, Xtc, M.tile_leaf.p, M.leaf_tile0.p,
+                                                h->tree->offsets.p, Y, ldy, nr, M.tc_err.p);
     HM_LAUNCH_CHECK();
     if (km) km->mark("k_mx_p2_tc", M.bytes_p2 + xbytes + 4ll * h->n * nr, s);
   }

@@ -1,6 +1,6 @@
 // hm_tc.cuh -- Blackwell (sm_100a) tensor-core helpers: tcgen05.mma with the
 // accumulator in tensor memory (TMEM), shared-memory matrix descriptors,
-// mbarriers with bounded waits, and cp.async copies.
+// mbarriers with bounded waits, and bulk copies.
 //
 // Operands sit in shared memory in the canonical K-major layout without
 // swizzle: "core matrices" of 8 rows x 16 bytes (8 BF16 along K), 128
@@ -9,7 +9,7 @@
 // bytes from the descriptor's start address.  One MMA of kind::f16 covers
 // K = 16 (two core matrices along K, LBO apart).
 //
-// Every wait on an mbarrier gives up after a time limit (globaltimer), so a
+// Every wait on an mbarrier gives up after a time limit (SM clocks), so a
 // schedule error ends the kernel with an error word set instead of a hang.
 #pragma once
 #include <cuda_runtime.h>
@@ -18,12 +18,6 @@
 namespace hm {
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-
-__device__ __forceinline__ uint64_t global_ns() {
-  uint64_t t;
-  asm volatile("mov.u64 %0, %%globaltimer;\n" : "=l"(t));
-  return t;
-}
 
 // ---- mbarriers ----------------------------------------------------------------
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
@@ -45,24 +39,30 @@ __device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
       : "memory");
   return ok != 0;
 }
-// Waits for the phase of the given parity to complete; false after limit_ns.
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, uint64_t limit_ns = 2000000000ull) {
+// Waits for the phase of the given parity to complete; false after `limit`
+// SM clocks (about 2 s).
+constexpr long long kWaitClocks = 4000000000ll;
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, long long limit = kWaitClocks) {
   if (mbar_test(bar, parity)) return true;
-  const uint64_t t0 = global_ns();
+  const long long t0 = clock64();
   while (!mbar_test(bar, parity))
-    if (global_ns() - t0 > limit_ns) return false;
+    if (clock64() - t0 > limit) return false;
   return true;
 }
 
 // As mbar_wait, but also gives up as soon as *abort (shared memory) is set.
 __device__ __forceinline__ bool mbar_wait_or(uint32_t bar, uint32_t parity, const volatile int* abort,
-                                             uint64_t limit_ns = 2000000000ull) {
+                                             long long limit = kWaitClocks) {
   if (mbar_test(bar, parity)) return true;
-  const uint64_t t0 = global_ns();
+  const long long t0 = clock64();
   while (!mbar_test(bar, parity)) {
-    if (*abort || global_ns() - t0 > limit_ns) return false;
+    if (*abort || clock64() - t0 > limit) return false;
   }
   return true;
+}
+// The whole warp waits and gives up as one (measured faster than one polling lane).
+__device__ __forceinline__ bool warp_wait_or(uint32_t bar, uint32_t parity, const volatile int* abort) {
+  return __all_sync(0xffffffffu, mbar_wait_or(bar, parity, abort));
 }
 __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(bar) : "memory");
@@ -79,25 +79,6 @@ __device__ __forceinline__ void bulk_g2s(uint32_t dst, const void* src, uint32_t
   asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n" ::"r"(dst),
                "l"(src), "r"(bytes), "r"(bar)
                : "memory");
-}
-
-// ---- cp.async (16 bytes per thread, any shared-memory destination) -------------
-__device__ __forceinline__ void cpa16(uint32_t saddr, const void* g) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(saddr), "l"(g) : "memory");
-}
-// 16 zero bytes (source size 0: nothing is read)
-__device__ __forceinline__ void cpa16_zero(uint32_t saddr, const void* g) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, 0;\n" ::"r"(saddr), "l"(g) : "memory");
-}
-__device__ __forceinline__ void cpa_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cpa_wait() {
-  asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
-}
-// Orders this thread's completed generic-proxy writes to shared memory (the
-// cp.async copies) before later reads by the tensor core (async proxy).
-__device__ __forceinline__ void fence_proxy_async_smem() {
-  asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
 }
 
 // ---- tensor memory ----------------------------------------------------------------
@@ -131,8 +112,17 @@ __device__ __forceinline__ uint64_t tc_sdesc_sw64(uint32_t saddr, uint32_t sbo) 
          (4ull << 61);
 }
 
+// An MN-major operand with the 64-byte swizzle: 32 BF16 along MN are 64
+// contiguous bytes, K rows 64 bytes apart, chunk c of K row r at chunk
+// c ^ ((r >> 1) & 3); LBO = the stride of groups of 32 along MN, SBO = the
+// stride of groups of 8 along K.
+__device__ __forceinline__ uint64_t tc_sdesc_sw64_mn(uint32_t saddr, uint32_t lbo, uint32_t sbo) {
+  return (uint64_t)((saddr >> 4) & 0x3FFFu) | ((uint64_t)((lbo >> 4) & 0x3FFFu) << 16) |
+         ((uint64_t)((sbo >> 4) & 0x3FFFu) << 32) | (1ull << 46) | (4ull << 61);
+}
+
 // Instruction descriptor of kind::f16: D FP32 (bits 4-5 = 1), A and B BF16
-// (bits 7-9 and 10-12 = 1), both K-major (bits 15, 16 = 0), N >> 3 in bits
+// (bits 7-9 and 10-12 = 1), both K-major (bits 15, 16 = 0; 1: MN-major), N >> 3 in bits
 // 17-22, M >> 4 in bits 24-28.
 __host__ __device__ constexpr uint32_t tc_idesc_bf16(int m, int n) {
   return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
@@ -169,26 +159,6 @@ __device__ __forceinline__ void tc_ld32(uint32_t taddr, uint32_t (&v)[32]) {
       : "r"(taddr)
       : "memory");
 }
-__device__ __forceinline__ void tc_ld16(uint32_t taddr, uint32_t (&v)[16]) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, "
-      "%15}, [%16];\n"
-      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
-        "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
-      : "r"(taddr)
-      : "memory");
-}
 __device__ __forceinline__ void tc_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory"); }
-// 16 consecutive 32-bit columns of this warp's 32 TMEM lanes from registers;
-// complete after tc_wait_st().
-__device__ __forceinline__ void tc_st16(uint32_t taddr, const uint32_t (&v)[16]) {
-  asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, "
-      "%15, %16};\n" ::"r"(taddr),
-      "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]), "r"(v[9]),
-      "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15])
-      : "memory");
-}
-__device__ __forceinline__ void tc_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;\n" ::: "memory"); }
 
 }  // namespace hm
