@@ -64,12 +64,11 @@ struct KmmArgs {
 // ---------------------------------------------------------------------------
 // k_kmm: out(rows x s) = K(rows, cols) W(cols x s) for one 64-row tile.
 // Thread t: row r = t % 64, q = t / 64 splits the s output columns into
-// `nslab` slabs of 32 and the chunk columns into 4/nslab groups.  Kernel
-// entries are FP32; products and sums are in the workspace type W (an FP32 x
-// FP32 product is exact in FP64, so W = double gives FP64-accurate samples).
+// `nslab` slabs of 32 and the chunk columns into 4/nslab groups.  FP32 working
+// precision in more than three dimensions (the others: k_kmm_fast, k_kmm64).
 // ---------------------------------------------------------------------------
-template <typename W>
-__global__ void __launch_bounds__(kKmmThreads) k_kmm(KmmArgs<W> a) {
+__global__ void __launch_bounds__(kKmmThreads) k_kmm(KmmArgs<float> a) {
+  using W = float;
   extern __shared__ __align__(16) unsigned char kmm_raw[];
   W* Wsm = reinterpret_cast<W*>(kmm_raw);          // [kTC][kColGroup]
   float* Asm = reinterpret_cast<float*>(Wsm + kTC * kColGroup);  // [kTC][kTR]
@@ -178,6 +177,147 @@ __global__ void __launch_bounds__(kKmmThreads) k_kmm(KmmArgs<W> a) {
       atomicAdd(&a.st[it.x].normA2, tot);
     }
   }
+}
+
+// ---------------------------------------------------------------------------
+// k_kmm64: the same product in FP64 (tolerances below what FP32 sums resolve)
+// on the FP64 tensor instruction (mma.sync m8n8k4).  CTA = 4 warps = 64
+// operator rows, warp = 16 rows: a lane evaluates two FP32 kernel entries per
+// four columns, which are its A fragments; the right-hand operand (Gaussian
+// numbers, or the basis) is staged as FP64, 64 rows at a time.  A warp whose
+// rows lie past the block only helps to stage.
+// Bound by the FP64 pipe (8 NT multiply-adds per entry) and the entries' 25
+// instructions alike.  Measured against one row per thread with FP64 FMAs on 32
+// columns whatever the sample's width: a 120000-point 2-D build's sketches and
+// projections 482 -> 155 ms.
+// D: dimension compiled for (0: any); NT: column tiles of 8.
+// ---------------------------------------------------------------------------
+template <int D, int NT>
+__global__ void __launch_bounds__(128) k_kmm64(KmmArgs<double> a) {
+  constexpr int LDC = 8 * NT + 4;  // a half-warp's 4 rows x 4 columns fall into 16 banks
+  constexpr int DD = D ? D : kMaxDim;
+  __shared__ double Wsm[kTC * LDC];
+  __shared__ float colc[DD][kTC];
+  __shared__ double red[4];
+  const int2 it = a.items[blockIdx.x];
+  const Prob P = a.probs[it.x];
+  const ProbState S = a.st[it.x];
+  if (a.mode == 0 && !S.active) return;
+  const int col0 = a.mode ? a.col0 : 0;
+  const int s = min(8 * NT, (a.mode == 0 ? a.bs : S.k) - col0);
+  if (s <= 0) return;
+  const int d = D ? D : a.d;
+  const int mr = a.mode ? P.n : P.m;        // rows of the operator
+  const int nc = a.mode ? P.m : P.n;        // columns of the operator
+  const int rbase = a.mode ? P.c0 : P.r0;
+  const int cbase = a.mode ? P.r0 : P.c0;
+  const int ldo = ara_ld(mr), ldq = ara_ld(P.m);
+  double* out = reinterpret_cast<double*>(a.mode ? P.b : P.y) + (size_t)col0 * ldo;
+  const double* Q = reinterpret_cast<const double*>(P.q) + (size_t)col0 * ldq;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+  const int row0 = it.y * kTR + warp * 16;
+  const bool busy = row0 < mr;  // the whole warp
+  const int ra = row0 + g, rb = ra + 8;
+  const bool ra_ok = ra < mr, rb_ok = rb < mr;
+  float rca[DD], rcb[DD];
+#pragma unroll
+  for (int k = 0; k < DD; ++k) {
+    rca[k] = k < d && ra_ok ? a.pts[(size_t)k * a.npts + rbase + ra] : 0.f;
+    rcb[k] = k < d && rb_ok ? a.pts[(size_t)k * a.npts + rbase + rb] : 0.f;
+  }
+  const int ntiles = (s + 7) >> 3;
+  double acc[2][NT][2];
+#pragma unroll
+  for (int i = 0; i < 2; ++i)
+#pragma unroll
+    for (int n = 0; n < NT; ++n) acc[i][n][0] = acc[i][n][1] = 0.0;
+  double nrm = 0.0;
+  const bool want_norm = a.mode == 0 && a.round == 0;
+  for (int c0 = 0; c0 < nc; c0 += kTC) {
+    __syncthreads();
+    for (int e = tid; e < d * kTC; e += 128) {
+      const int k = e / kTC, j = c0 + e % kTC;
+      colc[k][e % kTC] = j < nc ? a.pts[(size_t)k * a.npts + cbase + j] : 0.f;
+    }
+    for (int e = tid; e < kTC * 8 * ntiles; e += 128) {
+      const int jj = e % kTC, cc = e / kTC, j = c0 + jj;
+      double w = 0.0;
+      if (j < nc && cc < s)
+        w = a.mode == 0 ? (double)gauss_at(a.seed, (uint32_t)P.gid, (uint32_t)j, (uint32_t)(a.round * kMaxBs + cc))
+                        : Q[(size_t)cc * ldq + j];
+      Wsm[jj * LDC + cc] = w;
+    }
+    __syncthreads();
+    if (!busy) continue;
+    const int nq = (min(kTC, nc - c0) + 3) >> 2;
+    for (int q = 0; q < nq; ++q) {
+      const int jj = 4 * q + t;
+      float r2a = 0.f, r2b = 0.f;
+#pragma unroll
+      for (int k = 0; k < DD; ++k) {
+        if (D || k < d) {
+          const float c = colc[k][jj], da = rca[k] - c, db = rcb[k] - c;
+          r2a = fmaf(da, da, r2a);
+          r2b = fmaf(db, db, r2b);
+        }
+      }
+      const bool in = c0 + jj < nc;
+      const double va = in && ra_ok ? (double)kernel_r2(a.kp, r2a) : 0.0;
+      const double vb = in && rb_ok ? (double)kernel_r2(a.kp, r2b) : 0.0;
+      if (want_norm) nrm = fma(va, va, fma(vb, vb, nrm));
+      const double* w = Wsm + jj * LDC + g;
+#pragma unroll
+      for (int n = 0; n < NT; ++n) {
+        if (n < ntiles) {
+          const double b = w[8 * n];
+          mma_f64(acc[0][n], va, b);
+          mma_f64(acc[1][n], vb, b);
+        }
+      }
+    }
+  }
+  if (busy) {  // rows mr .. ldo - 1 (padding) get their zeros
+#pragma unroll
+    for (int n = 0; n < NT; ++n) {
+      if (n >= ntiles) continue;
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        const int c = 8 * n + 2 * t + u;
+        if (c < s) {
+          if (ra < ldo) out[(size_t)c * ldo + ra] = acc[0][n][u];
+          if (rb < ldo) out[(size_t)c * ldo + rb] = acc[1][n][u];
+        }
+      }
+    }
+  }
+  if (want_norm) {
+    for (int o = 16; o > 0; o >>= 1) nrm += __shfl_xor_sync(0xffffffffu, nrm, o);
+    if (lane == 0) red[warp] = nrm;
+    __syncthreads();
+    if (tid == 0) atomicAdd(&a.st[it.x].normA2, red[0] + red[1] + red[2] + red[3]);
+  }
+}
+
+template <int NT>
+void launch_kmm64(unsigned grid, cudaStream_t s, const KmmArgs<double>& a) {
+  if (a.d == 1)
+    k_kmm64<1, NT><<<grid, 128, 0, s>>>(a);
+  else if (a.d == 2)
+    k_kmm64<2, NT><<<grid, 128, 0, s>>>(a);
+  else if (a.d == 3)
+    k_kmm64<3, NT><<<grid, 128, 0, s>>>(a);
+  else
+    k_kmm64<0, NT><<<grid, 128, 0, s>>>(a);
+}
+// cols: right-hand columns the launch must cover, at most kGroup64
+constexpr int kGroup64 = 64;
+void launch_kmm64(int cols, unsigned grid, cudaStream_t s, const KmmArgs<double>& a) {
+  if (cols <= 16)
+    launch_kmm64<2>(grid, s, a);
+  else if (cols <= 32)
+    launch_kmm64<4>(grid, s, a);
+  else
+    launch_kmm64<8>(grid, s, a);
 }
 
 // ---------------------------------------------------------------------------
@@ -522,8 +662,8 @@ __global__ void k_dense_gen(const DenseItem* items, const float* pts, int npts, 
   }
 }
 
-template <typename W>
 size_t kmm_smem() {
+  using W = float;
   return sizeof(W) * (kTC * kColGroup) + sizeof(float) * (kTC * kTR + kMaxDim * kTC) +
          sizeof(double) * (kKmmThreads / 32);
 }
@@ -672,7 +812,8 @@ hm_status hmatrix_build(hm_kdtree t, hm_structure s, const double* d_points, con
   const bool fp64 = opt.tol < 5e-6;
   auto batch_loop = [&](auto tag) -> hm_status {
     using W = decltype(tag);
-    HM_CUDA(cudaFuncSetAttribute(k_kmm<W>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kmm_smem<W>()));
+    if (std::is_same<W, float>::value)
+      HM_CUDA(cudaFuncSetAttribute(k_kmm, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kmm_smem()));
     // The specialised sketch kernels draw a double-width first sample (the
     // generation of the kernel block, not its product with the sample, is
     // the cost of a pass, so blocks of rank bs..2 bs finish a pass earlier).
@@ -860,7 +1001,10 @@ hm_status hmatrix_build(hm_kdtree t, hm_structure s, const double* d_points, con
           ka.col0 = 0;
           ka.round = round;
           ka.items = drows.p;
-          k_kmm<W><<<(unsigned)items_rows.size(), kKmmThreads, kmm_smem<W>(), stream>>>(ka);
+          if constexpr (kTensor)
+            k_kmm<<<(unsigned)items_rows.size(), kKmmThreads, kmm_smem(), stream>>>(ka);
+          else
+            launch_kmm64(rbs, (unsigned)items_rows.size(), stream, ka);
         }
         HM_LAUNCH_CHECK();
         tr.mark("  round sketch", stream, round, 1);
@@ -938,9 +1082,13 @@ hm_status hmatrix_build(hm_kdtree t, hm_structure s, const double* d_points, con
         ka.items = dcols.p;
         int kmx = 0;
         for (int i = 0; i < nb; ++i) kmx = std::max(kmx, hst[i].k);
-        for (int c0 = 0; c0 < kmx; c0 += kColGroup) {
+        constexpr int kGroup = kTensor ? kColGroup : kGroup64;
+        for (int c0 = 0; c0 < kmx; c0 += kGroup) {
           ka.col0 = c0;
-          k_kmm<W><<<(unsigned)items_cols.size(), kKmmThreads, kmm_smem<W>(), stream>>>(ka);
+          if constexpr (kTensor)
+            k_kmm<<<(unsigned)items_cols.size(), kKmmThreads, kmm_smem(), stream>>>(ka);
+          else
+            launch_kmm64(std::min(kGroup, kmx - c0), (unsigned)items_cols.size(), stream, ka);
           HM_LAUNCH_CHECK();
         }
         ka.col0 = 0;
