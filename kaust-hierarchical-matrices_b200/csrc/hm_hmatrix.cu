@@ -335,8 +335,21 @@ void launch_kmm64(int cols, unsigned grid, cudaStream_t s, const KmmArgs<double>
 // coordinates stay in registers, and the right-hand operand (the Gaussian
 // table in sampling mode, the basis Q in projection mode) is read as
 // prepacked BF16 pairs straight from L1/L2 instead of being restaged per chunk.
+// Instruction issue bounds it, then the special-function unit (two of its
+// operations per entry; 75 % busy with 16 sampled columns): distances, kernel
+// values, the norm and the splits are done two entries per instruction
+// (FP32 pairs), only a block's ragged last step masks columns, and the MMAs of
+// a k-step stand in one straight run (the tables are padded to the tiles the
+// variant takes, so there is no test per tile).  First sampling round of a
+// 2^17-point 3-D Matern build, one batch: 32 columns 8.0 -> 5.7 ms, 16 columns
+// 6.4 -> 4.4 ms.
 // ---------------------------------------------------------------------------
 constexpr int kCC = 128;  // columns per coordinate chunk
+// column tiles of 8 of the right-hand tables: the Gaussian table has as many
+// as the sampling kernel's variant multiplies (its padding tiles are zeros),
+// the basis table an even number
+__host__ __device__ constexpr int sample_tiles(int bs) { return bs <= 16 ? 2 : bs <= 32 ? 4 : 8; }
+__host__ __device__ constexpr int q_tiles(int k) { return (k + 15) >> 4 << 1; }
 
 struct KmmFastArgs {
   const Prob* probs;
@@ -351,9 +364,8 @@ struct KmmFastArgs {
   // right-hand operand tables in fragment order: word (k-step, column tile,
   // lane (g,t)) holds the m16n8k16 B fragment {b0, b1} with
   // b0 = {W[16 ks + 2t][8 nt + g], W[16 ks + 2t + 1][..]}, b1 = rows + 8
-  const uint2* om;          // sampling: the Gaussian table, om_nt column tiles
-  int om_nt;
-  const uint4* qt;          // projection: {hi b0, hi b1, lo b0, lo b1} of Q, per problem
+  const uint2* om;          // sampling: the Gaussian table, NT column tiles (see sample_tiles)
+  const uint4* qt;          // projection: {hi b0, hi b1, lo b0, lo b1} of Q, per problem, tiles in pairs
   const long long* qpoff;   // per problem (batch index), 16-byte words
   int col0;                 // projection: first basis column of this launch
 };
@@ -371,30 +383,37 @@ __device__ __forceinline__ float sqrt_approx(float x) {
 
 constexpr float kLn2f = 0.6931471805599453f;
 
-// r2: squared distance of the scaled coordinates.
+// r2: squared distances of the scaled coordinates, two entries.
 //   KIND 0 (exp):    scale = log2(e)/l,         a = r log2(e)/l,  K = 2^-a
 //   KIND 1 (Matern): scale = sqrt(3) log2(e)/l,  K = (1 + a ln2) 2^-a
 //   KIND 2 (Gauss):  scale = sqrt(log2(e)/2)/l,  K = 2^-r2
 // derivatives dK/dl: exp a ln2 K / l, Matern (a ln2)^2 2^-a / l,
 // Gauss K q / l with q = r^2/l^2 = 2 ln2 r2.
 template <int KIND, bool DERIV>
-__device__ __forceinline__ float kval(float r2, float dscale) {
+__device__ __forceinline__ f32x2 kval2(f32x2 r2, f32x2 dscale) {
+  float x, y;
+  unpack2(r2, x, y);
   if (KIND == 2) {
-    const float v = ex2_approx(-r2);
-    return DERIV ? v * r2 * dscale : v;
+    const f32x2 v = pack2(ex2_approx(-x), ex2_approx(-y));
+    return DERIV ? mul2(mul2(v, r2), dscale) : v;
   }
-  const float a = sqrt_approx(r2);
-  const float e = ex2_approx(-a);
+  x = sqrt_approx(x);
+  y = sqrt_approx(y);
+  const f32x2 a = pack2(x, y), e = pack2(ex2_approx(-x), ex2_approx(-y));
   if (KIND == 1) {
-    const float al = a * kLn2f;
-    return DERIV ? al * al * e * dscale : fmaf(a, kLn2f, 1.0f) * e;
+    const f32x2 ln2 = pack2(kLn2f, kLn2f);
+    const f32x2 al = mul2(a, ln2);
+    return DERIV ? mul2(mul2(mul2(al, al), e), dscale) : mul2(fma2(a, ln2, pack2(1.f, 1.f)), e);
   }
-  return DERIV ? a * e * dscale : e;
+  return DERIV ? mul2(mul2(a, e), dscale) : e;
 }
 
+// CTAs an SM shall hold (0: left to the compiler, which is faster at two tiles)
+constexpr int kmm_ctas(int nt) { return nt == 2 ? 0 : nt == 4 ? 8 : nt == 8 ? 5 : 3; }
+
 template <int D, int KIND, int MODE, int NT>
-__global__ void __launch_bounds__(128) k_kmm_fast(KmmFastArgs a) {
-  __shared__ float colc[D][kCC];
+__global__ void __launch_bounds__(128, kmm_ctas(NT)) k_kmm_fast(KmmFastArgs a) {
+  __shared__ __align__(8) float colc[D][kCC];  // negated: a difference is one packed add
   __shared__ double red[4];
   const int2 it = a.items[blockIdx.x];
   const Prob P = a.probs[it.x];
@@ -413,121 +432,142 @@ __global__ void __launch_bounds__(128) k_kmm_fast(KmmFastArgs a) {
   const int ra = it.y * kTR + warp * 16 + g, rb = ra + 8;
   const bool ra_ok = ra < mr, rb_ok = rb < mr;
   const bool deriv = a.deriv != 0;
-  float rca[D], rcb[D];
+  f32x2 rca[D], rcb[D];
 #pragma unroll
   for (int k = 0; k < D; ++k) {
-    rca[k] = ra_ok ? a.pts[(size_t)k * a.npts + rbase + ra] * a.scale : 0.f;
-    rcb[k] = rb_ok ? a.pts[(size_t)k * a.npts + rbase + rb] * a.scale : 0.f;
+    const float xa = ra_ok ? a.pts[(size_t)k * a.npts + rbase + ra] * a.scale : 0.f;
+    const float xb = rb_ok ? a.pts[(size_t)k * a.npts + rbase + rb] * a.scale : 0.f;
+    rca[k] = pack2(xa, xa);
+    rcb[k] = pack2(xb, xb);
   }
-  const int ntiles = min(NT, (s + 7) >> 3);
-  const int tnt = MODE ? (S.k + 7) >> 3 : a.om_nt;  // column tiles of the table
+  const f32x2 dscale = pack2(a.dscale, a.dscale);
+  static_assert(NT % 2 == 0, "column tiles are taken in pairs");
+  const int tnt = MODE ? q_tiles(S.k) : NT;  // column tiles of the table
+  const int ntiles = MODE ? min(NT, tnt - (col0 >> 3)) : NT;
   const uint4* qt = MODE ? a.qt + a.qpoff[it.x] + (col0 >> 3) * 32 + lane : nullptr;
   const uint2* om = MODE ? nullptr : a.om + lane;
-  float acc[NT][4];
+  f32x2 acc[NT][2];  // rows ra, rb; columns 8 nt + 2t, + 1
 #pragma unroll
-  for (int nt = 0; nt < NT; ++nt) acc[nt][0] = acc[nt][1] = acc[nt][2] = acc[nt][3] = 0.f;
-  float nrm = 0.f;
+  for (int nt = 0; nt < NT; ++nt) acc[nt][0] = acc[nt][1] = pack2(0.f, 0.f);
+  f32x2 nrma = pack2(0.f, 0.f), nrmb = nrma;
   const bool want_norm = MODE == 0 && a.round == 0;
-  // B fragments of k-step kg (16 columns of the block): one word per lane and column tile
-  uint32_t bh[NT][2], bl[NT][2];
-  auto load_b = [&](int kg) {
-#pragma unroll
-    for (int nt = 0; nt < NT; ++nt) {
-      if (nt < ntiles) {
-        if (MODE == 1) {
-          const uint4 v = __ldg(qt + ((size_t)kg * tnt + nt) * 32);
-          bh[nt][0] = v.x;
-          bh[nt][1] = v.y;
-          bl[nt][0] = v.z;
-          bl[nt][1] = v.w;
-        } else {
-          const uint2 v = __ldg(om + ((size_t)kg * tnt + nt) * 32);
-          bh[nt][0] = v.x;
-          bh[nt][1] = v.y;
-        }
-      }
-    }
-  };
   const int nks = (nc + 15) >> 4;
-  if (MODE == 0) load_b(0);
   for (int kg = 0; kg < nks; ++kg) {
     const int c0 = (kg * 16) / kCC * kCC;
     if (kg * 16 == c0) {  // first k-step of a coordinate chunk
       __syncthreads();
       for (int e = threadIdx.x; e < D * kCC; e += blockDim.x) {
         const int k = e / kCC, jj = e % kCC;
-        colc[k][jj] = c0 + jj < nc ? a.pts[(size_t)k * a.npts + cbase + c0 + jj] * a.scale : 0.f;
+        colc[k][jj] = c0 + jj < nc ? -(a.pts[(size_t)k * a.npts + cbase + c0 + jj] * a.scale) : 0.f;
       }
       __syncthreads();
     }
-    uint32_t ch[NT][2];
-    if (MODE == 1) {
-      load_b(kg);  // issued before the entries are generated, used after (no second register set)
-    } else {
+    // B fragments of the k-step (16 columns of the block), one word per lane
+    // and column tile: issued before the entries are generated, used after
+    uint32_t bh[NT][2], bl[NT][2];
 #pragma unroll
-      for (int nt = 0; nt < NT; ++nt) {
-        ch[nt][0] = bh[nt][0];
-        ch[nt][1] = bh[nt][1];
+    for (int n2 = 0; n2 < NT; n2 += 2)
+      if (MODE == 0 || n2 < ntiles) {
+#pragma unroll
+        for (int nt = n2; nt < n2 + 2; ++nt) {
+          if (MODE == 1) {
+            const uint4 v = __ldg(qt + nt * 32);
+            bh[nt][0] = v.x;
+            bh[nt][1] = v.y;
+            bl[nt][0] = v.z;
+            bl[nt][1] = v.w;
+          } else {
+            const uint2 v = __ldg(om + nt * 32);
+            bh[nt][0] = v.x;
+            bh[nt][1] = v.y;
+          }
+        }
       }
-      if (kg + 1 < nks) load_b(kg + 1);  // in flight while this k-step's entries are generated
-    }
+    if (MODE == 1)
+      qt += tnt * 32;
+    else
+      om += NT * 32;
     const int cb = kg * 16 - c0 + 2 * t;  // chunk columns cb, cb+1, cb+8, cb+9
-    float e[8];
+    f32x2 e[4];                           // row ra: pairs cb, cb+8; row rb: pairs cb, cb+8
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const int c = cb + (q & 1) + ((q >> 1) << 3);
-      const bool cok = c0 + c < nc;
-      float r2a = 0.f, r2b = 0.f;
+    for (int h = 0; h < 2; ++h) {
+      f32x2 ra2, rb2;
 #pragma unroll
       for (int k = 0; k < D; ++k) {
-        const float cc = colc[k][c];
-        const float da = rca[k] - cc, db = rcb[k] - cc;
-        r2a = fmaf(da, da, r2a);
-        r2b = fmaf(db, db, r2b);
+        const f32x2 cc = *reinterpret_cast<const f32x2*>(&colc[k][cb + 8 * h]);
+        const f32x2 da = add2(rca[k], cc), db = add2(rcb[k], cc);
+        ra2 = k ? fma2(da, da, ra2) : mul2(da, da);
+        rb2 = k ? fma2(db, db, rb2) : mul2(db, db);
       }
-      const float va = deriv ? kval<KIND, true>(r2a, a.dscale) : kval<KIND, false>(r2a, a.dscale);
-      const float vb = deriv ? kval<KIND, true>(r2b, a.dscale) : kval<KIND, false>(r2b, a.dscale);
-      e[q] = (ra_ok && cok) ? va : 0.f;
-      e[4 + q] = (rb_ok && cok) ? vb : 0.f;
+      e[h] = ra2;
+      e[2 + h] = rb2;
+    }
+    if (deriv) {
+#pragma unroll
+      for (int q = 0; q < 4; ++q) e[q] = kval2<KIND, true>(e[q], dscale);
+    } else {
+#pragma unroll
+      for (int q = 0; q < 4; ++q) e[q] = kval2<KIND, false>(e[q], dscale);
+    }
+    if (kg * 16 + 16 > nc) {  // the last k-step of a ragged block: columns past it are zeros
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const int c = kg * 16 + 2 * t + 8 * (q & 1);
+        float x, y;
+        unpack2(e[q], x, y);
+        e[q] = pack2(c < nc ? x : 0.f, c + 1 < nc ? y : 0.f);
+      }
     }
     if (want_norm) {
-#pragma unroll
-      for (int q = 0; q < 8; ++q) nrm = fmaf(e[q], e[q], nrm);
+      nrma = fma2(e[1], e[1], fma2(e[0], e[0], nrma));
+      nrmb = fma2(e[3], e[3], fma2(e[2], e[2], nrmb));
     }
     uint32_t ah[4], al[4];
-    split_bf16x2(e[0], e[1], ah[0], al[0]);  // row g, cols cb, cb+1
-    split_bf16x2(e[4], e[5], ah[1], al[1]);  // row g+8
-    split_bf16x2(e[2], e[3], ah[2], al[2]);  // row g, cols cb+8, cb+9
-    split_bf16x2(e[6], e[7], ah[3], al[3]);  // row g+8
+    split2(e[0], ah[0], al[0]);  // row g, cols cb, cb+1
+    split2(e[2], ah[1], al[1]);  // row g+8
+    split2(e[1], ah[2], al[2]);  // row g, cols cb+8, cb+9
+    split2(e[3], ah[3], al[3]);  // row g+8
 #pragma unroll
-    for (int nt = 0; nt < NT; ++nt) {
-      if (nt < ntiles) {
-        float d[4] = {0.f, 0.f, 0.f, 0.f};
-        const uint32_t b0 = MODE == 1 ? bh[nt][0] : ch[nt][0], b1 = MODE == 1 ? bh[nt][1] : ch[nt][1];
-        if (MODE == 1) mma_bf16(d, ah[0], ah[1], ah[2], ah[3], bl[nt][0], bl[nt][1]);
-        mma_bf16(d, al[0], al[1], al[2], al[3], b0, b1);
-        mma_bf16(d, ah[0], ah[1], ah[2], ah[3], b0, b1);
-        add4(acc[nt], d);
+    for (int n2 = 0; n2 < NT; n2 += 2)
+      if (MODE == 0 || n2 < ntiles) {
+        float d[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+          if (MODE == 1) mma_bf16(d[j], ah[0], ah[1], ah[2], ah[3], bl[n2 + j][0], bl[n2 + j][1]);
+#pragma unroll
+        for (int j = 0; j < 2; ++j) mma_bf16(d[j], al[0], al[1], al[2], al[3], bh[n2 + j][0], bh[n2 + j][1]);
+#pragma unroll
+        for (int j = 0; j < 2; ++j) mma_bf16(d[j], ah[0], ah[1], ah[2], ah[3], bh[n2 + j][0], bh[n2 + j][1]);
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          acc[n2 + j][0] = add2(acc[n2 + j][0], pack2(d[j][0], d[j][1]));
+          acc[n2 + j][1] = add2(acc[n2 + j][1], pack2(d[j][2], d[j][3]));
+        }
       }
-    }
   }
   // rows mr .. ld - 1 (padding) get their zeros
 #pragma unroll
   for (int nt = 0; nt < NT; ++nt) {
     if (nt < ntiles) {
       const int c = nt * 8 + 2 * t;
+      float x, y;
+      unpack2(acc[nt][0], x, y);
       if (ra < ld) {
-        if (c < s) out[(size_t)c * ld + ra] = acc[nt][0];
-        if (c + 1 < s) out[(size_t)(c + 1) * ld + ra] = acc[nt][1];
+        if (c < s) out[(size_t)c * ld + ra] = ra_ok ? x : 0.f;
+        if (c + 1 < s) out[(size_t)(c + 1) * ld + ra] = ra_ok ? y : 0.f;
       }
+      unpack2(acc[nt][1], x, y);
       if (rb < ld) {
-        if (c < s) out[(size_t)c * ld + rb] = acc[nt][2];
-        if (c + 1 < s) out[(size_t)(c + 1) * ld + rb] = acc[nt][3];
+        if (c < s) out[(size_t)c * ld + rb] = rb_ok ? x : 0.f;
+        if (c + 1 < s) out[(size_t)(c + 1) * ld + rb] = rb_ok ? y : 0.f;
       }
     }
   }
   if (want_norm) {
-    double dn = nrm;
+    float na, na1, nb, nb1;
+    unpack2(nrma, na, na1);
+    unpack2(nrmb, nb, nb1);
+    double dn = (ra_ok ? (double)na + na1 : 0.0) + (rb_ok ? (double)nb + nb1 : 0.0);
     for (int o = 16; o > 0; o >>= 1) dn += __shfl_xor_sync(0xffffffffu, dn, o);
     if (lane == 0) red[warp] = dn;
     __syncthreads();
@@ -558,12 +598,12 @@ __global__ void k_omega_pack(uint2* om, int ksteps, int bs, int nt_tot, uint32_t
 
 // Q (m x k, column-major, ld m) of each problem in fragment order, hi and lo
 // (see KmmFastArgs): k-steps over the rows padded to whole coordinate chunks,
-// column tiles over k padded to 8.
+// column tiles over k padded to 16.
 __global__ void k_pack_q(const Prob* probs, const ProbState* st, const long long* qpoff, uint4* qt) {
   const Prob P = probs[blockIdx.x];
   const int k = st[blockIdx.x].k;
   if (k <= 0) return;
-  const int ntq = (k + 7) >> 3;
+  const int ntq = q_tiles(k);
   const int ksteps = (P.m + kCC - 1) / kCC * (kCC / 16);
   const float* Q = reinterpret_cast<const float*>(P.q);
   uint4* q = qt + qpoff[blockIdx.x];
@@ -924,13 +964,13 @@ hm_status hmatrix_build(hm_kdtree t, hm_structure s, const double* d_points, con
       KmmFastArgs kf{};
       DevBuf<uint2> om2;
       const int bs0 = gen_bs0;
-      const int bs8 = (bs0 + 7) & ~7;
+      const int om_nt = sample_tiles(std::max(bs0, bs));
       int om_rows2 = 0;
       if (fast) {
         int max_n = 1;
         for (const Prob& P : bp) max_n = std::max(max_n, P.n);
         om_rows2 = (max_n + kCC - 1) / kCC * (kCC / 2);  // column pairs; k-steps = om_rows2 / 8
-        if ((st = om2.alloc_async((size_t)(om_rows2 / 8) * (bs8 / 8) * 32, stream))) return st;
+        if ((st = om2.alloc_async((size_t)(om_rows2 / 8) * om_nt * 32, stream))) return st;
         const double il = 1.0 / opt.ell, log2e = 1.4426950408889634, ln2 = 0.6931471805599453;
         double sc = log2e * il, dsc = ln2 * il;
         if (opt.kernel == HM_KERNEL_MATERN32) {
@@ -949,7 +989,6 @@ hm_status hmatrix_build(hm_kdtree t, hm_structure s, const double* d_points, con
         kf.deriv = opt.derivative != 0;
         kf.bs = bs;
         kf.om = om2.p;
-        kf.om_nt = bs8 / 8;
       }
       tr.mark("batch setup", stream, nb, 0);
       const int max_rounds = kMaxCols / bs + 2;
@@ -990,12 +1029,12 @@ hm_status hmatrix_build(hm_kdtree t, hm_structure s, const double* d_points, con
           }
         }
         if (fast) {
-          k_omega_pack<<<592, 256, 0, stream>>>(om2.p, om_rows2 / 8, rbs, bs8 / 8, ka.seed, round);
+          k_omega_pack<<<592, 256, 0, stream>>>(om2.p, om_rows2 / 8, rbs, sample_tiles(rbs), ka.seed, round);
           HM_LAUNCH_CHECK();
           kf.round = round;
           kf.bs = rbs;
           kf.items = drows.p;
-          launch_kmm_fast(t->d, opt.kernel, 0, (rbs + 7) / 8, (unsigned)items_rows.size(), stream, kf);
+          launch_kmm_fast(t->d, opt.kernel, 0, sample_tiles(rbs), (unsigned)items_rows.size(), stream, kf);
         } else {
           ka.mode = 0;
           ka.col0 = 0;
@@ -1038,7 +1077,7 @@ hm_status hmatrix_build(hm_kdtree t, hm_structure s, const double* d_points, con
         for (int i = 0; i < nb; ++i) {
           qpoff[i] = (long long)qw;
           if (hst[i].k > 0)
-            qw += (size_t)(bp[i].m + kCC - 1) / kCC * (kCC / 16) * (size_t)((hst[i].k + 7) >> 3) * 32;
+            qw += (size_t)(bp[i].m + kCC - 1) / kCC * (kCC / 16) * (size_t)q_tiles(hst[i].k) * 32;
         }
         if ((st = qt.alloc_async(std::max<size_t>(qw, 1), stream)) || (st = dqpoff.alloc_async(nb, stream)))
           return st;

@@ -80,6 +80,42 @@ __device__ __forceinline__ void split_bf16x2(float x0, float x1, uint32_t& hi, u
   lo = pack_bf16(x0 - bf16_lo_as_float(hi), x1 - bf16_hi_as_float(hi));
 }
 
+// Two FP32 numbers in one register pair: one instruction does both, each
+// rounded as the scalar instruction rounds it.
+using f32x2 = unsigned long long;
+__device__ __forceinline__ f32x2 pack2(float x, float y) {
+  f32x2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
+  return r;
+}
+__device__ __forceinline__ void unpack2(f32x2 v, float& x, float& y) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(v));
+}
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+  f32x2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+// split_bf16x2 of a pair
+__device__ __forceinline__ void split2(f32x2 v, uint32_t& hi, uint32_t& lo) {
+  float x, y;
+  unpack2(v, x, y);
+  hi = pack_bf16(x, y);
+  const f32x2 rest = fma2(pack2(bf16_lo_as_float(hi), bf16_hi_as_float(hi)), pack2(-1.f, -1.f), v);
+  unpack2(rest, x, y);
+  lo = pack_bf16(x, y);
+}
+
 __device__ __forceinline__ void mma_bf16(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
                                          uint32_t b0, uint32_t b1) {
   asm volatile(
