@@ -278,7 +278,7 @@ __global__ void __launch_bounds__(32 * SP, SP == 1 ? 24 : 16 / SP)
       my_nct = P.nct;
     }
   }
-  const int d0 = leaf_dptr[x], d1 = leaf_dptr[x + 1];
+  const int d0 = SP > 1 ? leaf_dptr[x] : 0, d1 = SP > 1 ? leaf_dptr[x + 1] : 0;
   // this warp's run [lo, hi) of the row tile's column tiles
   int lo = 0, hi = 0, my_end = 0;
   if (SP > 1) {
@@ -315,43 +315,47 @@ __global__ void __launch_bounds__(32 * SP, SP == 1 ? 24 : 16 / SP)
       fp_p2_step<NB>(acc, ah, al, bh, bl);
     }
   }
+  auto dense_step = [&](const uint4* dp, int xt0, int ct) {
+    const uint4 a0 = __ldcs(dp + (2 * ct) * 32), a1 = __ldcs(dp + (2 * ct + 1) * 32);
+    const size_t xt = ((size_t)(xt0 + (ct >> 2)) * 8 + (ct & 3)) * 32 + lane;
+    const uint4 xh = __ldg(Xf + xt), xl = __ldg(Xf + xt + 128);
+    uint32_t ah[2][4], al[2][4];
+    split4(a0, ah[0], al[0]);
+    split4(a1, ah[1], al[1]);
+    const uint32_t bh[2][2] = {{xh.x, xh.z}, {xh.y, xh.w}};
+    const uint32_t bl[2][2] = {{xl.x, xl.z}, {xl.y, xl.w}};
+    fp_p2_step<NB>(acc, ah, al, bh, bl);
+  };
+  if (SP == 1) {
+    for (int q = leaf_dptr[x]; q < leaf_dptr[x + 1]; ++q) {
+      const MxDense D = dense[leaf_dblk[q]];
+      const uint4* dp = store + (D.hi + (long long)(G - D.row_tile0) * D.nct * 2) * 32 + lane;
+      for (int ct = 0; ct < D.nct; ++ct) dense_step(dp, D.col_tile0, ct);
+    }
+  }
   int at = SP > 1 ? __shfl_sync(0xffffffffu, my_end, 31) : 0;
-  for (int q0 = d0; q0 < d1; q0 += 32) {
+  for (int q0 = d0; SP > 1 && q0 < d1; q0 += 32) {
     // up to 32 dense blocks' descriptors at once
     long long my_d = 0;
-    int my_x = 0, my_c = 0, my_e = 0;
+    int my_x = 0, my_c = 0;
     if (q0 + lane < d1) {
       const MxDense D = dense[leaf_dblk[q0 + lane]];
       my_d = D.hi + (long long)(G - D.row_tile0) * D.nct * 2;
       my_x = D.col_tile0;
       my_c = D.nct;
     }
-    if (SP > 1) my_e = at + warp_scan(my_c, lane);
+    const int my_e = at + warp_scan(my_c, lane);
     const int nq = min(32, d1 - q0);
     for (int q = 0; q < nq; ++q) {
-      int c1 = __shfl_sync(0xffffffffu, my_c, q), c0 = 0;
-      if (SP > 1) {
-        const int a = __shfl_sync(0xffffffffu, my_e, q) - c1;
-        c0 = max(0, lo - a);
-        c1 = min(c1, hi - a);
-        if (c0 >= c1) continue;
-      }
+      const int n = __shfl_sync(0xffffffffu, my_c, q), a = __shfl_sync(0xffffffffu, my_e, q) - n;
+      const int c0 = max(0, lo - a), c1 = min(n, hi - a);
+      if (c0 >= c1) continue;
       const uint4* dp = store + __shfl_sync(0xffffffffu, my_d, q) * 32 + lane;
       const int xt0 = __shfl_sync(0xffffffffu, my_x, q);
-#pragma unroll(SP == 1 ? 1 : 4)
-      for (int ct = c0; ct < c1; ++ct) {
-        const uint4 a0 = __ldcs(dp + (2 * ct) * 32), a1 = __ldcs(dp + (2 * ct + 1) * 32);
-        const size_t xt = ((size_t)(xt0 + (ct >> 2)) * 8 + (ct & 3)) * 32 + lane;
-        const uint4 xh = __ldg(Xf + xt), xl = __ldg(Xf + xt + 128);
-        uint32_t ah[2][4], al[2][4];
-        split4(a0, ah[0], al[0]);
-        split4(a1, ah[1], al[1]);
-        const uint32_t bh[2][2] = {{xh.x, xh.z}, {xh.y, xh.w}};
-        const uint32_t bl[2][2] = {{xl.x, xl.z}, {xl.y, xl.w}};
-        fp_p2_step<NB>(acc, ah, al, bh, bl);
-      }
+#pragma unroll 4
+      for (int ct = c0; ct < c1; ++ct) dense_step(dp, xt0, ct);
     }
-    if (SP > 1) at = __shfl_sync(0xffffffffu, my_e, 31);
+    at = __shfl_sync(0xffffffffu, my_e, 31);
   }
   const int base = leaf_off[x] + 32 * (G - leaf_tile0[x]), lim = leaf_off[x + 1];
   // sum i of lane L: rows 16 mt + g (+ 8), column 8 nb + 2 t (+ 1) of C fragment (mt, nb)

@@ -958,7 +958,7 @@ hm_status hmatrix_build(hm_kdtree t, hm_structure s, const double* d_points, con
       OrthPlan orth;
       if ((st = orth_plan<W>(bp, &orth, stream))) return st;
       // FP32 working precision and d <= 3: specialised tensor-core sketch
-      // kernels; otherwise the SIMT kernel in the working precision
+      // kernels; d > 3: the SIMT kernel; FP64: the FP64 tensor instruction
       constexpr bool kTensor = std::is_same<W, float>::value;
       const bool fast = kTensor && t->d <= 3;
       KmmFastArgs kf{};

@@ -38,8 +38,9 @@
 // slower), straight-line MMA code and 32 descriptors per load give, at 131072
 // mixture points, 0.31 ms for phase 1 (0.38 before) and 0.36 ms for phase 2
 // (1.15 with A rearranged word by word, 0.60 with one copy warp).
-// The tensor core's own sums do not round to nearest, so the chains are kept short: 24 MMAs for columns with low parts, a drift far
-// below the BF16 hi + lo rounding of T.  At a unit's end each drain thread
+// The tensor core's own sums do not round to nearest, so the chains are kept
+// short: 24 MMAs for columns with low parts, a drift far below the BF16 hi + lo
+// rounding of T.  At a unit's end each drain thread
 // stores its column (its TMEM lane): as T (into the mirror column's slots,
 // split hi + lo or hi only) when the panel is projected in one row chunk,
 // else as the chunk's partial S (per column its 128 FP32 sums, contiguous).
@@ -60,8 +61,8 @@
 // bytes, so the K-major image of V^T is the M-major image of U and the copy
 // engine moves it as it is; the rows of D come out in the tiles' order rho and
 // go to their place at the store.  (Rearranging the other tile order by 4-byte
-// cp.async with 27 copy warps took 1.15 ms at 131072 mixture points.)  Dense blocks keep a copy in the
-// same order for these passes, their columns in X's row order rho so that B
+// cp.async with 27 copy warps took 1.15 ms at 131072 mixture points.)  Dense
+// blocks keep a copy in the same order for these passes, their columns in X's row order rho so that B
 // is X's image of the column cluster's tile.  Panels' columns with low parts
 // take three products per 16 columns, 32 columns per step; the others one per
 // 16 columns, 64 per step; dense blocks three per 16 columns, 32 per step.
