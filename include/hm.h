@@ -396,8 +396,8 @@ HM_API hm_status hm_hmatrix_load(hm_kdtree t, hm_structure s, const char* path, 
 /* Waits for the stream, then returns HM_ERR_TIMEOUT if a bounded device-side
  * wait in one of this matrix's product kernels gave up since the last check
  * (the products concerned hold wrong values; the report is cleared), else
- * HM_OK.  Only the tcgen05 phase 1 of the mixed form's 128-column passes
- * waits on the device; the wait ends the kernel instead of hanging it. */
+ * HM_OK.  Only the tcgen05 kernels of the mixed form's 128-column passes
+ * wait on the device; a wait ends the kernel instead of hanging it. */
 HM_API hm_status hm_hmatrix_check(hm_hmatrix h, void* stream);
 
 /* Schedule autotuner (no counterpart in the reference).  Times the product's
