@@ -427,6 +427,8 @@ struct LocalArgs {
 };
 
 constexpr unsigned kNone = 0xffffu;  // no point at this position
+constexpr size_t kLocalBoxes = 2 * 32 * kMaxDim * sizeof(double);  // k_local's static shared memory
+constexpr size_t kLocalMaxSmem = 227 * 1024 - kLocalBoxes;         // what a CTA may have beyond it
 
 struct LocalSmem {
   double* coord;        // [d][seg_cap]
@@ -880,9 +882,10 @@ hm_status kdtree_build(const double* d_points, int n, int d, int bucket, cudaStr
   la.perm = t->perm.p;
   la.pts_tree = t->pts_tree.p;
   la.pts_tree_f = t->pts_tree_f.p;
-  size_t smem = local_smem_bytes(d, pcap, pcap, nlocal);
-  if ((s = cu(cudaFuncSetAttribute(k_local, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   (int)smem),
+  const size_t smem = local_smem_bytes(d, pcap, pcap, nlocal);
+  // the limit is the function's, not this launch's: always the most it can
+  // have, so that threads that build at once do not lower one another's
+  if ((s = cu(cudaFuncSetAttribute(k_local, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kLocalMaxSmem),
               "cudaFuncSetAttribute")))
     return cleanup(s);
   k_local<<<1 << j0, std::min(kLocalThreads, std::max(128, pcap / 2)), smem, stream>>>(la);

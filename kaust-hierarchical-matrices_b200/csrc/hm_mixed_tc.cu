@@ -66,6 +66,8 @@
 // is X's image of the column cluster's tile.  Panels' columns with low parts
 // take three products per 16 columns, 32 columns per step; the others one per
 // 16 columns, 64 per step; dense blocks three per 16 columns, 32 per step.
+#include <atomic>
+
 #include "hm_hmatrix.h"
 #include "hm_mixed.h"
 #include "hm_mma.cuh"
@@ -640,10 +642,10 @@ hm_status mixed_tc_pass(hm_hmatrix_s* h, int nr, const uint4* Xtc, float* S, uin
                         cudaStream_t s, KernelMarks* km) {
   MxPlan& M = h->mx;
   // the kernels' shared-memory limit, once per device of this process
-  static unsigned long long attr_done = 0;
+  static std::atomic<unsigned long long> attr_done{0};
   int dev = 0;
   HM_CUDA(cudaGetDevice(&dev));
-  if (dev >= 64 || !((attr_done >> dev) & 1ull)) {
+  if (dev >= 64 || !((attr_done.load() >> dev) & 1ull)) {
     HM_CUDA(cudaFuncSetAttribute(k_mx_p1_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kP1Smem));
     HM_CUDA(cudaFuncSetAttribute(k_mx_p2_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kP2Smem));
     if (dev < 64) attr_done |= 1ull << dev;

@@ -518,7 +518,10 @@ size_t orth_smem(int kcap) {
 template <typename W, int NT, int RW, bool CL>
 hm_status launch(const OrthPlan::Class& c, OrthArgs a, cudaStream_t s) {
   const size_t smem = orth_smem<W, RW>(c.kcap);
-  HM_CUDA(cudaFuncSetAttribute(k_orth<W, NT, RW, CL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  // the limit is the function's, not this launch's: always that of the widest
+  // basis, so that threads that build at once do not lower one another's
+  HM_CUDA(cudaFuncSetAttribute(k_orth<W, NT, RW, CL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)orth_smem<W, RW>(kMaxCols)));
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3((unsigned)c.count * c.cluster);
   cfg.blockDim = dim3(NT);
