@@ -76,7 +76,8 @@ struct PhaseTrace {
 // ms for every allocation after a synchronisation.  (A 2^17-point build spent
 // 75 of its 200 ms there.)  The pool keeps at most kPoolKeep bytes that are not
 // in use, a fortieth of the device's memory; hm_release_memory hands them
-// back, and so does an allocation that fails.  Safe from any thread.
+// back, and so does an allocation that fails.  Safe from any thread, also while
+// a stream is being captured.
 constexpr size_t kPoolMax = size_t(1) << 30, kPoolKeep = size_t(4) << 30;
 // On the current device (*dev): usable on every stream on return; in the order of s.
 cudaError_t dev_alloc(void** p, size_t bytes, int* dev);

@@ -1,6 +1,7 @@
 // hm_memory.cu -- the library's device memory: cudaMalloc for large blocks, a
 // bounded pool per device for the small ones (hm_internal.h).
 #include <mutex>
+#include <vector>
 
 #include "hm_internal.h"
 
@@ -9,12 +10,29 @@ namespace {
 
 constexpr int kMaxDevices = 64;
 
+struct Block {
+  void* p;
+  size_t bytes;
+};
+
 struct DevicePool {
   cudaMemPool_t pool = nullptr;
   cudaStream_t stream = nullptr;  // orders the allocations of long-lived blocks
+  std::vector<void*> tokens;      // see wait_device
+  std::vector<Block> parked;      // released, but not yet known to be out of use
 };
 std::mutex g_mu;
 DevicePool g_pools[kMaxDevices];
+
+// Lets this thread allocate and release while a stream is being captured, by
+// itself or by another thread: neither touches what is captured.
+struct WhileCapturing {
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  WhileCapturing() { cudaThreadExchangeStreamCaptureMode(&mode); }
+  ~WhileCapturing() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
+constexpr size_t kToken = 256;
 
 // The current device's pool, made on its first use.
 cudaError_t device_pool(DevicePool** out, int* dev) {
@@ -22,6 +40,7 @@ cudaError_t device_pool(DevicePool** out, int* dev) {
   if (e != cudaSuccess) return e;
   if (*dev >= kMaxDevices) return cudaErrorInvalidDevice;
   DevicePool& P = g_pools[*dev];
+  WhileCapturing guard;
   std::lock_guard<std::mutex> lock(g_mu);
   if (!P.pool) {
     cudaMemPoolProps pr{};
@@ -36,6 +55,13 @@ cudaError_t device_pool(DevicePool** out, int* dev) {
       cudaMemPoolDestroy(pool);
       return e;
     }
+    // two tokens: one stays while the other is released, so that the driver's
+    // block that holds them stays mapped
+    for (int i = 0; i < 2; ++i) {
+      void* t = nullptr;
+      if (cudaMalloc(&t, kToken) == cudaSuccess) P.tokens.push_back(t);
+    }
+    cudaGetLastError();
     P.pool = pool;
   }
   *out = &P;
@@ -58,10 +84,74 @@ struct OnDevice {
   }
 };
 
+// Waits for the device's work on every stream, graphs in flight included, by
+// releasing a small cudaMalloc block: cudaFree synchronises (30.0 ms behind a
+// 30 ms kernel on a non-blocking stream) and may be called while streams are
+// being captured.  cudaDeviceSynchronize may not: whichever thread captures and
+// in whatever mode, it fails and invalidates that capture.  On an idle device
+// 3.5 us, the next token included, against 1.5.
+cudaError_t wait_device(DevicePool* P) {
+  WhileCapturing guard;
+  void* t = nullptr;
+  {
+    std::lock_guard<std::mutex> lock(g_mu);
+    if (!P->tokens.empty()) {
+      t = P->tokens.back();
+      P->tokens.pop_back();
+    }
+  }
+  cudaError_t e = cudaSuccess;
+  if (!t && (e = cudaMalloc(&t, kToken)) == cudaErrorMemoryAllocation) {
+    cudaGetLastError();
+    cudaMemPoolTrimTo(P->pool, 0);  // what is idle already
+    e = cudaMalloc(&t, kToken);
+  }
+  if (e == cudaSuccess) e = cudaFree(t);
+  if (e == cudaSuccess && cudaMalloc(&t, kToken) == cudaSuccess) {
+    std::lock_guard<std::mutex> lock(g_mu);
+    P->tokens.push_back(t);
+  }
+  cudaGetLastError();  // reported by e, or the next call makes its own token
+  return e;
+}
+
+// Blocks of long-lived buffers, after a wait: to the pool, or to the device.
+void give_block(DevicePool* P, const Block& b) {
+  WhileCapturing guard;
+  const cudaError_t e = b.bytes >= kPoolMax ? cudaFree(b.p) : cudaFreeAsync(b.p, P->stream);
+  if (e != cudaSuccess) {
+    cudaGetLastError();  // not the caller's
+    std::lock_guard<std::mutex> lock(g_mu);
+    P->parked.push_back(b);
+  }
+}
+
+// A wait, and what earlier waits that failed left behind with it.
+cudaError_t wait_and_unpark(DevicePool* P) {
+  std::vector<Block> parked;
+  {
+    std::lock_guard<std::mutex> lock(g_mu);
+    parked.swap(P->parked);
+  }
+  const cudaError_t e = wait_device(P);
+  for (const Block& b : parked) {
+    if (e == cudaSuccess) {
+      give_block(P, b);
+    } else {
+      std::lock_guard<std::mutex> lock(g_mu);
+      P->parked.push_back(b);
+    }
+  }
+  return e;
+}
+
 // What the pool keeps goes back to the device.
 cudaError_t give_back(DevicePool* P) {
-  const cudaError_t e = cudaDeviceSynchronize();  // releases in flight count as kept only then
-  return e != cudaSuccess ? e : cudaMemPoolTrimTo(P->pool, 0);
+  const cudaError_t e = wait_and_unpark(P);  // releases in flight count as kept only then
+  if (e != cudaSuccess) return e;
+  WhileCapturing guard;
+  const cudaError_t sync = cudaStreamSynchronize(P->stream);
+  return sync != cudaSuccess ? sync : cudaMemPoolTrimTo(P->pool, 0);
 }
 
 cudaError_t pool_alloc(DevicePool* P, void** p, size_t bytes, cudaStream_t s) {
@@ -75,6 +165,7 @@ cudaError_t pool_alloc(DevicePool* P, void** p, size_t bytes, cudaStream_t s) {
 }
 
 cudaError_t large_alloc(DevicePool* P, void** p, size_t bytes) {
+  WhileCapturing guard;
   cudaError_t e = cudaMalloc(p, bytes);
   if (e == cudaErrorMemoryAllocation) {
     cudaGetLastError();
@@ -105,21 +196,25 @@ cudaError_t dev_alloc_async(void** p, size_t bytes, cudaStream_t s, int* dev) {
 }
 
 void dev_free(void* p, size_t bytes, int dev) {
-  if (bytes >= kPoolMax) {
-    cudaFree(p);
+  OnDevice on(dev);
+  DevicePool* P = &g_pools[dev];
+  const Block b{p, bytes};
+  // cudaFree waits by itself; a block of the pool may be in use on any stream
+  if (bytes >= kPoolMax || wait_and_unpark(P) == cudaSuccess) {
+    give_block(P, b);
     return;
   }
-  OnDevice on(dev);
-  cudaDeviceSynchronize();  // as cudaFree: the block may be in use on any stream
-  cudaFreeAsync(p, g_pools[dev].stream);
+  std::lock_guard<std::mutex> lock(g_mu);
+  P->parked.push_back(b);
 }
 
 void dev_free_async(void* p, size_t bytes, cudaStream_t s, int dev) {
+  if (bytes >= kPoolMax) {
+    dev_free(p, bytes, dev);
+    return;
+  }
   OnDevice on(dev);
-  if (bytes >= kPoolMax)
-    cudaFree(p);
-  else
-    cudaFreeAsync(p, s);
+  cudaFreeAsync(p, s);
 }
 
 }  // namespace hm
