@@ -821,8 +821,7 @@ hm_status hmatrix_build(hm_kdtree t, hm_structure s, const double* d_points, con
 
   tr.mark("problems", stream, -1, 0);
   // ---- batches bounded by the workspace budget -----------------------------
-  size_t freeb = 0, totb = 0;
-  HM_CUDA(cudaMemGetInfo(&freeb, &totb));
+  const size_t freeb = dev_available();
   // per-problem results that survive the batch: rank (-1: stored dense, -2:
   // split into its child blocks), low-part columns, and the factor location.
   // A problem that misses the tolerance at its rank cap above the leaf level
@@ -876,10 +875,29 @@ hm_status hmatrix_build(hm_kdtree t, hm_structure s, const double* d_points, con
     auto need_of = [&](const Prob& P) {
       return ((size_t)ara_ld(P.m) * (std::min(P.kmax, kQCols) + wmax) + (size_t)ara_ld(P.n) * kMaxBs) * sizeof(W);
     };
+    // The most a problem can come to if its basis reaches the cap: every width
+    // its basis had (superseded ones stay until the end of the batch), B, the
+    // packed basis, the Gram partials and its factors or dense blocks.  A batch
+    // whose blocks all did would need up to 12 times the budget, so the sum over
+    // a batch stays within three quarters of the memory there is.
+    auto most_of = [&](const Prob& P) {
+      const size_t m = ara_ld(P.m), n = ara_ld(P.n), k = P.kmax;
+      size_t q = std::min(P.kmax, kQCols), w = q + wmax;
+      while (q < k) w += q = std::min(2 * q, k);
+      size_t bytes = (m * w + n * k) * sizeof(W);
+      if (fastW) bytes += (size_t)(P.m + kCC - 1) / kCC * (kCC / 16) * q_tiles(P.kmax) * 32 * sizeof(uint4);
+      const size_t kt = std::min<size_t>(k, kTruncMax);
+      bytes += kt * kt * ((n + 2047) / 2048 * sizeof(double) + sizeof(float));
+      const size_t factors = (size_t)(P.m + P.n) * k, blocks = P.level == depth ? 2 * (size_t)P.m * P.n : 0;
+      return bytes + std::max(factors, blocks) * sizeof(float);
+    };
+    DevBuf<W> ws, wb;  // Q and Y; B (kept from batch to batch)
+    size_t room = 0;   // memory for the next batch
     size_t budget = 0;
     int gen_bs0 = 0;  // first-round columns of the problems listed last
     long long gen_end = 0;
     auto next_batch = [&](long long ps) {
+      room = (dev_available() + (ws.n + wb.n) * sizeof(W)) / 4 * 3;
       if (ps >= gen_end) {
         gen_end = (long long)probs.size();
         size_t all = 0;
@@ -892,16 +910,16 @@ hm_status hmatrix_build(hm_kdtree t, hm_structure s, const double* d_points, con
         budget = std::min(std::max(all / 8, kBatchMin), std::min<size_t>(freeb / 8, kBatchMax));
       }
       long long pe = ps;
-      size_t sz = 0;
+      size_t sz = 0, most = 0;
       while (pe < gen_end) {
         const size_t need = need_of(probs[pe]);
-        if (pe > ps && sz + need > budget) break;
+        most += most_of(probs[pe]);
+        if (pe > ps && (sz + need > budget || most > room)) break;
         sz += need;
         ++pe;
       }
       return pe;
     };
-    DevBuf<W> ws, wb;  // Q and Y; B (kept from batch to batch)
     while (pstart < (long long)probs.size()) {
       const long long pend = next_batch(pstart);
       const int nb = (int)(pend - pstart);

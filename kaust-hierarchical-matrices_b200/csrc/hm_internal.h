@@ -82,6 +82,7 @@ constexpr size_t kPoolMax = size_t(1) << 30, kPoolKeep = size_t(4) << 30;
 // On the current device (*dev): usable on every stream on return; in the order of s.
 cudaError_t dev_alloc(void** p, size_t bytes, int* dev);
 cudaError_t dev_alloc_async(void** p, size_t bytes, cudaStream_t s, int* dev);
+size_t dev_available();  // bytes of the current device that are free, the pool's idle part included
 void dev_free(void* p, size_t bytes, int dev);  // after all work of the device, as cudaFree
 void dev_free_async(void* p, size_t bytes, cudaStream_t s, int dev);
 

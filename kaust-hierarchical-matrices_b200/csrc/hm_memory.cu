@@ -195,6 +195,18 @@ cudaError_t dev_alloc_async(void** p, size_t bytes, cudaStream_t s, int* dev) {
   return bytes >= kPoolMax ? large_alloc(P, p, bytes) : pool_alloc(P, p, bytes, s);
 }
 
+size_t dev_available() {
+  DevicePool* P = nullptr;
+  int dev = 0;
+  size_t freeb = 0, total = 0;
+  unsigned long long held = 0, used = 0;
+  if (cudaMemGetInfo(&freeb, &total) != cudaSuccess || device_pool(&P, &dev) != cudaSuccess ||
+      cudaMemPoolGetAttribute(P->pool, cudaMemPoolAttrReservedMemCurrent, &held) != cudaSuccess ||
+      cudaMemPoolGetAttribute(P->pool, cudaMemPoolAttrUsedMemCurrent, &used) != cudaSuccess)
+    return freeb;
+  return freeb + (held > used ? held - used : 0);
+}
+
 void dev_free(void* p, size_t bytes, int dev) {
   OnDevice on(dev);
   DevicePool* P = &g_pools[dev];
