@@ -266,10 +266,11 @@ __global__ void k_gather_rows(const float* __restrict__ X, int ldx, const int* _
     Xp[c * n + i] = X[c * ldx + perm[i]];
 }
 
-__global__ void k_scatter_rows(const float* __restrict__ Yp, const int* __restrict__ perm, int n,
+// Rows [r0, r1) of the tree order: a block-row shard's, or all n.
+__global__ void k_scatter_rows(const float* __restrict__ Yp, const int* __restrict__ perm, int n, int r0, int r1,
                                float* __restrict__ Y, int ldy) {
   const size_t c = blockIdx.y;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+  for (int i = r0 + blockIdx.x * blockDim.x + threadIdx.x; i < r1; i += gridDim.x * blockDim.x)
     Y[c * ldy + perm[i]] = Yp[c * n + i];
 }
 
@@ -285,14 +286,15 @@ __global__ void k_narrow_rows(const double* __restrict__ X, int ldx, const int* 
   }
 }
 
-// ... and the FP32 result Yp (ld n) widened into Y (double, ldy; rows
-// scattered through perm when perm != null)
-__global__ void k_widen_rows(const float* __restrict__ Yp, const int* __restrict__ perm, int n, int nrhs,
-                             double* __restrict__ Y, int ldy) {
-  long long tot = (long long)n * nrhs;
+// ... and rows [r0, r1) of the FP32 result Yp (ld n) widened into Y (double,
+// ldy; rows scattered through perm when perm != null)
+__global__ void k_widen_rows(const float* __restrict__ Yp, const int* __restrict__ perm, int n, int r0, int r1,
+                             int nrhs, double* __restrict__ Y, int ldy) {
+  const int m = r1 - r0;
+  long long tot = (long long)m * nrhs;
   for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < tot;
        e += (long long)gridDim.x * blockDim.x) {
-    int i = (int)(e % n), c = (int)(e / n);
+    int i = r0 + (int)(e % m), c = (int)(e / m);
     Y[(size_t)c * ldy + (perm ? perm[i] : i)] = (double)Yp[(size_t)c * n + i];
   }
 }
@@ -538,6 +540,8 @@ hm_status hmatvec(hm_hmatrix h, int trans, int nrhs, const float* X, int ldx, fl
   // dense blocks are generated from a symmetric kernel), so H^T X = H X
   MatvecPlan& P = h->plan;
   const int n = h->n;
+  // the rows that are written: a block-row shard leaves the others untouched
+  const int r0 = h->tree->h_offsets[h->leaf_lo], r1 = h->tree->h_offsets[h->leaf_hi];
   for (int c0 = 0; c0 < nrhs;) {
     const int nr = std::min(pass_width(h), nrhs - c0);
     const float* Xin = X + (size_t)c0 * ldx;
@@ -572,7 +576,7 @@ hm_status hmatvec(hm_hmatrix h, int trans, int nrhs, const float* X, int ldx, fl
     HM_TRY(run_panel(h, nr, Xt, ldxt, Yt, ldyt, P.T.p, original_order && fuse_x ? perm : nullptr,
                      original_order && fuse_y ? perm : nullptr, stream, nullptr));
     if (original_order && !fuse_y) {
-      k_scatter_rows<<<grid, 256, 0, stream>>>(P.Yp.p, perm, n, Yout, ldy);
+      k_scatter_rows<<<grid, 256, 0, stream>>>(P.Yp.p, perm, n, r0, r1, Yout, ldy);
       HM_LAUNCH_CHECK();
     }
     c0 += nr;
@@ -593,12 +597,13 @@ hm_status hmatvec_f64(hm_hmatrix h, int trans, int nrhs, const double* X, int ld
   MatvecPlan& P = h->plan;
   const int n = h->n;
   const int* perm = original_order ? h->tree->perm.p : nullptr;
+  const int r0 = h->tree->h_offsets[h->leaf_lo], r1 = h->tree->h_offsets[h->leaf_hi];  // as in hmatvec
   for (int c0 = 0; c0 < nrhs;) {
     const int nr = std::min(pass_width(h), nrhs - c0);
     k_narrow_rows<<<592, 256, 0, stream>>>(X + (size_t)c0 * ldx, ldx, perm, n, nr, P.Xp.p);
     HM_LAUNCH_CHECK();
     HM_TRY(run_panel(h, nr, P.Xp.p, n, P.Yp.p, n, P.T.p, nullptr, nullptr, stream, nullptr));
-    k_widen_rows<<<592, 256, 0, stream>>>(P.Yp.p, perm, n, nr, Y + (size_t)c0 * ldy, ldy);
+    k_widen_rows<<<592, 256, 0, stream>>>(P.Yp.p, perm, n, r0, r1, nr, Y + (size_t)c0 * ldy, ldy);
     HM_LAUNCH_CHECK();
     c0 += nr;
   }
