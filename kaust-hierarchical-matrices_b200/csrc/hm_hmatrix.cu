@@ -1380,7 +1380,7 @@ hm_status hmatrix_build(hm_kdtree t, hm_structure s, const double* d_points, con
     hm_status mst = mixed_build(h, mp, md, stream);
     if (mst) return cleanup(mst);
     if (opt.precision == HM_PREC_MIXED) {
-      h->stats.mixed_bytes = (h->mx.store_tiles - h->mx.tc_dense_tiles) * 512;
+      h->stats.mixed_bytes = h->mx.store_tiles * 512;
       release_fp32(h);
     }
   }

@@ -56,6 +56,22 @@ __host__ __device__ __forceinline__ int p1_slot(int lane) {
   return 4 * g + (t ^ ((g >> 1) & 3));
 }
 
+// A dense tile (32 rows x 32 columns of a dense block, hi or lo, 2 KB) is the
+// image of a K-major tcgen05 operand with the 64-byte swizzle, columns along K
+// in X's order: group q of eight 64-byte rows holds rows rho(q, 0..7), 16-byte
+// chunk t of a row its columns rho(t, 0..7), rho(a, e) = 8 (e / 2) + 2 a + e % 2.
+// The warp-level kernel reads the same tile: lane (g, t) finds row g + 8 w of
+// its A fragments' columns {2t, 2t+1 | + 8 | + 16 | + 24} in one 16-byte word, a
+// quarter-warp's words are whole 128-byte lines, and no second copy is kept.
+__host__ __device__ __forceinline__ int dense_word(int row, int t) {
+  const int w = row >> 3;
+  return 32 * ((row & 7) >> 1) + 8 * w + 4 * (row & 1) + (t ^ w);
+}
+// From row g's word of a tile (64-byte aligned rows) to row g + 8 w's.
+__device__ __forceinline__ const uint4* dense_row(const uint4* p, int w) {
+  return reinterpret_cast<const uint4*>(reinterpret_cast<uintptr_t>(p) ^ (uintptr_t)(16 * w)) + 8 * w;
+}
+
 __device__ __forceinline__ void mma_a4(float (&d)[4], const uint4& a, uint32_t b0, uint32_t b1) {
   mma_bf16(d, a.x, a.y, a.z, a.w, b0, b1);
 }
@@ -599,6 +615,21 @@ __device__ __forceinline__ void mx_p2_step_hi(float (&acc)[2][2][4], const uint4
   }
 }
 
+// acc[nb] += A (16 rows x 16 columns, fragments a hi, c lo) X (16 x 8, hi and lo)
+__device__ __forceinline__ void mx_p2_dense(float (&acc)[2][4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
+                                            uint32_t c0, uint32_t c1, uint32_t c2, uint32_t c3, const uint4& xh,
+                                            const uint4& xl) {
+#pragma unroll
+  for (int nb = 0; nb < 2; ++nb) {
+    const uint32_t bh0 = nb ? xh.y : xh.x, bh1 = nb ? xh.w : xh.z, bl0 = nb ? xl.y : xl.x, bl1 = nb ? xl.w : xl.z;
+    float d[4] = {0.f, 0.f, 0.f, 0.f};
+    mma_bf16(d, a0, a1, a2, a3, bl0, bl1);
+    mma_bf16(d, c0, c1, c2, c3, bh0, bh1);
+    mma_bf16(d, a0, a1, a2, a3, bh0, bh1);
+    add4(acc[nb], d);
+  }
+}
+
 // One row tile (32 rows of one leaf): every ancestor cluster's panel rows
 // times its T, then the dense blocks of the leaf row.
 // (one warp per CTA, 28 per SM, measured: the kernel is bound by loads in
@@ -609,9 +640,10 @@ __device__ __forceinline__ void mx_p2_step_hi(float (&acc)[2][2][4], const uint4
 // same row tile, part group w % WPC parts w NH .., and share its factor tiles
 // through L1.
 // SP > 1 (few row tiles, passes of up to 32): SP warps share the row tile's
-// sources.  A source step is one pair of column tiles; steps with low parts
-// count twice; the steps are laid end to end and warp s takes the s-th
-// of SP equal runs.  The warps' sums are added in order.
+// sources.  A source step is one pair of column tiles, or a dense block's
+// 32-column tile; a pair with low parts counts two, a dense tile four; the
+// steps are laid end to end and warp s takes the s-th of SP equal runs.  The
+// warps' sums are added in order.
 constexpr int kP2PerSm = 28, kP2PerSm2 = 16;
 template <int NH, int WPC, int SP>
 __global__ void __launch_bounds__(32 * WPC * SP, (NH == 1 && SP == 1 ? kP2PerSm : kP2PerSm2) / (WPC * SP))
@@ -737,49 +769,79 @@ __global__ void __launch_bounds__(32 * WPC * SP, (NH == 1 && SP == 1 ? kP2PerSm 
       }
     }
   }
-  int at = SP > 1 ? __shfl_sync(0xffffffffu, my_end, 31) : 0;
-  for (int q0 = d0; q0 < d1; q0 += 32) {
-    // up to 32 dense blocks' descriptors at once
-    long long my_dh = 0, my_dl = 0;
-    int my_x = 0, my_c = 0, my_e = 0;
-    if (q0 + lane < d1) {
-      const MxDense D = dense[leaf_dblk[q0 + lane]];
-      const long long rt = G - D.row_tile0;
-      my_dh = D.hi + rt * D.nct;
-      my_dl = D.lo + rt * D.nct;
-      my_x = D.col_tile0;
-      my_c = D.nct;
-    }
-    if (SP > 1) my_e = at + warp_scan(my_c, lane);
-    const int nq = min(32, d1 - q0);
-    for (int q = 0; q < nq; ++q) {
-      const int nct = __shfl_sync(0xffffffffu, my_c, q);
-      int ca = 0, cb = nct;  // this warp's column tiles (nct is a multiple of 4)
-      if (SP > 1) {
-        int a, b;
-        run(__shfl_sync(0xffffffffu, my_e, q) - nct, nct >> 1, 2, a, b);
-        ca = 2 * a;
-        cb = 2 * b;
-        if (ca >= cb) continue;
-      }
-      const uint4* dh = store + __shfl_sync(0xffffffffu, my_dh, q) * 32 + lane;
-      const uint4* dl = store + __shfl_sync(0xffffffffu, my_dl, q) * 32 + lane;
-      const int xt0 = __shfl_sync(0xffffffffu, my_x, q);
-#pragma unroll(SP == 1 ? 1 : 2)
-      for (int ct = ca; ct < cb; ct += 2) {
-        const uint4 h0 = ld_tile<SH>(dh + ct * 32), h1 = ld_tile<SH>(dh + (ct + 1) * 32);
-        const uint4 l0 = ld_tile<SH>(dl + ct * 32), l1 = ld_tile<SH>(dl + (ct + 1) * 32);
-        const size_t xt = (size_t)(xt0 + (ct >> 2)) * 128 + (size_t)((ct >> 1) & 1) * 32 + lane;
+  if (SP == 1) {
+    // Descriptors as they come, and 16 columns a step in 8-byte words: what this
+    // variant holds at 28 warps per SM.  2^20 points, 16 right-hand sides: 2065
+    // us against 2074 with the loop below, 2260 with both row halves of a tile
+    // in one step; 2^18 points, 64 right-hand sides: 1393 against 1423.
+    for (int q = d0; q < d1; ++q) {
+      const MxDense& D = dense[leaf_dblk[q]];
+      const uint4* dh = store + (D.hi + (long long)(G - D.row_tile0) * D.nct) * 32 + dense_word(lane >> 2, lane & 3);
+      const uint4* dl = dh + (D.lo - D.hi) * 32;
+      const int xt0 = D.col_tile0, nc2 = D.nct >> 1;
+#pragma unroll 1
+      for (int c2 = 0; c2 < nc2; ++c2) {
+        const int tile = (c2 >> 1) * 128, half = c2 & 1;
+        uint2 rh[4], rl[4];  // rows g + 8 w
+#pragma unroll
+        for (int w = 0; w < 4; ++w) {
+          rh[w] = __ldg(reinterpret_cast<const uint2*>(dense_row(dh + tile, w)) + half);
+          rl[w] = __ldg(reinterpret_cast<const uint2*>(dense_row(dl + tile, w)) + half);
+        }
+        const size_t xt = (size_t)(xt0 + (c2 >> 1)) * 128 + lane + 32 * half;
 #pragma unroll
         for (int h = 0; h < NH; ++h) {
           const uint4 xh = __ldg(Xf + h * xh_ + xt), xl = __ldg(Xf + h * xh_ + xt + 64);
-          const uint32_t bh[2][2] = {{xh.x, xh.z}, {xh.y, xh.w}};
-          const uint32_t bl[2][2] = {{xl.x, xl.z}, {xl.y, xl.w}};
-          mx_p2_step(acc[h], h0, h1, l0, l1, bh, bl, true);
+#pragma unroll
+          for (int mt = 0; mt < 2; ++mt)
+            mx_p2_dense(acc[h][mt], rh[2 * mt].x, rh[2 * mt + 1].x, rh[2 * mt].y, rh[2 * mt + 1].y, rl[2 * mt].x,
+                        rl[2 * mt + 1].x, rl[2 * mt].y, rl[2 * mt + 1].y, xh, xl);
         }
       }
     }
-    if (SP > 1) at = __shfl_sync(0xffffffffu, my_e, 31);
+  }
+  int at = SP > 1 ? __shfl_sync(0xffffffffu, my_end, 31) : 0;
+  for (int q0 = d0; SP > 1 && q0 < d1; q0 += 32) {
+    // up to 32 dense blocks' descriptors at once
+    long long my_dh = 0;
+    int my_dl = 0, my_x = 0, my_c = 0;  // my_dl: from the high parts to the low ones
+    if (q0 + lane < d1) {
+      const MxDense D = dense[leaf_dblk[q0 + lane]];
+      my_dh = D.hi + (long long)(G - D.row_tile0) * D.nct;
+      my_dl = (int)(D.lo - D.hi);
+      my_x = D.col_tile0;
+      my_c = D.nct;
+    }
+    const int my_e = at + warp_scan(my_c, lane);
+    const int nq = min(32, d1 - q0);
+    for (int q = 0; q < nq; ++q) {
+      const int nct = __shfl_sync(0xffffffffu, my_c, q);
+      int ca, cb;  // this warp's 32-column tiles
+      run(__shfl_sync(0xffffffffu, my_e, q) - nct, nct >> 2, 4, ca, cb);
+      if (ca >= cb) continue;
+      const uint4* dh = store + __shfl_sync(0xffffffffu, my_dh, q) * 32 + dense_word(lane >> 2, lane & 3);
+      const uint4* dl = dh + (long long)__shfl_sync(0xffffffffu, my_dl, q) * 32;
+      const int xt0 = __shfl_sync(0xffffffffu, my_x, q);
+      // rows 16 mt + g and + 8 of every tile in turn
+#pragma unroll
+      for (int mt = 0; mt < 2; ++mt) {
+#pragma unroll(NH == 2 ? 1 : 2)
+        for (int ct = ca; ct < cb; ++ct) {
+          const uint4 h0 = ld_tile<SH>(dense_row(dh + ct * 128, 2 * mt));
+          const uint4 h1 = ld_tile<SH>(dense_row(dh + ct * 128, 2 * mt + 1));
+          const uint4 l0 = ld_tile<SH>(dense_row(dl + ct * 128, 2 * mt));
+          const uint4 l1 = ld_tile<SH>(dense_row(dl + ct * 128, 2 * mt + 1));
+          const size_t xt = (size_t)(xt0 + ct) * 128 + lane;
+#pragma unroll
+          for (int h = 0; h < NH; ++h) {
+            const uint4* xp = Xf + h * xh_ + xt;
+            mx_p2_dense(acc[h][mt], h0.x, h1.x, h0.y, h1.y, l0.x, l1.x, l0.y, l1.y, __ldg(xp), __ldg(xp + 64));
+            mx_p2_dense(acc[h][mt], h0.z, h1.z, h0.w, h1.w, l0.z, l1.z, l0.w, l1.w, __ldg(xp + 32), __ldg(xp + 96));
+          }
+        }
+      }
+    }
+    at = __shfl_sync(0xffffffffu, my_e, 31);
   }
   const int base = leaf_off[x] + 32 * (G - leaf_tile0[x]), lim = leaf_off[x + 1];
   // sum i of lane L: half i / 16, rows 16 mt + g (+ 8), column 8 nb + 2 t (+ 1) of C fragment (mt, nb)
@@ -862,7 +924,7 @@ __global__ void k_mx_conv_panels(const MxPanel* __restrict__ panels, const long 
   }
 }
 
-// One warp per 32 x 8 tile of a dense block (P2 order, hi + lo)
+// One warp per quarter (rows g + 8 w) of a 32 x 32 dense tile, hi and lo (dense_word's order)
 __global__ void k_mx_conv_dense(const MxDense* __restrict__ dense, const long long* __restrict__ unit_start,
                                 int ndense, long long nunits, const int* __restrict__ tile_leaf,
                                 const int* __restrict__ leaf_tile0, const int* __restrict__ leaf_off,
@@ -873,36 +935,28 @@ __global__ void k_mx_conv_dense(const MxDense* __restrict__ dense, const long lo
   const int di = find_item(unit_start, ndense, w);
   const MxDense D = dense[di];
   const long long local = w - unit_start[di];
-  const int rt = (int)(local / D.nct), ct = (int)(local % D.nct);
+  const int rt = (int)(local / D.nct), quarter = (int)(local % D.nct), ct = quarter >> 2, w8 = quarter & 3;
   const int G = D.row_tile0 + rt;
   const int x = tile_leaf[G];
   const int rbase = leaf_off[x] + 32 * (G - leaf_tile0[x]) - D.r0;
   const int rlim = leaf_off[x + 1] - D.r0;
-  const int pc = 8 * ct + 2 * t;  // padded column (even; pc and pc + 1 share a 32-column tile)
-  const int GC = D.col_tile0 + (pc >> 5);
+  const int GC = D.col_tile0 + ct;
   const int y = tile_leaf[GC];
-  const int cbase = leaf_off[y] + 32 * (GC - leaf_tile0[y]) - D.c0 + (pc & 31);
+  const int cbase = leaf_off[y] + 32 * (GC - leaf_tile0[y]) - D.c0 + 2 * t;
   const int clim = leaf_off[y + 1] - D.c0;
   auto val = [&](int r, int c) -> float {
     const int lr = rbase + r;
     return (lr < rlim && c < clim) ? D.src[(size_t)c * D.m + lr] : 0.f;
   };
+  const int r = g + 8 * w8;
   uint4 h, l;
-  split_bf16x2(val(g, cbase), val(g, cbase + 1), h.x, l.x);
-  split_bf16x2(val(g + 8, cbase), val(g + 8, cbase + 1), h.y, l.y);
-  split_bf16x2(val(g + 16, cbase), val(g + 16, cbase + 1), h.z, l.z);
-  split_bf16x2(val(g + 24, cbase), val(g + 24, cbase + 1), h.w, l.w);
-  store[(D.hi + (long long)rt * D.nct + ct) * 32 + lane] = h;
-  store[(D.lo + (long long)rt * D.nct + ct) * 32 + lane] = l;
-  // the P1 copy: lane (g, t) holds column 8 (g / 2) + 2 (ct % 4) + g % 2 of the
-  // 32-column tile at rows 2t, 2t+1, 2t+8, .. (k_mx_conv_panels' order)
-  const int c1 = leaf_off[y] + 32 * (GC - leaf_tile0[y]) - D.c0 + 8 * (g >> 1) + 2 * (ct & 3) + (g & 1);
-  split_bf16x2(val(2 * t, c1), val(2 * t + 1, c1), h.x, l.x);
-  split_bf16x2(val(2 * t + 8, c1), val(2 * t + 9, c1), h.y, l.y);
-  split_bf16x2(val(2 * t + 16, c1), val(2 * t + 17, c1), h.z, l.z);
-  split_bf16x2(val(2 * t + 24, c1), val(2 * t + 25, c1), h.w, l.w);
-  store[(D.hi1 + (long long)rt * D.nct + ct) * 32 + p1_slot(lane)] = h;
-  store[(D.lo1 + (long long)rt * D.nct + ct) * 32 + p1_slot(lane)] = l;
+  split_bf16x2(val(r, cbase), val(r, cbase + 1), h.x, l.x);
+  split_bf16x2(val(r, cbase + 8), val(r, cbase + 9), h.y, l.y);
+  split_bf16x2(val(r, cbase + 16), val(r, cbase + 17), h.z, l.z);
+  split_bf16x2(val(r, cbase + 24), val(r, cbase + 25), h.w, l.w);
+  const long long tile = (long long)rt * D.nct + 4 * ct;
+  store[(D.hi + tile) * 32 + dense_word(r, t)] = h;
+  store[(D.lo + tile) * 32 + dense_word(r, t)] = l;
 }
 
 // A stored pair's columns in the panels: factor columns fu, fv at panel columns
@@ -1143,7 +1197,6 @@ hm_status mixed_build(hm_hmatrix_s* h, const std::vector<MxPair>& pairs, const s
   std::vector<MxDense> dense;
   std::vector<std::vector<int>> leaf_d(nleaf);
   long long bytes_dense = 0;
-  M.tc_dense_tiles = 0;
   for (const MxDenseIn& di : dense_in) {
     if (di.m <= 0 || di.n <= 0) continue;
     int xs, xe, ys, ye;
@@ -1162,14 +1215,7 @@ hm_status mixed_build(hm_hmatrix_s* h, const std::vector<MxPair>& pairs, const s
     D.hi = tiles;
     tiles += (long long)D.nrt * D.nct * tu;
     D.lo = tiles;
-    if (!f32) {
-      const long long nt = (long long)D.nrt * D.nct;
-      tiles += nt;
-      D.hi1 = tiles;
-      D.lo1 = tiles + nt;
-      tiles += 2 * nt;
-      M.tc_dense_tiles += 2 * nt;
-    }
+    if (!f32) tiles += (long long)D.nrt * D.nct;
     for (int x = xs; x < xe; ++x) leaf_d[x].push_back((int)dense.size());
     locs.push_back(MxLoc{di.D, 1, (int)dense.size(), di.m, di.n, 0, 0, 0});
     dense.push_back(D);
@@ -1261,7 +1307,7 @@ hm_status mixed_build(hm_hmatrix_s* h, const std::vector<MxPair>& pairs, const s
           const MxDense& D = dense[dblk[q]];
           const long long rb = G0 - D.row_tile0;
           for (int j0 = 0; j0 < D.nct; j0 += 4)
-            steps.push_back(P2Step{D.hi1 + rb * D.nct + j0, D.lo1 + rb * D.nct + j0,
+            steps.push_back(P2Step{D.hi + rb * D.nct + j0, D.lo + rb * D.nct + j0,
                                    (long long)(D.col_tile0 + j0 / 4) * 1024, (long long)(D.col_tile0 + j0 / 4) * 1024 + 512,
                                    D.nct, D.nct, 2 | (4 << 2) | (mask_of(k, k2) << 8), 0});
         }
@@ -1368,6 +1414,13 @@ __device__ __forceinline__ float p2_elem(const uint4* __restrict__ store, long l
   return (cc & 1) ? bf16_hi_as_float(w) : bf16_lo_as_float(w);
 }
 
+// element (rr, cc) of the dense tile at unit `tile`, as a float
+__device__ __forceinline__ float dense_elem(const uint4* __restrict__ store, long long tile, int rr, int cc) {
+  const uint4* word = store + tile * 32 + dense_word(rr, (cc & 7) >> 1);
+  const uint32_t w = reinterpret_cast<const uint32_t*>(word)[cc >> 3];
+  return (cc & 1) ? bf16_hi_as_float(w) : bf16_lo_as_float(w);
+}
+
 __global__ void k_mx_unpack(const UnpackJob* __restrict__ jobs, const long long* __restrict__ start, int njobs,
                             long long total, const MxPanel* __restrict__ panels, const MxDense* __restrict__ dense,
                             const uint4* __restrict__ store, const int* __restrict__ leaf_off,
@@ -1378,13 +1431,13 @@ __global__ void k_mx_unpack(const UnpackJob* __restrict__ jobs, const long long*
   const UnpackJob J = jobs[j];
   const long long local = e - start[j];
   const int r = (int)(local % J.rows), c = (int)(local / J.rows);
-  int G, rr, ct, cc;
+  int G, rr, cc;
   long long thi, tlo = -1;
   if (J.kind == 0) {
     const MxPanel P = panels[J.idx];
     row_tile(leaf_off, leaf_tile0, nleaf, P.r0 + r, &G, &rr);
     const int pc = c < J.khi ? J.colL + c : J.colH + c - J.khi;
-    ct = pc >> 3;
+    const int ct = pc >> 3;
     cc = pc & 7;
     thi = P.hi2 + (long long)(G - P.tile0) * P.nct + ct;
     if (ct < P.nctl) tlo = P.lo2 + (long long)(G - P.tile0) * P.nctl + ct;
@@ -1393,16 +1446,14 @@ __global__ void k_mx_unpack(const UnpackJob* __restrict__ jobs, const long long*
     row_tile(leaf_off, leaf_tile0, nleaf, D.r0 + r, &G, &rr);
     int GC, cr;
     row_tile(leaf_off, leaf_tile0, nleaf, D.c0 + c, &GC, &cr);
-    const int pc = (GC - D.col_tile0) * 32 + cr;
-    ct = pc >> 3;
-    cc = pc & 7;
-    thi = D.hi + (long long)(G - D.row_tile0) * D.nct + ct;
-    tlo = D.lo + (long long)(G - D.row_tile0) * D.nct + ct;
+    cc = cr;
+    thi = D.hi + (long long)(G - D.row_tile0) * D.nct + 4 * (GC - D.col_tile0);
+    tlo = thi + D.lo - D.hi;
   }
-  const float hi = p2_elem(store, thi, rr, cc);
+  const float hi = J.kind ? dense_elem(store, thi, rr, cc) : p2_elem(store, thi, rr, cc);
   float y = hi;
   if (tlo >= 0) {
-    const float lo = p2_elem(store, tlo, rr, cc);
+    const float lo = J.kind ? dense_elem(store, tlo, rr, cc) : p2_elem(store, tlo, rr, cc);
     y = hi + lo;  // exact: hi + lo has at most 24 significant bits
     // a tie (|lo| half a BF16 ulp of hi) would round to the other neighbour
     if (bf16_lo_as_float(pack_bf16(y, 0.f)) != hi) y = nextafterf(y, hi);

@@ -78,17 +78,15 @@ struct TcUnit {
 // A rows of the block's tiles that the source does not cover (mask bit k
 // clear) are zero.
 struct P2Step {
-  long long a_hi, a_lo;  // P1 tile (512-byte units) of the block's tile 0 at the step's first column tile
+  long long a_hi, a_lo;  // P1 or dense tile (512-byte units) of the block's tile 0 at the step's first column tile
   long long b_hi, b_lo;  // 16-byte offset of B: T blocks (kinds 0, 1) or X's image (kind 2)
   int a_stride, a_stride_lo;  // tiles per row tile of the source (hi, lo)
   int info;                   // kind | column tiles << 2 | mask << 8
   int pad;
 };
 
-struct MxDense {  // a dense block in P2 order, hi + lo, [row tile][col tile]
+struct MxDense {  // a dense block, hi + lo, [row tile][32-column tile] (FP32 format: [row tile][col tile])
   long long hi, lo;
-  long long hi1, lo1;        // BF16 format: a copy in P1 order for 128-column passes; column tile 4 i + c holds
-                             // columns 32 i + 8 (g / 2) + 2 c + g % 2, g = 0..7 (X's image's K order)
   int row_tile0, col_tile0;  // global row tiles of its row and column clusters
   int nrt, nct;              // nct: 8-column tiles, a multiple of 4
   int r0, c0, m, n;
@@ -112,7 +110,6 @@ struct MxPlan {
   DevBuf<uint4> store;  // all BF16 tiles
   long long store_tiles = 0;
   long long zero_tile = 0;   // eight zero tiles past the last one
-  long long tc_dense_tiles = 0;  // the dense blocks' P1 copies, read by 128-column passes only
   DevBuf<MxPanel> panels;
   int num_panels = 0;
   DevBuf<int> pan_of;      // heap-ordered cluster (2^l - 1 + a) -> panel or -1

@@ -62,8 +62,9 @@
 // engine moves it as it is; the rows of D come out in the tiles' order rho and
 // go to their place at the store.  (Rearranging the other tile order by 4-byte
 // cp.async with 27 copy warps took 1.15 ms at 131072 mixture points.)  Dense
-// blocks keep a copy in the same order for these passes, their columns in X's row order rho so that B
-// is X's image of the column cluster's tile.  Panels' columns with low parts
+// blocks' 32 x 32 tiles are K-major images as stored (dense_word): their rows
+// are in the same order rho, their columns in X's, so that B is X's image of
+// the column cluster's tile.  Panels' columns with low parts
 // take three products per 16 columns, 32 columns per step; the others one per
 // 16 columns, 64 per step; dense blocks three per 16 columns, 32 per step.
 #include <atomic>
@@ -403,7 +404,9 @@ __global__ void k_mx_reduce_tc(const int2* __restrict__ mtiles, long long nmt, c
 // tile k at 4096 k), B_hi 16384 (8 K blocks).  A: column tiles as stored (P1
 // order), 512 bytes each, M-major with the 64-byte swizzle: 32 rows of a
 // column are 64 contiguous bytes, the row tiles (LBO) and the groups of 8
-// columns (512 = SBO) apart; row i of a tile is rho(i / 8, i % 8).  B: T blocks
+// columns (512 = SBO) apart; kind 2: dense tiles as stored, K-major with the
+// 64-byte swizzle, groups of 8 rows 512 (SBO) apart.  Row i of a tile is
+// rho(i / 8, i % 8).  B: T blocks
 // MN-major (right-hand side n at 2 (n % 8) + 128 (n / 8), column c at 16 c;
 // SBO 128, LBO 2048), X's image K-major (n at 16 (n % 8) + 128 (n / 8); SBO
 // 128, LBO 2048).  Row tiles outside a step's mask, the odd last column tile
@@ -413,7 +416,6 @@ constexpr int kP2Bufs = 4;       // TMEM accumulators of 128 columns (all 512)
 constexpr int kP2Chain = 4;      // steps per MMA chain
 constexpr int kP2BarBytes = 8 * (2 * kP2Stages + 2 * kP2Bufs + 1);
 constexpr size_t kP2Smem = (size_t)kP2Stages * kTcStage + kP2BarBytes + 16;
-constexpr uint32_t kIdescAmn = kIdesc | (1u << 15);      // A MN-major
 constexpr uint32_t kIdescABmn = kIdescBmn | (1u << 15);  // A and B MN-major
 
 __global__ void __launch_bounds__(kTcThreads, 1)
@@ -521,6 +523,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
     __syncwarp();
   } else if (warp == kMmaWarp) {  // ---- MMA issuer (lane 0; the others hold descriptors)
     const uint64_t adesc0 = tc_sdesc_sw64_mn(sbase, 2048, 512), adesc1 = tc_sdesc_sw64_mn(sbase, 4096, 512);
+    const uint64_t adesc2 = tc_sdesc_sw64(sbase, 512);   // dense tiles: groups of 8 rows, row tiles end to end
     const uint64_t bdesc0 = tc_sdesc(sbase, 2048, 128);  // T blocks and X's image: SBO 128, LBO 2048
     long long j = 0;
     int chain = -1;
@@ -544,11 +547,14 @@ __global__ void __launch_bounds__(kTcThreads, 1)
             const int kind = info & 3, cnt = (info >> 2) & 15, nq = kind == 3 ? 1 : (cnt + 1) >> 1;
             // this stage's start; an offset of o bytes adds o >> 4 to the start address field
             const uint64_t off = (uint64_t)((s * kTcStage) >> 4);
-            const uint64_t da = (kind == 1 ? adesc1 : adesc0) + off, db = bdesc0 + off;
+            const uint64_t da = (kind == 1 ? adesc1 : kind == 2 ? adesc2 : adesc0) + off, db = bdesc0 + off;
             const uint32_t d = tmem + (uint32_t)((chain % kP2Bufs) * 128);
             uint32_t acc = in_chain == 0 ? 0u : 1u;
-            const uint32_t idesc = kind == 2 ? kIdescAmn : kIdescABmn;  // T blocks are MN-major, X's image K-major
-            // 16 columns at a time: two column tiles (1024 bytes of A), two K blocks (4096 of B at 16384)
+            // dense tiles and X's image are K-major, panels' tiles and T blocks MN-major
+            const uint32_t idesc = kind == 2 ? kIdesc : kIdescABmn;
+            // 16 columns at a time: two column tiles (1024 bytes of A) or half a dense tile's rows (32 bytes),
+            // two K blocks (4096 bytes of B at 16384)
+            const uint32_t aq = kind == 2 ? 2u : 64u;
             if (kind == 1) {
 #pragma unroll
               for (int q = 0; q < 4; ++q)
@@ -557,10 +563,10 @@ __global__ void __launch_bounds__(kTcThreads, 1)
 #pragma unroll
               for (int q = 0; q < 2; ++q)
                 if (q < nq) {
-                  tc_mma_bf16(d, da + q * 64, db + (1024 + q * 256), idesc, q ? 1u : acc);  // U_hi T_hi
+                  tc_mma_bf16(d, da + q * aq, db + (1024 + q * 256), idesc, q ? 1u : acc);  // U_hi T_hi
                   if (kind != 3) {
-                    tc_mma_bf16(d, da + q * 64, db + (1536 + q * 256), idesc, 1u);        // U_hi T_lo
-                    tc_mma_bf16(d, da + (512 + q * 64), db + (1024 + q * 256), idesc, 1u);  // U_lo T_hi
+                    tc_mma_bf16(d, da + q * aq, db + (1536 + q * 256), idesc, 1u);        // U_hi T_lo
+                    tc_mma_bf16(d, da + (512 + q * aq), db + (1024 + q * 256), idesc, 1u);  // U_lo T_hi
                   }
                 }
             }
