@@ -427,17 +427,29 @@ struct LocalArgs {
 };
 
 constexpr unsigned kNone = 0xffffu;  // no point at this position
-constexpr size_t kLocalBoxes = 2 * 32 * kMaxDim * sizeof(double);  // k_local's static shared memory
-constexpr size_t kLocalMaxSmem = 227 * 1024 - kLocalBoxes;         // what a CTA may have beyond it
+constexpr size_t kLocalMaxSmem = 227 * 1024;  // what a CTA may have
+constexpr int kLocalMaxCap = 1 << 13;         // most points of a segment (eight positions per thread)
 
 struct LocalSmem {
   double* coord;        // [d][seg_cap]
   int* idx;             // [seg_cap]
-  unsigned* key;        // [pcap] leading 32 bits of the point's split coordinate (order preserving)
+  unsigned* key;        // [pcap] leading 32 bits of the point's split coordinate (order preserving), while a
+                        // level sorts
+  double* box;          // [2][warps][d] a segment's warps' boxes, between sorts (the same memory)
   unsigned short* ord;  // [pcap] position -> slot
   int* ldims;           // local levels' split dims, level j at [2^(j-j0) - 1]
   int* adims;           // ancestors' split dims for levels < j0
 };
+
+__host__ __device__ __forceinline__ int local_threads(int pcap) {
+  return pcap / 2 > kLocalThreads ? kLocalThreads : pcap / 2 > 128 ? pcap / 2 : 128;
+}
+// The keys (a tree of one leaf sorts nothing) or the warps' boxes, whichever is more.
+__host__ __device__ __forceinline__ size_t local_scratch_bytes(int d, int pcap, int nlocal) {
+  const size_t keys = nlocal > 0 ? sizeof(unsigned) * (size_t)pcap : 0;
+  const size_t boxes = 2 * sizeof(double) * (size_t)(local_threads(pcap) / 32) * d;
+  return keys > boxes ? keys : boxes;
+}
 
 __device__ __forceinline__ int local_dim(const LocalArgs& a, const LocalSmem& sm, int root, int lv,
                                          int node) {
@@ -472,16 +484,16 @@ __device__ __noinline__ bool chain_less(const LocalArgs& a, const LocalSmem& sm,
 // 0.60 ms, 2^20 points (256 CTAs) 2.48 -> 0.53 ms.
 __global__ void __launch_bounds__(kLocalThreads) k_local(LocalArgs a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  __shared__ double rmin[32][kMaxDim], rmax[32][kMaxDim];  // a segment's warps' boxes
   LocalSmem sm;
   size_t off = 0;
   sm.coord = reinterpret_cast<double*>(smem_raw);
   off += sizeof(double) * (size_t)a.d * a.seg_cap;
   sm.idx = reinterpret_cast<int*>(smem_raw + off);
   off += sizeof(int) * (size_t)a.seg_cap;
-  sm.key = reinterpret_cast<unsigned*>(smem_raw + off);
-  off += sizeof(unsigned) * (size_t)a.pcap;
   int nlocal = a.depth - a.j0;  // local levels that sort
+  sm.key = reinterpret_cast<unsigned*>(smem_raw + off);
+  sm.box = reinterpret_cast<double*>(smem_raw + off);
+  off += local_scratch_bytes(a.d, a.pcap, nlocal);
   sm.ldims = reinterpret_cast<int*>(smem_raw + off);
   off += sizeof(int) * (size_t)((1 << nlocal) + 1);
   sm.adims = reinterpret_cast<int*>(smem_raw + off);
@@ -547,8 +559,8 @@ __global__ void __launch_bounds__(kLocalThreads) k_local(LocalArgs a) {
         }
         if (lane == 0) {
           if (wps > 1) {
-            rmin[warp][k] = mn;
-            rmax[warp][k] = mx;
+            sm.box[warp * a.d + k] = mn;
+            sm.box[(nwarp + warp) * a.d + k] = mx;
           } else {
             a.bmin[gnode * a.d + k] = mn;
             a.bmax[gnode * a.d + k] = mx;
@@ -573,10 +585,12 @@ __global__ void __launch_bounds__(kLocalThreads) k_local(LocalArgs a) {
         int best = 0;
         double bspan = 0;
         for (int k = 0; k < a.d; ++k) {
-          double mn = rmin[t * wps][k], mx = rmax[t * wps][k];
+          const double* lo = sm.box + t * wps * a.d + k;
+          const double* hi = lo + nwarp * a.d;
+          double mn = lo[0], mx = hi[0];
           for (int w = 1; w < wps; ++w) {
-            mn = fmin(mn, rmin[t * wps + w][k]);
-            mx = fmax(mx, rmax[t * wps + w][k]);
+            mn = fmin(mn, lo[w * a.d]);
+            mx = fmax(mx, hi[w * a.d]);
           }
           a.bmin[gnode * a.d + k] = mn;
           a.bmax[gnode * a.d + k] = mx;
@@ -670,7 +684,7 @@ __global__ void __launch_bounds__(kLocalThreads) k_local(LocalArgs a) {
 }
 
 size_t local_smem_bytes(int d, int seg_cap, int pcap, int nlocal) {
-  return sizeof(double) * (size_t)d * seg_cap + sizeof(int) * (size_t)seg_cap + sizeof(unsigned) * (size_t)pcap +
+  return sizeof(double) * (size_t)d * seg_cap + sizeof(int) * (size_t)seg_cap + local_scratch_bytes(d, pcap, nlocal) +
          sizeof(int) * (size_t)((1 << nlocal) + 1) + sizeof(int) * (size_t)(kMaxDepth + 1) +
          sizeof(unsigned short) * (size_t)pcap + 64;
 }
@@ -712,8 +726,8 @@ hm_status kdtree_build(const double* d_points, int n, int d, int bucket, cudaStr
   if (depth > kMaxDepth) return fail(HM_ERR_UNSUPPORTED, "hm_kdtree_build: tree too deep");
 
   // shared-memory capacity of the local phase: largest power of two whose
-  // per-point state fits in 216 KB (8 KB more hold the warps' boxes)
-  int seg_cap = 1 << 13;
+  // per-point state fits in 216 KB
+  int seg_cap = kLocalMaxCap;
   while (seg_cap > 64 && local_smem_bytes(d, seg_cap, seg_cap, 1) +
                                  sizeof(int) * (size_t)(4 * seg_cap / std::max(bucket, 1) + 4) >
                              216 * 1024)
@@ -728,6 +742,9 @@ hm_status kdtree_build(const double* d_points, int n, int d, int bucket, cudaStr
   int pcap = 32;  // at least a warp's
   while (pcap < maxlen) pcap <<= 1;
   const int nlocal = depth - j0;
+  const size_t smem = local_smem_bytes(d, pcap, pcap, nlocal);
+  if (pcap > kLocalMaxCap || smem > kLocalMaxSmem)  // one leaf of many points
+    return fail(HM_ERR_UNSUPPORTED, "hm_kdtree_build: bucket too large for this dimension");
 
   hm_kdtree_s* t = new hm_kdtree_s();
   t->n = n;
@@ -882,13 +899,12 @@ hm_status kdtree_build(const double* d_points, int n, int d, int bucket, cudaStr
   la.perm = t->perm.p;
   la.pts_tree = t->pts_tree.p;
   la.pts_tree_f = t->pts_tree_f.p;
-  const size_t smem = local_smem_bytes(d, pcap, pcap, nlocal);
   // the limit is the function's, not this launch's: always the most it can
   // have, so that threads that build at once do not lower one another's
   if ((s = cu(cudaFuncSetAttribute(k_local, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kLocalMaxSmem),
               "cudaFuncSetAttribute")))
     return cleanup(s);
-  k_local<<<1 << j0, std::min(kLocalThreads, std::max(128, pcap / 2)), smem, stream>>>(la);
+  k_local<<<1 << j0, local_threads(pcap), smem, stream>>>(la);
   if ((s = cu(cudaGetLastError(), "k_local"))) return cleanup(s);
   if ((s = cu(cudaStreamSynchronize(stream), "sync"))) return cleanup(s);
   *out = t;
