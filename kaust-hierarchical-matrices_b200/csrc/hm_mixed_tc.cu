@@ -232,10 +232,10 @@ __global__ void __launch_bounds__(kTcThreads, 1)
         j += nsteps;
       }
     }
-    // Every step's MMAs wait for its copies, so these have landed when the MMAs
-    // are done; after a wait that gave up, the copies this warp may still have
-    // in flight are waited for here (bounded).
-    if (failed && lane == 0)
+    // The kernel may not end with copies in flight.  The MMAs wait for every
+    // step's, but not once any role has given up, which this warp need not have
+    // seen: its last copies are waited for here (bounded), whatever happened.
+    if (lane == 0)
       for (long long js = last; js >= 0 && js > last - kP1Stages; js -= kCopyWarps)
         mbar_wait(full + 8u * (uint32_t)(js % kP1Stages), (uint32_t)((js / kP1Stages) & 1), kWaitClocks / 8);
     __syncwarp();
@@ -514,10 +514,10 @@ __global__ void __launch_bounds__(kTcThreads, 1)
       }
       j += ns;
     }
-    // Every step's MMAs wait for its copies, so these have landed when the MMAs
-    // are done; after a wait that gave up, the copies this warp may still have
-    // in flight are waited for here (bounded).
-    if (failed && lane == 0)
+    // The kernel may not end with copies in flight.  The MMAs wait for every
+    // step's, but not once any role has given up, which this warp need not have
+    // seen: its last copies are waited for here (bounded), whatever happened.
+    if (lane == 0)
       for (long long js = last; js >= 0 && js > last - kP2Stages; js -= kCopyWarps)
         mbar_wait(full + 8u * (uint32_t)(js % kP2Stages), (uint32_t)((js / kP2Stages) & 1), kWaitClocks / 8);
     __syncwarp();
