@@ -160,7 +160,7 @@ struct MxPlan {
   int p2_blocks = 0;
   DevBuf<int> p2_cta_ptr, p2_cta_blocks;  // CTA c's blocks: p2_cta_blocks[p2_cta_ptr[c] .. p2_cta_ptr[c + 1])
   int p2_ctas = 0;
-  DevBuf<int> tc_err;  // set when a bounded wait of those kernels gave up
+  DevBuf<int> tc_err;  // a bounded wait of those kernels gave up: 1 phase 1, 2 phase 2, 3 both
   bool tc_pass(int halves) const { return wide_tc && fmt == 0 && halves == 8; }
   // scratch of one 16-column panel of right-hand sides, in floats: X
   // fragments, chunk partials, T (the projections by expanding column: BF16

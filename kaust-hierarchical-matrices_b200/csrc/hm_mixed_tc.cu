@@ -352,10 +352,10 @@ __global__ void __launch_bounds__(kTcThreads, 1)
       }
     }
   }
-  if (failed) atomicExch(err, 1);
+  if (failed) atomicOr(err, 1);
   // the tensor memory is released once every MMA is done (thread 0 waits,
   // bounded; the others wait at the barrier)
-  if (tid == 0 && !mbar_wait(done, 0, 5 * kWaitClocks)) atomicExch(err, 1);
+  if (tid == 0 && !mbar_wait(done, 0, 5 * kWaitClocks)) atomicOr(err, 1);
   tc_fence_before();
   __syncthreads();
   if (warp == 0) {
@@ -632,8 +632,8 @@ __global__ void __launch_bounds__(kTcThreads, 1)
       for (int i = 0; i < kDrainCols; ++i) acc[i] = 0.f;
     }
   }
-  if (failed) atomicExch(err, 1);
-  if (tid == 0 && !mbar_wait(done, 0, 5 * kWaitClocks)) atomicExch(err, 1);
+  if (failed) atomicOr(err, 2);
+  if (tid == 0 && !mbar_wait(done, 0, 5 * kWaitClocks)) atomicOr(err, 2);
   tc_fence_before();
   __syncthreads();
   if (warp == 0) {
@@ -690,5 +690,7 @@ extern "C" hm_status hm_hmatrix_check(hm_hmatrix h, void* stream) {
   HM_CUDA(cudaMemcpy(&v, h->mx.tc_err.p, sizeof v, cudaMemcpyDeviceToHost));
   if (v == 0) return HM_OK;
   HM_CUDA(cudaMemset(h->mx.tc_err.p, 0, sizeof v));
-  return fail(HM_ERR_TIMEOUT, "a bounded wait of the tcgen05 phase-1 kernel gave up: products since the last check are wrong");
+  return fail(HM_ERR_TIMEOUT, std::string("a bounded wait of the tcgen05 ") +
+                                  (v == 1 ? "phase-1 kernel" : v == 2 ? "phase-2 kernel" : "kernels of both phases") +
+                                  " gave up: products since the last check are wrong");
 }
