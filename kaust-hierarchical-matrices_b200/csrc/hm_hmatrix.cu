@@ -892,12 +892,12 @@ hm_status hmatrix_build(hm_kdtree t, hm_structure s, const double* d_points, con
       return bytes + std::max(factors, blocks) * sizeof(float);
     };
     DevBuf<W> ws, wb;  // Q and Y; B (kept from batch to batch)
-    size_t room = 0;   // memory for the next batch
+    size_t room = freeb / 4 * 3;  // memory for the next batch
     size_t budget = 0;
     int gen_bs0 = 0;  // first-round columns of the problems listed last
     long long gen_end = 0;
     auto next_batch = [&](long long ps) {
-      room = (dev_available() + (ws.n + wb.n) * sizeof(W)) / 4 * 3;
+      if (ps > 0) room = (dev_available() + (ws.n + wb.n) * sizeof(W)) / 4 * 3;
       if (ps >= gen_end) {
         gen_end = (long long)probs.size();
         size_t all = 0;
