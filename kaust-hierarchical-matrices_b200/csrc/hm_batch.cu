@@ -229,6 +229,9 @@ hm_status hm_batch_matvec(hm_batch b, int nrhs, const float* X, int ldx, float* 
   return HM_OK;
 }
 
-void hm_batch_free(hm_batch b) { delete b; }
+void hm_batch_free(hm_batch b) {
+  hm::FreeTogether together;
+  delete b;
+}
 
 }  // extern "C"

@@ -177,6 +177,9 @@ hm_status hm_kdtree_copy_out(hm_kdtree t, int* perm, int* offsets, double* bmin,
 const int* hm_kdtree_device_perm(hm_kdtree t) { return t ? t->perm.p : nullptr; }
 const int* hm_kdtree_device_offsets(hm_kdtree t) { return t ? t->offsets.p : nullptr; }
 
-void hm_kdtree_free(hm_kdtree t) { delete t; }
+void hm_kdtree_free(hm_kdtree t) {
+  hm::FreeTogether together;
+  delete t;
+}
 
 }  // extern "C"

@@ -478,7 +478,7 @@ hm_status fp32_convert(hm_hmatrix_s* h, const float* const* colsrc, const std::v
       tot += (long long)panels[p].nrt * panels[p].nct;
     }
     DevBuf<long long> dstart;
-    HM_TRY(dstart.alloc(np));
+    HM_TRY(dstart.alloc_async(np, s));
     HM_CUDA(cudaMemcpyAsync(dstart.p, start.data(), sizeof(long long) * np, cudaMemcpyHostToDevice, s));
     if (tot > 0) {
       k_fp_conv_panels<<<(unsigned)((tot * 32 + 255) / 256), 256, 0, s>>>(
@@ -495,7 +495,7 @@ hm_status fp32_convert(hm_hmatrix_s* h, const float* const* colsrc, const std::v
       tot += (long long)dense[i].nrt * dense[i].nct;
     }
     DevBuf<long long> ds;
-    HM_TRY(ds.alloc(dense.size()));
+    HM_TRY(ds.alloc_async(dense.size(), s));
     HM_CUDA(cudaMemcpyAsync(ds.p, start.data(), sizeof(long long) * start.size(), cudaMemcpyHostToDevice, s));
     if (tot > 0) {
       k_fp_conv_dense<<<(unsigned)((tot * 32 + 255) / 256), 256, 0, s>>>(

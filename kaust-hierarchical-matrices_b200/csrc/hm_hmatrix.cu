@@ -897,7 +897,6 @@ hm_status hmatrix_build(hm_kdtree t, hm_structure s, const double* d_points, con
     int gen_bs0 = 0;  // first-round columns of the problems listed last
     long long gen_end = 0;
     auto next_batch = [&](long long ps) {
-      if (ps > 0) room = (dev_available() + (ws.n + wb.n) * sizeof(W)) / 4 * 3;
       if (ps >= gen_end) {
         gen_end = (long long)probs.size();
         size_t all = 0;
@@ -911,9 +910,14 @@ hm_status hmatrix_build(hm_kdtree t, hm_structure s, const double* d_points, con
       }
       long long pe = ps;
       size_t sz = 0, most = 0;
+      bool asked = ps == 0;  // (70 us: only a batch of some size asks again)
       while (pe < gen_end) {
         const size_t need = need_of(probs[pe]);
         most += most_of(probs[pe]);
+        if (!asked && most > freeb / 16) {
+          asked = true;
+          room = (dev_available() + (ws.n + wb.n) * sizeof(W)) / 4 * 3;
+        }
         if (pe > ps && (sz + need > budget || most > room)) break;
         sz += need;
         ++pe;
@@ -935,7 +939,7 @@ hm_status hmatrix_build(hm_kdtree t, hm_structure s, const double* d_points, con
         for (int tt = 0; tt * kTR < P.n; ++tt) items_cols.push_back(make_int2(i, tt));
       }
       if (off > ws.n) {
-        hm_status st0 = ws.alloc(off);
+        hm_status st0 = ws.alloc_async(off, stream);
         if (st0) return st0;
       }
       off = 0;
@@ -1079,7 +1083,7 @@ hm_status hmatrix_build(hm_kdtree t, hm_structure s, const double* d_points, con
       {
         size_t bsz = 0;
         for (int i = 0; i < nb; ++i) bsz += (size_t)ara_ld(bp[i].n) * hst[i].k;
-        if (bsz > wb.n && (st = wb.alloc(bsz))) return st;
+        if (bsz > wb.n && (st = wb.alloc_async(bsz, stream))) return st;
         bsz = 0;
         for (int i = 0; i < nb; ++i) {
           bp[i].b = wb.p + bsz;
@@ -1310,7 +1314,7 @@ hm_status hmatrix_build(hm_kdtree t, hm_structure s, const double* d_points, con
     DevBuf<float> chunk;
     DevBuf<DenseItem> ddi;
     hm_status st;
-    if ((st = chunk.alloc(std::max<size_t>(tot, 1))) || (st = ddi.alloc(nown))) return cleanup(st);
+    if ((st = chunk.alloc(std::max<size_t>(tot, 1))) || (st = ddi.alloc_async(nown, stream))) return cleanup(st);
     HM_CUDA(cudaMemcpyAsync(ddi.p, dens.data(), sizeof(DenseItem) * nown, cudaMemcpyHostToDevice, stream));
     k_dense_gen<<<nown, 256, 0, stream>>>(ddi.p, t->pts_tree_f.p, t->n, t->d, h->kp, chunk.p);
     HM_LAUNCH_CHECK();
@@ -1411,7 +1415,10 @@ hm_status hmatrix_build(hm_kdtree t, hm_structure s, const double* d_points, con
 void release_fp32(hm_hmatrix_s* h) {
   h->chunk_meta.clear();
   for (const auto& c : h->storage) h->chunk_meta.push_back({c.p, c.n});
-  h->storage.clear();
+  {
+    FreeTogether together;
+    h->storage.clear();
+  }
   h->fp32_released = true;
 }
 
@@ -1534,6 +1541,9 @@ hm_status hm_hmatrix_dense_block(hm_hmatrix h, int i, float* D) {
   return HM_OK;
 }
 
-void hm_hmatrix_free(hm_hmatrix h) { delete h; }
+void hm_hmatrix_free(hm_hmatrix h) {
+  hm::FreeTogether together;
+  delete h;
+}
 
 }  // extern "C"

@@ -85,6 +85,24 @@ cudaError_t dev_alloc_async(void** p, size_t bytes, cudaStream_t s, int* dev);
 size_t dev_available();  // bytes of the current device that are free, the pool's idle part included
 void dev_free(void* p, size_t bytes, int dev);  // after all work of the device, as cudaFree
 void dev_free_async(void* p, size_t bytes, cudaStream_t s, int dev);
+// What dev_free is given on this thread while one of these lives is released
+// at its end, after one wait for all of it: an object's buffers.
+class FreeTogether {
+ public:
+  FreeTogether();
+  ~FreeTogether();
+  FreeTogether(const FreeTogether&) = delete;
+  FreeTogether& operator=(const FreeTogether&) = delete;
+  struct Block {
+    void* p;
+    size_t bytes;
+    int dev;
+  };
+  std::vector<Block> blocks;
+
+ private:
+  FreeTogether* outer;
+};
 
 // ---- device buffer RAII -----------------------------------------------------
 // alloc: long-lived buffers.  alloc_async: temporaries of a build step, used

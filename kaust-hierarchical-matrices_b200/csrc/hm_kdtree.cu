@@ -789,6 +789,7 @@ hm_status kdtree_build(const double* d_points, int n, int d, int bucket, cudaStr
     const int maxw = depth + 2;
     const int nseg_max = 1 << (j0 - 1);
     const size_t wide_nodes = (size_t)((1 << j0) - 1);
+    FreeTogether together;  // one wait for all of these
     DevBuf<unsigned long long> bmin_tw, bmax_tw, chosen;
     DevBuf<SelState> st;
     DevBuf<unsigned int> hist;
@@ -873,8 +874,6 @@ hm_status kdtree_build(const double* d_points, int n, int d, int bucket, cudaStr
     k_untwiddle<<<64, 256, 0, stream>>>(wide_nodes * d, bmin_tw.p, t->bmin.p);
     k_untwiddle<<<64, 256, 0, stream>>>(wide_nodes * d, bmax_tw.p, t->bmax.p);
     if ((s = cu(cudaGetLastError(), "k_untwiddle"))) return cleanup(s);
-    // the device buffers above are freed at scope exit: make sure the GPU is
-    // done with them first
     int h_err = 0;
     if ((s = cu(cudaMemcpyAsync(&h_err, err.p, 4, cudaMemcpyDeviceToHost, stream), "err")) ||
         (s = cu(cudaStreamSynchronize(stream), "sync")))

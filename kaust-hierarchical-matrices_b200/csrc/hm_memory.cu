@@ -10,10 +10,7 @@ namespace {
 
 constexpr int kMaxDevices = 64;
 
-struct Block {
-  void* p;
-  size_t bytes;
-};
+using Block = FreeTogether::Block;
 
 struct DevicePool {
   cudaMemPool_t pool = nullptr;
@@ -115,6 +112,8 @@ cudaError_t wait_device(DevicePool* P) {
   return e;
 }
 
+thread_local FreeTogether* t_together = nullptr;
+
 // Blocks of long-lived buffers, after a wait: to the pool, or to the device.
 void give_block(DevicePool* P, const Block& b) {
   WhileCapturing guard;
@@ -208,9 +207,13 @@ size_t dev_available() {
 }
 
 void dev_free(void* p, size_t bytes, int dev) {
+  const Block b{p, bytes, dev};
+  if (t_together) {
+    t_together->blocks.push_back(b);
+    return;
+  }
   OnDevice on(dev);
   DevicePool* P = &g_pools[dev];
-  const Block b{p, bytes};
   // cudaFree waits by itself; a block of the pool may be in use on any stream
   if (bytes >= kPoolMax || wait_and_unpark(P) == cudaSuccess) {
     give_block(P, b);
@@ -218,6 +221,30 @@ void dev_free(void* p, size_t bytes, int dev) {
   }
   std::lock_guard<std::mutex> lock(g_mu);
   P->parked.push_back(b);
+}
+
+FreeTogether::FreeTogether() : outer(t_together) { t_together = this; }
+
+FreeTogether::~FreeTogether() {
+  t_together = outer;
+  if (outer) {
+    outer->blocks.insert(outer->blocks.end(), blocks.begin(), blocks.end());
+    return;
+  }
+  for (size_t i = 0; i < blocks.size();) {  // runs of blocks of one device
+    const int dev = blocks[i].dev;
+    OnDevice on(dev);
+    DevicePool* P = &g_pools[dev];
+    const cudaError_t e = wait_and_unpark(P);
+    for (; i < blocks.size() && blocks[i].dev == dev; ++i) {
+      if (e == cudaSuccess || blocks[i].bytes >= kPoolMax) {
+        give_block(P, blocks[i]);
+      } else {
+        std::lock_guard<std::mutex> lock(g_mu);
+        P->parked.push_back(blocks[i]);
+      }
+    }
+  }
 }
 
 void dev_free_async(void* p, size_t bytes, cudaStream_t s, int dev) {

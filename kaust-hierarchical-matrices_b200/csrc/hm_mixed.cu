@@ -1035,9 +1035,11 @@ std::vector<int> deal(const std::vector<long long>& cost, int ctas, std::vector<
   return order;
 }
 
+// build_only: the buffer is used and released in the order of s
 template <class T>
-hm_status upload(DevBuf<T>& b, const std::vector<T>& v, cudaStream_t s) {
-  HM_TRY(b.alloc(std::max<size_t>(v.size(), 1)));
+hm_status upload(DevBuf<T>& b, const std::vector<T>& v, cudaStream_t s, bool build_only = false) {
+  const size_t n = std::max<size_t>(v.size(), 1);
+  HM_TRY(build_only ? b.alloc_async(n, s) : b.alloc(n));
   if (!v.empty()) HM_CUDA(cudaMemcpyAsync(b.p, v.data(), sizeof(T) * v.size(), cudaMemcpyHostToDevice, s));
   return HM_OK;
 }
@@ -1255,9 +1257,9 @@ hm_status mixed_build(hm_hmatrix_s* h, const std::vector<MxPair>& pairs, const s
   {
     DevBuf<PairColumns> dpc;
     DevBuf<int> mirror;  // partner column (an involution), -1 for padding
-    HM_TRY(upload(dpc, pcols, s));
-    HM_TRY(colsrc.alloc(std::max<size_t>(ncols, 1)));
-    HM_TRY(mirror.alloc(std::max<size_t>(ncols, 1)));
+    HM_TRY(upload(dpc, pcols, s, true));
+    HM_TRY(colsrc.alloc_async(std::max<size_t>(ncols, 1), s));
+    HM_TRY(mirror.alloc_async(std::max<size_t>(ncols, 1), s));
     HM_TRY(M.tslot.alloc(std::max<size_t>(ncols, 1)));
     HM_TRY(M.tslot_tc.alloc(f32 ? 1 : std::max<size_t>(ncols, 1)));
     if (ncols > 0) {
@@ -1356,7 +1358,7 @@ hm_status mixed_build(hm_hmatrix_s* h, const std::vector<MxPair>& pairs, const s
       start[p] = tot;
       tot += (long long)panels[p].nrt * panels[p].nct;
     }
-    HM_TRY(upload(dstart, start, s));
+    HM_TRY(upload(dstart, start, s, true));
     if (tot > 0) {
       k_mx_conv_panels<<<(unsigned)((tot * 32 + 255) / 256), 256, 0, s>>>(
           M.panels.p, dstart.p, np, tot, colsrc.p, M.tile_leaf.p, M.leaf_tile0.p, h->tree->offsets.p, M.store.p);
@@ -1372,7 +1374,7 @@ hm_status mixed_build(hm_hmatrix_s* h, const std::vector<MxPair>& pairs, const s
       tot += (long long)dense[i].nrt * dense[i].nct;
     }
     DevBuf<long long> ds;
-    HM_TRY(upload(ds, start, s));
+    HM_TRY(upload(ds, start, s, true));
     if (tot > 0) {
       k_mx_conv_dense<<<(unsigned)((tot * 32 + 255) / 256), 256, 0, s>>>(
           M.dense.p, ds.p, (int)dense.size(), tot, M.tile_leaf.p, M.leaf_tile0.p, h->tree->offsets.p, M.store.p);
@@ -1499,8 +1501,8 @@ hm_status mixed_unpack(hm_hmatrix_s* h, const std::vector<std::pair<int, float*>
   if (tot == 0) return HM_OK;
   DevBuf<UnpackJob> dj;
   DevBuf<long long> ds;
-  HM_TRY(upload(dj, uj, s));
-  HM_TRY(upload(ds, start, s));
+  HM_TRY(upload(dj, uj, s, true));
+  HM_TRY(upload(ds, start, s, true));
   k_mx_unpack<<<(unsigned)((tot + 255) / 256), 256, 0, s>>>(dj.p, ds.p, (int)uj.size(), tot, M.panels.p, M.dense.p,
                                                             M.store.p, h->tree->offsets.p, M.leaf_tile0.p,
                                                             1 << h->depth);

@@ -404,6 +404,9 @@ hm_status hm_structure_jds(hm_structure s, int level, int* row_ptr, int* csr_blk
   return HM_OK;
 }
 
-void hm_structure_free(hm_structure s) { delete s; }
+void hm_structure_free(hm_structure s) {
+  hm::FreeTogether together;
+  delete s;
+}
 
 }  // extern "C"
