@@ -80,9 +80,11 @@ HM_API const char* hm_version(void);
 
 /* Device memory.  The library keeps up to 4 GB of device memory that its
  * objects have released, for the next ones (mapping and unmapping memory costs
- * a build up to a second).  hm_release_memory waits for the current device and
- * hands that memory back; memory in use is not touched.  An allocation of the
- * library that fails does the same and tries again. */
+ * a build up to a second).  While less than 16 GB of the device are free, it
+ * keeps at most 256 MB after a build or the release of a matrix.
+ * hm_release_memory waits for the current device and hands that memory back;
+ * memory in use is not touched.  An allocation of the library that fails does
+ * the same and tries again. */
 HM_API hm_status hm_release_memory(void);
 
 /* --- points ------------------------------------------------------------- */

@@ -230,8 +230,11 @@ hm_status hm_batch_matvec(hm_batch b, int nrhs, const float* X, int ldx, float* 
 }
 
 void hm_batch_free(hm_batch b) {
-  hm::FreeTogether together;
-  delete b;
+  {
+    hm::FreeTogether together;
+    delete b;
+  }
+  hm::dev_settle();
 }
 
 }  // extern "C"

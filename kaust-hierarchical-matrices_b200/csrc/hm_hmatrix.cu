@@ -1459,7 +1459,9 @@ void hm_build_opts_default(int d, hm_build_opts* o) {
 
 hm_status hm_hmatrix_build(hm_kdtree t, hm_structure s, const double* d_points, const hm_build_opts* opts,
                            void* stream, hm_hmatrix* out) {
-  return hm::hmatrix_build(t, s, d_points, opts, hm::as_stream(stream), out, 0, -1);
+  const hm_status st = hm::hmatrix_build(t, s, d_points, opts, hm::as_stream(stream), out, 0, -1);
+  hm::dev_settle();
+  return st;
 }
 
 hm_status hm_hmatrix_build_rows(hm_kdtree t, hm_structure s, const double* d_points, const hm_build_opts* opts,
@@ -1468,7 +1470,9 @@ hm_status hm_hmatrix_build_rows(hm_kdtree t, hm_structure s, const double* d_poi
   if (!t) return hm::fail(HM_ERR_INVALID, "hm_hmatrix_build_rows: null tree");
   if (leaf_begin < 0 || leaf_begin >= leaf_end || leaf_end > (1 << t->depth))
     return hm::fail(HM_ERR_INVALID, "hm_hmatrix_build_rows: need 0 <= leaf_begin < leaf_end <= 2^depth");
-  return hm::hmatrix_build(t, s, d_points, opts, hm::as_stream(stream), out, leaf_begin, leaf_end);
+  const hm_status st = hm::hmatrix_build(t, s, d_points, opts, hm::as_stream(stream), out, leaf_begin, leaf_end);
+  hm::dev_settle();
+  return st;
 }
 
 hm_status hm_hmatrix_stats_get(hm_hmatrix h, hm_hmatrix_stats* st) {
@@ -1542,8 +1546,11 @@ hm_status hm_hmatrix_dense_block(hm_hmatrix h, int i, float* D) {
 }
 
 void hm_hmatrix_free(hm_hmatrix h) {
-  hm::FreeTogether together;
-  delete h;
+  {
+    hm::FreeTogether together;
+    delete h;
+  }
+  hm::dev_settle();
 }
 
 }  // extern "C"

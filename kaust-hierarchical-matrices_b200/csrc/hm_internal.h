@@ -75,16 +75,20 @@ struct PhaseTrace {
 // stream-ordered pool 6.5 ms/GB each way, and with no memory kept at least 0.25
 // ms for every allocation after a synchronisation.  (A 2^17-point build spent
 // 75 of its 200 ms there.)  The pool keeps at most kPoolKeep bytes that are not
-// in use, a fortieth of the device's memory; hm_release_memory hands them
-// back, and so does an allocation that fails.  Safe from any thread, also while
-// a stream is being captured.
-constexpr size_t kPoolMax = size_t(1) << 30, kPoolKeep = size_t(4) << 30;
+// in use, a fortieth of the device's memory, and after a build or the release
+// of a matrix at most kPoolLow while less than kPoolRoom of the device is free,
+// so that a program's other allocators, which cannot reclaim it, do not run out
+// because of it; hm_release_memory hands it back, and so does an allocation
+// that fails.  Safe from any thread, also while a stream is being captured.
+constexpr size_t kPoolMax = size_t(1) << 30, kPoolKeep = size_t(4) << 30, kPoolRoom = 4 * kPoolKeep,
+                 kPoolLow = size_t(256) << 20;
 // On the current device (*dev): usable on every stream on return; in the order of s.
 cudaError_t dev_alloc(void** p, size_t bytes, int* dev);
 cudaError_t dev_alloc_async(void** p, size_t bytes, cudaStream_t s, int* dev);
 size_t dev_available();  // bytes of the current device that are free, the pool's idle part included
 void dev_free(void* p, size_t bytes, int dev);  // after all work of the device, as cudaFree
 void dev_free_async(void* p, size_t bytes, cudaStream_t s, int dev);
+void dev_settle();  // see kPoolRoom
 // What dev_free is given on this thread while one of these lives is released
 // at its end, after one wait for all of it: an object's buffers.
 class FreeTogether {

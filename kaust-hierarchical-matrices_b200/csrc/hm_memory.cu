@@ -206,6 +206,25 @@ size_t dev_available() {
   return freeb + (held > used ? held - used : 0);
 }
 
+void dev_settle() {
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev >= kMaxDevices) return;
+  DevicePool* P = &g_pools[dev];
+  {
+    std::lock_guard<std::mutex> lock(g_mu);
+    if (!P->pool) return;  // nothing was allocated here yet
+  }
+  size_t freeb = 0, total = 0;
+  unsigned long long held = 0, used = 0;
+  WhileCapturing guard;
+  // (cudaMemGetInfo takes 70 us, the pool's own numbers 0.1)
+  if (cudaMemPoolGetAttribute(P->pool, cudaMemPoolAttrReservedMemCurrent, &held) == cudaSuccess &&
+      cudaMemPoolGetAttribute(P->pool, cudaMemPoolAttrUsedMemCurrent, &used) == cudaSuccess &&
+      held > used + kPoolLow && cudaMemGetInfo(&freeb, &total) == cudaSuccess && freeb < kPoolRoom)
+    give_back(P);
+  cudaGetLastError();  // the entry point's own status stands
+}
+
 void dev_free(void* p, size_t bytes, int dev) {
   const Block b{p, bytes, dev};
   if (t_together) {
