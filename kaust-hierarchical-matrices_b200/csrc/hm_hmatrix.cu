@@ -13,16 +13,17 @@
 //
 // B200 design.  Every block of every level is compressed directly from the
 // kernel function (no dense tiles in HBM, no leaf-TLR stage): each ARA pass is
-// one batched "kernel block x tall-skinny" launch (k_kmm) whose tiles are
-// generated on the fly from the tree-ordered FP32 coordinates, so the O(N^2)
-// part never touches memory.  Orthogonalisation runs per block in one CTA
-// (k_orth): block classical Gram-Schmidt applied twice against the basis, then
-// a pivoted Cholesky-QR of the sample with two Cholesky-QR refinements, Gram
-// matrices in FP64.  The kernel matrix is symmetric, so of each block pair
-// (u, v) / (v, u) only the one with v > u is compressed; the mirror block uses
-// the same factors exchanged.  Leaf blocks that do not reach the tolerance
-// within the leaf rank cap (bucket/2 as in src/constructTLRMatrix.cu:14) are
-// stored dense, as are the diagonal leaves.
+// one batched "kernel block x tall-skinny" launch (k_kmm_fast and its FP64 and
+// general forms) whose tiles are generated on the fly from the tree-ordered
+// FP32 coordinates, so the O(N^2) part never touches memory.  Orthogonalisation
+// runs per block in one CTA, tall blocks in a cluster of up to eight
+// (hm_orth.cu): block classical Gram-Schmidt applied twice against the basis,
+// then a pivoted Cholesky-QR of the sample with two Cholesky-QR refinements,
+// Gram matrices in FP64.  The kernel matrix
+// is symmetric, so of each block pair (u, v) / (v, u) only the one with v > u is
+// compressed; the mirror block uses the same factors exchanged.  Leaf blocks
+// that do not reach the tolerance within the leaf rank cap (bucket/2 as in
+// src/constructTLRMatrix.cu:14) are stored dense, as are the diagonal leaves.
 #include <algorithm>
 #include <cmath>
 #include <cstdio>
@@ -321,20 +322,18 @@ void launch_kmm64(int cols, unsigned grid, cudaStream_t s, const KmmArgs<double>
 }
 
 // ---------------------------------------------------------------------------
-// k_kmm_tc: the same product on the tensor cores (FP32 working precision).
-// CTA = 4 warps = 64 operator rows, warp = 16 rows; each lane evaluates the
-// eight kernel entries of its m16n8k16 A fragment in registers and splits
-// them into BF16 hi + lo (relative error ~2^-17 of an entry).  Sample pass:
-// W = a Gaussian table whose entries are BF16 numbers, 2 MMAs per tile.
-// Projection pass: W = Q split hi + lo, 3 MMAs per tile (hi*hi, lo*hi, hi*lo).
-// ---------------------------------------------------------------------------
-// k_kmm_fast: the tensor-core sketch product specialised on the dimension
-// (1-3), the kernel and its derivative.  Coordinates are pre-scaled so that
-// each entry costs one hardware square root and one hardware exp2 (PTX
-// sqrt.approx / ex2.approx, both within a few ulp of FP32), the row
-// coordinates stay in registers, and the right-hand operand (the Gaussian
-// table in sampling mode, the basis Q in projection mode) is read as
-// prepacked BF16 pairs straight from L1/L2 instead of being restaged per chunk.
+// k_kmm_fast: the same product on the tensor cores (FP32 working precision),
+// specialised on the dimension (1-3), the kernel and its derivative.  CTA = 4
+// warps = 64 operator rows, warp = 16 rows; each lane evaluates the eight
+// kernel entries of its m16n8k16 A fragment in registers and splits them into
+// BF16 hi + lo (relative error ~2^-17 of an entry).  Sample pass: W = a Gaussian
+// table whose entries are BF16 numbers, 2 MMAs per tile.  Projection pass: W = Q
+// split hi + lo, 3 MMAs per tile (hi*hi, lo*hi, hi*lo).  Coordinates are
+// pre-scaled so that each entry costs one hardware square root and one hardware
+// exp2 (PTX sqrt.approx / ex2.approx, both within a few ulp of FP32), the row
+// coordinates stay in registers, and the right-hand operand (the Gaussian table
+// in sampling mode, the basis Q in projection mode) is read as prepacked BF16
+// pairs straight from L1/L2 instead of being restaged per chunk.
 // Instruction issue bounds it, then the special-function unit (two of its
 // operations per entry; 75 % busy with 16 sampled columns): distances, kernel
 // values, the norm and the splits are done two entries per instruction
