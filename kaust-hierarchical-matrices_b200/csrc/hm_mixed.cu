@@ -769,42 +769,11 @@ __global__ void __launch_bounds__(32 * WPC * SP, (NH == 1 && SP == 1 ? kP2PerSm 
       }
     }
   }
-  if (SP == 1) {
-    // Descriptors as they come, and 16 columns a step in 8-byte words: what this
-    // variant holds at 28 warps per SM.  2^20 points, 16 right-hand sides: 2065
-    // us against 2074 with the loop below, 2260 with both row halves of a tile
-    // in one step; 2^18 points, 64 right-hand sides: 1393 against 1423.
-    for (int q = d0; q < d1; ++q) {
-      const MxDense& D = dense[leaf_dblk[q]];
-      const uint4* dh = store + (D.hi + (long long)(G - D.row_tile0) * D.nct) * 32 + dense_word(lane >> 2, lane & 3);
-      const uint4* dl = dh + (D.lo - D.hi) * 32;
-      const int xt0 = D.col_tile0, nc2 = D.nct >> 1;
-#pragma unroll 1
-      for (int c2 = 0; c2 < nc2; ++c2) {
-        const int tile = (c2 >> 1) * 128, half = c2 & 1;
-        uint2 rh[4], rl[4];  // rows g + 8 w
-#pragma unroll
-        for (int w = 0; w < 4; ++w) {
-          rh[w] = __ldg(reinterpret_cast<const uint2*>(dense_row(dh + tile, w)) + half);
-          rl[w] = __ldg(reinterpret_cast<const uint2*>(dense_row(dl + tile, w)) + half);
-        }
-        const size_t xt = (size_t)(xt0 + (c2 >> 1)) * 128 + lane + 32 * half;
-#pragma unroll
-        for (int h = 0; h < NH; ++h) {
-          const uint4 xh = __ldg(Xf + h * xh_ + xt), xl = __ldg(Xf + h * xh_ + xt + 64);
-#pragma unroll
-          for (int mt = 0; mt < 2; ++mt)
-            mx_p2_dense(acc[h][mt], rh[2 * mt].x, rh[2 * mt + 1].x, rh[2 * mt].y, rh[2 * mt + 1].y, rl[2 * mt].x,
-                        rl[2 * mt + 1].x, rl[2 * mt].y, rl[2 * mt + 1].y, xh, xl);
-        }
-      }
-    }
-  }
   int at = SP > 1 ? __shfl_sync(0xffffffffu, my_end, 31) : 0;
-  for (int q0 = d0; SP > 1 && q0 < d1; q0 += 32) {
+  for (int q0 = d0; q0 < d1; q0 += 32) {
     // up to 32 dense blocks' descriptors at once
     long long my_dh = 0;
-    int my_dl = 0, my_x = 0, my_c = 0;  // my_dl: from the high parts to the low ones
+    int my_dl = 0, my_x = 0, my_c = 0, my_e = 0;  // my_dl: from the high parts to the low ones
     if (q0 + lane < d1) {
       const MxDense D = dense[leaf_dblk[q0 + lane]];
       my_dh = D.hi + (long long)(G - D.row_tile0) * D.nct;
@@ -812,36 +781,73 @@ __global__ void __launch_bounds__(32 * WPC * SP, (NH == 1 && SP == 1 ? kP2PerSm 
       my_x = D.col_tile0;
       my_c = D.nct;
     }
-    const int my_e = at + warp_scan(my_c, lane);
+    if (SP > 1) my_e = at + warp_scan(my_c, lane);
     const int nq = min(32, d1 - q0);
     for (int q = 0; q < nq; ++q) {
       const int nct = __shfl_sync(0xffffffffu, my_c, q);
-      int ca, cb;  // this warp's 32-column tiles
-      run(__shfl_sync(0xffffffffu, my_e, q) - nct, nct >> 2, 4, ca, cb);
-      if (ca >= cb) continue;
+      int ca = 0, cb = nct >> 2;  // this warp's 32-column tiles
+      if (SP > 1) {
+        run(__shfl_sync(0xffffffffu, my_e, q) - nct, nct >> 2, 4, ca, cb);
+        if (ca >= cb) continue;
+      }
       const uint4* dh = store + __shfl_sync(0xffffffffu, my_dh, q) * 32 + dense_word(lane >> 2, lane & 3);
       const uint4* dl = dh + (long long)__shfl_sync(0xffffffffu, my_dl, q) * 32;
       const int xt0 = __shfl_sync(0xffffffffu, my_x, q);
-      // rows 16 mt + g and + 8 of every tile in turn
+      if (SP == 1) {
+        // 16 columns a step in 8-byte words (the second half of a tile comes
+        // from L1): a whole tile's words spill at 28 warps per SM.  2^20 points,
+        // 16 right-hand sides: 2101 us, 2456 with whole tiles, 2115 with two of
+        // the four row groups a step; 143668 2-D points with many dense leaf
+        // blocks, 48 right-hand sides: 15.8 ms, 19.5 and 18.0.
+#pragma unroll 1
+        for (int c2 = 0; c2 < 2 * cb; ++c2) {
+          const int tile = (c2 >> 1) * 128, half = c2 & 1;
+          uint2 rh[4], rl[4];  // rows g + 8 w
 #pragma unroll
-      for (int mt = 0; mt < 2; ++mt) {
-#pragma unroll(NH == 2 ? 1 : 2)
-        for (int ct = ca; ct < cb; ++ct) {
-          const uint4 h0 = ld_tile<SH>(dense_row(dh + ct * 128, 2 * mt));
-          const uint4 h1 = ld_tile<SH>(dense_row(dh + ct * 128, 2 * mt + 1));
-          const uint4 l0 = ld_tile<SH>(dense_row(dl + ct * 128, 2 * mt));
-          const uint4 l1 = ld_tile<SH>(dense_row(dl + ct * 128, 2 * mt + 1));
-          const size_t xt = (size_t)(xt0 + ct) * 128 + lane;
+          for (int w = 0; w < 4; ++w) {
+            rh[w] = __ldg(reinterpret_cast<const uint2*>(dense_row(dh + tile, w)) + half);
+            rl[w] = __ldg(reinterpret_cast<const uint2*>(dense_row(dl + tile, w)) + half);
+          }
+          const size_t xt = (size_t)(xt0 + (c2 >> 1)) * 128 + lane + 32 * half;
 #pragma unroll
           for (int h = 0; h < NH; ++h) {
-            const uint4* xp = Xf + h * xh_ + xt;
-            mx_p2_dense(acc[h][mt], h0.x, h1.x, h0.y, h1.y, l0.x, l1.x, l0.y, l1.y, __ldg(xp), __ldg(xp + 64));
-            mx_p2_dense(acc[h][mt], h0.z, h1.z, h0.w, h1.w, l0.z, l1.z, l0.w, l1.w, __ldg(xp + 32), __ldg(xp + 96));
+            const uint4 xh = __ldg(Xf + h * xh_ + xt), xl = __ldg(Xf + h * xh_ + xt + 64);
+#pragma unroll
+            for (int mt = 0; mt < 2; ++mt)
+              mx_p2_dense(acc[h][mt], rh[2 * mt].x, rh[2 * mt + 1].x, rh[2 * mt].y, rh[2 * mt + 1].y, rl[2 * mt].x,
+                          rl[2 * mt + 1].x, rl[2 * mt].y, rl[2 * mt + 1].y, xh, xl);
           }
+        }
+      } else {
+        // whole tiles: 18227 2-D points, 4 right-hand sides 221 us, 244 with two
+        // of the four row groups a step
+#pragma unroll 1
+        for (int ct = ca; ct < cb; ++ct) {
+          uint4 rh[4], rl[4];  // rows g + 8 w
+#pragma unroll
+          for (int w = 0; w < 4; ++w) rh[w] = ld_tile<SH>(dense_row(dh + ct * 128, w));
+#pragma unroll
+          for (int w = 0; w < 4; ++w) rl[w] = ld_tile<SH>(dense_row(dl + ct * 128, w));
+          const size_t xt = (size_t)(xt0 + ct) * 128 + lane;
+#pragma unroll
+          for (int c = 0; c < 2; ++c)
+#pragma unroll
+            for (int h = 0; h < NH; ++h) {
+              const uint4* xp = Xf + h * xh_ + xt + 32 * c;
+              const uint4 xh = __ldg(xp), xl = __ldg(xp + 64);
+#pragma unroll
+              for (int mt = 0; mt < 2; ++mt) {
+                const uint4 &h0 = rh[2 * mt], &h1 = rh[2 * mt + 1], &l0 = rl[2 * mt], &l1 = rl[2 * mt + 1];
+                if (c == 0)
+                  mx_p2_dense(acc[h][mt], h0.x, h1.x, h0.y, h1.y, l0.x, l1.x, l0.y, l1.y, xh, xl);
+                else
+                  mx_p2_dense(acc[h][mt], h0.z, h1.z, h0.w, h1.w, l0.z, l1.z, l0.w, l1.w, xh, xl);
+              }
+            }
         }
       }
     }
-    at = __shfl_sync(0xffffffffu, my_e, 31);
+    if (SP > 1) at = __shfl_sync(0xffffffffu, my_e, 31);
   }
   const int base = leaf_off[x] + 32 * (G - leaf_tile0[x]), lim = leaf_off[x + 1];
   // sum i of lane L: half i / 16, rows 16 mt + g (+ 8), column 8 nb + 2 t (+ 1) of C fragment (mt, nb)
