@@ -1,5 +1,6 @@
 // hm_memory.cu -- the library's device memory: cudaMalloc for large blocks, a
 // bounded pool per device for the small ones (hm_internal.h).
+#include <chrono>
 #include <mutex>
 #include <vector>
 
@@ -17,6 +18,8 @@ struct DevicePool {
   cudaStream_t stream = nullptr;  // orders the allocations of long-lived blocks
   std::vector<void*> tokens;      // see wait_device
   std::vector<Block> parked;      // released, but not yet known to be out of use
+  std::chrono::steady_clock::time_point asked;  // dev_settle's last question, and what was idle then
+  unsigned long long idle = 0;
 };
 std::mutex g_mu;
 DevicePool g_pools[kMaxDevices];
@@ -217,11 +220,24 @@ void dev_settle() {
   size_t freeb = 0, total = 0;
   unsigned long long held = 0, used = 0;
   WhileCapturing guard;
-  // (cudaMemGetInfo takes 70 us, the pool's own numbers 0.1)
   if (cudaMemPoolGetAttribute(P->pool, cudaMemPoolAttrReservedMemCurrent, &held) == cudaSuccess &&
       cudaMemPoolGetAttribute(P->pool, cudaMemPoolAttrUsedMemCurrent, &used) == cudaSuccess &&
-      held > used + kPoolLow && cudaMemGetInfo(&freeb, &total) == cudaSuccess && freeb < kPoolRoom)
-    give_back(P);
+      held > used + kPoolLow) {
+    // cudaMemGetInfo takes 70 us, a small build 500: at most every 10 ms, or
+    // when more has become idle
+    const auto now = std::chrono::steady_clock::now();
+    const unsigned long long idle = held - used;
+    bool ask;
+    {
+      std::lock_guard<std::mutex> lock(g_mu);
+      ask = idle > P->idle + (kPoolLow >> 2) || now - P->asked > std::chrono::milliseconds(10);
+      if (ask) P->asked = now, P->idle = idle;
+    }
+    if (ask && cudaMemGetInfo(&freeb, &total) == cudaSuccess && freeb < kPoolRoom && give_back(P) == cudaSuccess) {
+      std::lock_guard<std::mutex> lock(g_mu);
+      P->idle = 0;
+    }
+  }
   cudaGetLastError();  // the entry point's own status stands
 }
 
