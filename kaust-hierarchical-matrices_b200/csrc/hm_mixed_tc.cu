@@ -550,23 +550,28 @@ __global__ void __launch_bounds__(kTcThreads, 1)
             const uint64_t da = (kind == 1 ? adesc1 : kind == 2 ? adesc2 : adesc0) + off, db = bdesc0 + off;
             const uint32_t d = tmem + (uint32_t)((chain % kP2Bufs) * 128);
             uint32_t acc = in_chain == 0 ? 0u : 1u;
-            // dense tiles and X's image are K-major, panels' tiles and T blocks MN-major
-            const uint32_t idesc = kind == 2 ? kIdesc : kIdescABmn;
             // 16 columns at a time: two column tiles (1024 bytes of A) or half a dense tile's rows (32 bytes),
-            // two K blocks (4096 bytes of B at 16384)
-            const uint32_t aq = kind == 2 ? 2u : 64u;
+            // two K blocks (4096 bytes of B at 16384).  Dense tiles and X's image are K-major, panels' tiles and T
+            // blocks MN-major.
             if (kind == 1) {
 #pragma unroll
               for (int q = 0; q < 4; ++q)
                 if (q < nq) tc_mma_bf16(d, da + q * 64, db + (1024 + q * 256), kIdescABmn, q ? 1u : acc);
+            } else if (kind == 2) {
+#pragma unroll
+              for (int q = 0; q < 2; ++q) {
+                tc_mma_bf16(d, da + q * 2, db + (1024 + q * 256), kIdesc, q ? 1u : acc);  // D_hi X_hi
+                tc_mma_bf16(d, da + q * 2, db + (1536 + q * 256), kIdesc, 1u);          // D_hi X_lo
+                tc_mma_bf16(d, da + (512 + q * 2), db + (1024 + q * 256), kIdesc, 1u);  // D_lo X_hi
+              }
             } else {
 #pragma unroll
               for (int q = 0; q < 2; ++q)
                 if (q < nq) {
-                  tc_mma_bf16(d, da + q * aq, db + (1024 + q * 256), idesc, q ? 1u : acc);  // U_hi T_hi
+                  tc_mma_bf16(d, da + q * 64, db + (1024 + q * 256), kIdescABmn, q ? 1u : acc);  // U_hi T_hi
                   if (kind != 3) {
-                    tc_mma_bf16(d, da + q * aq, db + (1536 + q * 256), idesc, 1u);        // U_hi T_lo
-                    tc_mma_bf16(d, da + (512 + q * aq), db + (1024 + q * 256), idesc, 1u);  // U_lo T_hi
+                    tc_mma_bf16(d, da + q * 64, db + (1536 + q * 256), kIdescABmn, 1u);        // U_hi T_lo
+                    tc_mma_bf16(d, da + (512 + q * 64), db + (1024 + q * 256), kIdescABmn, 1u);  // U_lo T_hi
                   }
                 }
             }
